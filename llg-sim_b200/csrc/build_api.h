@@ -11,11 +11,17 @@ void llg_set_error_message(const char* msg);
 namespace llg {
 
 FftPlan make_plan(int L);
-// Alternative radix plans of length L for the autotuner (the first is make_plan(L)).
+// Radix plans of length L for the autotuner (the first is make_plan(L)), unpadded.
 std::vector<FftPlan> plan_candidates(int L);
+// The plan with padded signals where `buffers` of them fit smem_max bytes, else unpadded.
+FftPlan padded_plan(FftPlan p, bool fp64, int buffers, size_t smem_max);
+// Pass tables of a plan (fft_smem.cuh) into out[2L].
+cudaError_t launch_pass_tables(const FftPlan& plan, void* out, bool fp64, cudaStream_t s);
 cudaError_t launch_twiddles(void* tw, int L2, bool fp64, cudaStream_t s);
+// In-place transforms of nsig_a * nsig_b strided signals of length L = base.L; tw: the
+// pass tables of the plan, tw2: exp(-2 pi i k / (2L)).
 template <typename R>
-cudaError_t launch_fft_strided(void* data, int L, const void* tw2, long long elem_stride, int nsig_a,
+cudaError_t launch_fft_strided(void* data, const FftPlan& base, const void* tw, const void* tw2, long long elem_stride, int nsig_a,
                                long long stride_a, int nsig_b, long long stride_b, bool inverse, cudaStream_t s);
 
 // Unscaled FP64 k-space kernel planes [4][py][px] complex for pbc_x / pbc_y images.

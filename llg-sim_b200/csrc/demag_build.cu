@@ -214,17 +214,18 @@ __global__ void k_twiddles(cx<R>* tw, int L2) {
 }
 
 template <typename R>
-__global__ void k_fft_strided(cx<R>* data, FftPlan plan, const cx<R>* tw2, long long elem_stride, int nsig_a,
-                              long long stride_a, long long stride_b, int inverse) {
+__global__ void __launch_bounds__(256) k_fft_strided(cx<R>* data, FftPlan plan, const cx<R>* tw, const cx<R>* tw2,
+                                                     long long elem_stride, int nsig_a, long long stride_a,
+                                                     long long stride_b, int inverse) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cx<R>* A = reinterpret_cast<cx<R>*>(smem_raw);
-    cx<R>* B = A + plan.L;
+    cx<R>* B = A + plan.stride();
     const int sig = blockIdx.x;
     const long long base = (long long)(sig % nsig_a) * stride_a + (long long)(sig / nsig_a) * stride_b;
-    for (int t = threadIdx.x; t < plan.L; t += blockDim.x) A[t] = data[base + t * elem_stride];
+    for (int t = threadIdx.x; t < plan.L; t += blockDim.x) A[plan.at(t)] = data[base + t * elem_stride];
     __syncthreads();
-    cx<R>* res = fft_smem<R>(A, B, 1, plan, tw2, inverse != 0);
-    for (int t = threadIdx.x; t < plan.L; t += blockDim.x) data[base + t * elem_stride] = res[t];
+    cx<R>* res = inverse ? fft_smem<R, true>(A, B, 1, plan, tw, tw2) : fft_smem<R, false>(A, B, 1, plan, tw, tw2);
+    for (int t = threadIdx.x; t < plan.L; t += blockDim.x) data[base + t * elem_stride] = res[plan.at(t)];
 }
 
 // Column transforms of adjacent signals (stride between signals 1 element): a block
@@ -232,99 +233,153 @@ __global__ void k_fft_strided(cx<R>* data, FftPlan plan, const cx<R>* tw2, long 
 // elements in memory (whole 32-byte sectors in FP64 instead of half ones); each
 // signal's arithmetic is the one of k_fft_strided.
 template <typename R>
-__global__ void k_fft_strided_tiled(cx<R>* data, FftPlan plan, const cx<R>* tw2, long long elem_stride, int nsig_a,
-                                    long long stride_b, int ns, int inverse) {
+__global__ void __launch_bounds__(256) k_fft_strided_tiled(cx<R>* data, FftPlan plan, const cx<R>* tw,
+                                                           const cx<R>* tw2, long long elem_stride, int nsig_a,
+                                                           long long stride_b, int ns, int inverse) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int L = plan.L;
+    const int L = plan.L, LP = plan.stride();
     cx<R>* A = reinterpret_cast<cx<R>*>(smem_raw);
-    cx<R>* B = A + (size_t)ns * L;
+    cx<R>* B = A + (size_t)ns * LP;
     const int tiles_a = nsig_a / ns;
     const long long base = (long long)(blockIdx.x % tiles_a) * ns + (long long)(blockIdx.x / tiles_a) * stride_b;
     for (int e = threadIdx.x; e < ns * L; e += blockDim.x) {
         const int c = e % ns, t = e / ns;
-        A[(size_t)c * L + t] = data[base + c + t * elem_stride];
+        A[(size_t)c * LP + plan.at(t)] = data[base + c + t * elem_stride];
     }
     __syncthreads();
-    cx<R>* res = fft_smem<R>(A, B, ns, plan, tw2, inverse != 0);
+    cx<R>* res = inverse ? fft_smem<R, true>(A, B, ns, plan, tw, tw2) : fft_smem<R, false>(A, B, ns, plan, tw, tw2);
     for (int e = threadIdx.x; e < ns * L; e += blockDim.x) {
         const int c = e % ns, t = e / ns;
-        data[base + c + t * elem_stride] = res[(size_t)c * L + t];
+        data[base + c + t * elem_stride] = res[(size_t)c * LP + plan.at(t)];
     }
 }
 
 template __global__ void k_twiddles<float>(cx<float>*, int);
 template __global__ void k_twiddles<double>(cx<double>*, int);
 
-FftPlan make_plan(int L) {
-    FftPlan p{};
-    p.L = L;
-    p.npass = 0;
-    int r = L;
-    for (int f : {8, 4, 2, 3, 5}) {
-        while (r % f == 0 && r > 1) {
-            p.radix[p.npass++] = f;
-            r /= f;
-        }
-    }
-    for (int f = 7; r > 1; f += 2) {
-        while (r % f == 0) {
-            p.radix[p.npass++] = f;
-            r /= f;
-        }
-    }
-    return p;
+template <typename R>
+__global__ void k_pass_tables_smem(FftPlan plan, cx<R>* out) {
+    double s, c;
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; pass_table_entry(plan, e, &c, &s); e += gridDim.x * blockDim.x)
+        out[e] = mkc((R)c, (R)s);
 }
 
-// Candidate radix plans of the generic Stockham transform of length L (any radix
-// order is a valid Stockham plan): the powers of two grouped mostly as 8s or
-// mostly as 4s, each with the odd factors last (make_plan's order), first, or the
-// powers of two in ascending order.  The first candidate is make_plan(L).
+static constexpr int kRadices[] = {16, 12, 10, 8, 6, 5, 4, 3, 2};   // radices with a register butterfly
+
+// Radix plans of the generic Stockham transform of length L: the fewest passes over
+// the radices with a register butterfly (16, 12, 10, 8, 6, 5, 4, 3, 2; a larger
+// prime factor is a pass of its own), each multiset of radices in descending and in
+// ascending order, the ones with the smallest sum of radices (fewest registers and
+// the most even split) first.
 std::vector<FftPlan> plan_candidates(int L) {
-    std::vector<FftPlan> out;
-    out.push_back(make_plan(L));
-    int r = L, e2 = 0;
-    while (r % 2 == 0 && r > 1) {
-        r /= 2;
-        ++e2;
-    }
-    std::vector<int> odd;
-    for (int f : {3, 5}) while (r % f == 0) { odd.push_back(f); r /= f; }
-    for (int f = 7; r > 1; f += 2) while (r % f == 0) { odd.push_back(f); r /= f; }
-    auto twos = [&](bool eights) {
-        std::vector<int> v;
-        int e = e2;
-        if (eights) {
-            while (e >= 3) { v.push_back(8); e -= 3; }
-            if (e == 2) v.push_back(4);
-            if (e == 1) v.push_back(2);
-        } else {
-            while (e >= 2) { v.push_back(4); e -= 2; }
-            if (e == 1) v.push_back(2);
+    std::vector<int> primes;   // factors without a register butterfly
+    int r = L;
+    for (int f : {2, 3, 5})
+        while (r % f == 0) r /= f;
+    for (int f = 7; r > 1; f += 2)
+        while (r % f == 0) {
+            primes.push_back(f);
+            r /= f;
         }
-        return v;
+    int smooth = L;
+    for (int p : primes) smooth /= p;
+    std::vector<std::vector<int>> best;
+    std::vector<int> cur;
+    auto search = [&](auto&& self, int rest, int max_radix, size_t depth) -> void {
+        if (rest == 1) {
+            if (cur.size() == depth) best.push_back(cur);
+            return;
+        }
+        if (cur.size() >= depth) return;
+        for (int p : kRadices)
+            if (p <= max_radix && rest % p == 0) {
+                cur.push_back(p);
+                self(self, rest / p, p, depth);
+                cur.pop_back();
+            }
     };
-    auto add = [&](const std::vector<int>& rad) {
-        if (rad.empty() || (int)rad.size() > kMaxRadices) return;
+    for (size_t depth = 0; best.empty() && depth <= (size_t)kMaxRadices; ++depth) search(search, smooth, 16, depth);
+    std::stable_sort(best.begin(), best.end(), [](const std::vector<int>& a, const std::vector<int>& b) {
+        int sa = 0, sb = 0;
+        for (int x : a) sa += x;
+        for (int x : b) sb += x;
+        return sa < sb;
+    });
+    std::vector<FftPlan> out;
+    auto add = [&](std::vector<int> rad) {
+        rad.insert(rad.end(), primes.begin(), primes.end());
         FftPlan p{};
         p.L = L;
+        p.sh = 30;
         p.npass = (int)rad.size();
         for (size_t i = 0; i < rad.size(); ++i) p.radix[i] = rad[i];
         for (const FftPlan& q : out)
-            if (q.npass == p.npass && std::equal(q.radix, q.radix + q.npass, p.radix)) return;
+            if (std::equal(q.radix, q.radix + q.npass, p.radix)) return;
         out.push_back(p);
     };
-    for (bool eights : {true, false}) {
-        std::vector<int> t = twos(eights);
-        std::vector<int> a = t, b = odd, c = t;
-        a.insert(a.end(), odd.begin(), odd.end());           // powers of two first
-        b.insert(b.end(), t.begin(), t.end());               // odd factors first
-        std::reverse(c.begin(), c.end());                    // ascending powers of two, then odd
-        c.insert(c.end(), odd.begin(), odd.end());
-        add(a);
-        add(b);
-        add(c);
+    for (size_t i = 0; i < best.size() && i < 3; ++i) {
+        add(best[i]);
+        std::reverse(best[i].begin(), best[i].end());
+        add(best[i]);
     }
     return out;
+}
+
+namespace {
+// Descending radices of the 2-3-5-smooth `rest` in exactly `depth` passes with the
+// smallest sum (the first such in search order, as in plan_candidates).
+void best_radices(int rest, int max_radix, int n, int depth, int sum, int* cur, int* best, int* best_sum) {
+    if (rest == 1) {
+        if (n == depth && sum < *best_sum) {
+            *best_sum = sum;
+            std::copy(cur, cur + n, best);
+        }
+        return;
+    }
+    if (n >= depth) return;
+    for (int p : kRadices)
+        if (p <= max_radix && rest % p == 0) {
+            cur[n] = p;
+            best_radices(rest / p, p, n + 1, depth, sum + p, cur, best, best_sum);
+        }
+}
+}  // namespace
+
+// plan_candidates(L)[0] without allocations (plans are also formed per call).
+FftPlan make_plan(int L) {
+    FftPlan p{};
+    p.L = L;
+    p.sh = 30;
+    int smooth = L;
+    for (int f : {2, 3, 5})
+        while (smooth % f == 0) smooth /= f;
+    int rest = smooth;
+    smooth = L / smooth;
+    int cur[kMaxRadices], best_sum = 1 << 30;
+    for (int depth = 0; depth <= kMaxRadices && best_sum == 1 << 30; ++depth) {
+        best_radices(smooth, 16, 0, depth, 0, cur, p.radix, &best_sum);
+        p.npass = depth;
+    }
+    for (int f = 7; rest > 1; f += 2)
+        while (rest % f == 0) {
+            p.radix[p.npass++] = f;
+            rest /= f;
+        }
+    return p;
+}
+
+FftPlan padded_plan(FftPlan p, bool fp64, int buffers, size_t smem_max) {
+    const size_t elem = fp64 ? sizeof(cx<double>) : sizeof(cx<float>);
+    p.sh = fp64 ? 3 : 4;
+    if (elem * (size_t)buffers * p.stride() > smem_max) p.sh = 30;
+    return p;
+}
+
+cudaError_t launch_pass_tables(const FftPlan& plan, void* out, bool fp64, cudaStream_t s) {
+    const int blocks = (2 * plan.L + 255) / 256;
+    if (fp64) k_pass_tables_smem<double><<<blocks, 256, 0, s>>>(plan, reinterpret_cast<cx<double>*>(out));
+    else k_pass_tables_smem<float><<<blocks, 256, 0, s>>>(plan, reinterpret_cast<cx<float>*>(out));
+    return cudaGetLastError();
 }
 
 cudaError_t launch_twiddles(void* tw, int L2, bool fp64, cudaStream_t s) {
@@ -335,36 +390,40 @@ cudaError_t launch_twiddles(void* tw, int L2, bool fp64, cudaStream_t s) {
 }
 
 template <typename R>
-cudaError_t launch_fft_strided(void* data, int L, const void* tw2, long long elem_stride, int nsig_a, long long stride_a,
-                               int nsig_b, long long stride_b, bool inverse, cudaStream_t s) {
-    FftPlan plan = make_plan(L);
+cudaError_t launch_fft_strided(void* data, const FftPlan& base, const void* tw, const void* tw2, long long elem_stride, int nsig_a,
+                               long long stride_a, int nsig_b, long long stride_b, bool inverse, cudaStream_t s) {
+    constexpr bool fp64 = sizeof(R) == 8;
+    constexpr size_t kMax = 227 * 1024;
+    const int L = base.L;
     if (elem_stride > 1 && stride_a == 1) {
         // adjacent columns: tile NS of them per block where shared memory allows
         int ns = 1;
         while (ns < 8 && nsig_a % (2 * ns) == 0 && 2 * (size_t)(2 * ns) * L * sizeof(cx<R>) <= 200 * 1024) ns *= 2;
         if (ns > 1) {
-            const size_t smem = 2 * (size_t)ns * L * sizeof(cx<R>);
+            const FftPlan plan = padded_plan(base, fp64, 2 * ns, kMax);
+            const size_t smem = 2 * (size_t)ns * plan.stride() * sizeof(cx<R>);
             cudaError_t e = cudaFuncSetAttribute(k_fft_strided_tiled<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  (int)smem);
             if (e != cudaSuccess) return e;
             k_fft_strided_tiled<R><<<(nsig_a / ns) * nsig_b, 256, smem, s>>>(
-                reinterpret_cast<cx<R>*>(data), plan, reinterpret_cast<const cx<R>*>(tw2), elem_stride, nsig_a,
-                stride_b, ns, inverse ? 1 : 0);
+                reinterpret_cast<cx<R>*>(data), plan, reinterpret_cast<const cx<R>*>(tw),
+                reinterpret_cast<const cx<R>*>(tw2), elem_stride, nsig_a, stride_b, ns, inverse ? 1 : 0);
             return cudaGetLastError();
         }
     }
-    size_t smem = 2 * (size_t)L * sizeof(cx<R>);
+    const FftPlan plan = padded_plan(base, fp64, 2, kMax);
+    size_t smem = 2 * (size_t)plan.stride() * sizeof(cx<R>);
     cudaError_t e = cudaFuncSetAttribute(k_fft_strided<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_fft_strided<R><<<nsig_a * nsig_b, 256, smem, s>>>(reinterpret_cast<cx<R>*>(data), plan,
-                                                        reinterpret_cast<const cx<R>*>(tw2), elem_stride, nsig_a,
-                                                        stride_a, stride_b, inverse ? 1 : 0);
+    k_fft_strided<R><<<nsig_a * nsig_b, 256, smem, s>>>(
+        reinterpret_cast<cx<R>*>(data), plan, reinterpret_cast<const cx<R>*>(tw),
+        reinterpret_cast<const cx<R>*>(tw2), elem_stride, nsig_a, stride_a, stride_b, inverse ? 1 : 0);
     return cudaGetLastError();
 }
-template cudaError_t launch_fft_strided<float>(void*, int, const void*, long long, int, long long, int, long long,
-                                               bool, cudaStream_t);
-template cudaError_t launch_fft_strided<double>(void*, int, const void*, long long, int, long long, int, long long,
-                                                bool, cudaStream_t);
+template cudaError_t launch_fft_strided<float>(void*, const FftPlan&, const void*, const void*, long long, int, long long, int,
+                                               long long, bool, cudaStream_t);
+template cudaError_t launch_fft_strided<double>(void*, const FftPlan&, const void*, const void*, long long, int, long long, int,
+                                                long long, bool, cudaStream_t);
 
 #define CK(x)                                  \
     do {                                       \
@@ -391,8 +450,8 @@ cudaError_t build_demag_kernel(int nx, int ny, double dx, double dy, double dz, 
     do {
         if ((err = cudaMalloc(&quad, sizeof(double) * 4 * (size_t)nx * ny)) != cudaSuccess) break;
         if ((err = cudaMalloc(&planes, sizeof(cx<double>) * 4 * (size_t)np)) != cudaSuccess) break;
-        if ((err = cudaMalloc(&twx, sizeof(cx<double>) * 2 * (size_t)px)) != cudaSuccess) break;
-        if ((err = cudaMalloc(&twy, sizeof(cx<double>) * 2 * (size_t)py)) != cudaSuccess) break;
+        if ((err = cudaMalloc(&twx, sizeof(cx<double>) * 4 * (size_t)px)) != cudaSuccess) break;
+        if ((err = cudaMalloc(&twy, sizeof(cx<double>) * 4 * (size_t)py)) != cudaSuccess) break;
         {
             long long warps = (long long)nx * ny;
             long long threads = warps * 32;
@@ -404,10 +463,12 @@ cudaError_t build_demag_kernel(int nx, int ny, double dx, double dy, double dz, 
         if ((err = cudaGetLastError()) != cudaSuccess) break;
         if ((err = launch_twiddles(twx, 2 * px, true, s)) != cudaSuccess) break;
         if ((err = launch_twiddles(twy, 2 * py, true, s)) != cudaSuccess) break;
+        if ((err = launch_pass_tables(make_plan(px), twx + 2 * px, true, s)) != cudaSuccess) break;
+        if ((err = launch_pass_tables(make_plan(py), twy + 2 * py, true, s)) != cudaSuccess) break;
         // rows: length px, contiguous; signals = py rows x 4 planes
-        if ((err = launch_fft_strided<double>(planes, px, twx, 1, py, px, 4, np, false, s)) != cudaSuccess) break;
+        if ((err = launch_fft_strided<double>(planes, make_plan(px), twx + 2 * px, twx, 1, py, px, 4, np, false, s)) != cudaSuccess) break;
         // columns: length py, stride px; signals = px columns x 4 planes
-        if ((err = launch_fft_strided<double>(planes, py, twy, px, px, 1, 4, np, false, s)) != cudaSuccess) break;
+        if ((err = launch_fft_strided<double>(planes, make_plan(py), twy + 2 * py, twy, px, px, 1, 4, np, false, s)) != cudaSuccess) break;
         const double scale = 1.0 / (double)np;
         int blocks = ((nx + 1) * (ny + 1) + 255) / 256;
         if (fp64_out)
@@ -439,8 +500,8 @@ cudaError_t build_demag_kernel_pbc(int nx, int ny, double dx, double dy, double 
     cudaError_t err = cudaSuccess;
     do {
         if ((err = cudaMalloc(&comp, sizeof(double) * 4 * (size_t)ndisp)) != cudaSuccess) break;
-        if ((err = cudaMalloc(&twx, sizeof(cx<double>) * 2 * (size_t)px)) != cudaSuccess) break;
-        if ((err = cudaMalloc(&twy, sizeof(cx<double>) * 2 * (size_t)py)) != cudaSuccess) break;
+        if ((err = cudaMalloc(&twx, sizeof(cx<double>) * 4 * (size_t)px)) != cudaSuccess) break;
+        if ((err = cudaMalloc(&twy, sizeof(cx<double>) * 4 * (size_t)py)) != cudaSuccess) break;
         const long long blocks = (ndisp * 32 + 255) / 256;
         k_kernel_displacements<<<(unsigned)blocks, 256, 0, s>>>(sx_max, sy_max, dx, dy, dz, 10.0, comp);
         if ((err = cudaGetLastError()) != cudaSuccess) break;
@@ -448,8 +509,10 @@ cudaError_t build_demag_kernel_pbc(int nx, int ny, double dx, double dy, double 
         if ((err = cudaGetLastError()) != cudaSuccess) break;
         if ((err = launch_twiddles(twx, 2 * px, true, s)) != cudaSuccess) break;
         if ((err = launch_twiddles(twy, 2 * py, true, s)) != cudaSuccess) break;
-        if ((err = launch_fft_strided<double>(planes, px, twx, 1, py, px, 4, np, false, s)) != cudaSuccess) break;
-        if ((err = launch_fft_strided<double>(planes, py, twy, px, px, 1, 4, np, false, s)) != cudaSuccess) break;
+        if ((err = launch_pass_tables(make_plan(px), twx + 2 * px, true, s)) != cudaSuccess) break;
+        if ((err = launch_pass_tables(make_plan(py), twy + 2 * py, true, s)) != cudaSuccess) break;
+        if ((err = launch_fft_strided<double>(planes, make_plan(px), twx + 2 * px, twx, 1, py, px, 4, np, false, s)) != cudaSuccess) break;
+        if ((err = launch_fft_strided<double>(planes, make_plan(py), twy + 2 * py, twy, px, px, 1, 4, np, false, s)) != cudaSuccess) break;
         err = cudaStreamSynchronize(s);
     } while (0);
     if (comp) cudaFree(comp);

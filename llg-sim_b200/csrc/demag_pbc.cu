@@ -36,8 +36,9 @@ struct llg_demag_op {
     llg::cx<double>* K = nullptr;    // [4][py][px] unscaled kernel spectrum
     llg::cx<double>* M = nullptr;    // [3][py][px] work planes
     double* stage = nullptr;         // [nx*ny*3] AoS staging
-    llg::cx<double>* twx = nullptr;
+    llg::cx<double>* twx = nullptr;  // [2 px] exp(-2 pi i k / (2 px)), then [2 px] pass tables of planx
     llg::cx<double>* twy = nullptr;
+    llg::FftPlan planx{}, plany{};
 };
 
 namespace {
@@ -109,12 +110,12 @@ int demag_op_apply_device(llg_demag_op* op, double ms, const double* d_m_aos, do
     const long long np = (long long)op->px * op->py;
     k_pbc_pack<<<1184, 256, 0, s>>>(d_m_aos, op->nx, op->ny, op->px, op->py, ms, op->M);
     PBC_TRY(cudaGetLastError());
-    PBC_TRY(llg::launch_fft_strided<double>(op->M, op->px, op->twx, 1, op->py, op->px, 3, np, false, s));
-    PBC_TRY(llg::launch_fft_strided<double>(op->M, op->py, op->twy, op->px, op->px, 1, 3, np, false, s));
+    PBC_TRY(llg::launch_fft_strided<double>(op->M, op->planx, op->twx + 2 * op->px, op->twx, 1, op->py, op->px, 3, np, false, s));
+    PBC_TRY(llg::launch_fft_strided<double>(op->M, op->plany, op->twy + 2 * op->py, op->twy, op->px, op->px, 1, 3, np, false, s));
     k_pbc_multiply<<<1184, 256, 0, s>>>(op->K, np, op->M);
     PBC_TRY(cudaGetLastError());
-    PBC_TRY(llg::launch_fft_strided<double>(op->M, op->px, op->twx, 1, op->py, op->px, 3, np, true, s));
-    PBC_TRY(llg::launch_fft_strided<double>(op->M, op->py, op->twy, op->px, op->px, 1, 3, np, true, s));
+    PBC_TRY(llg::launch_fft_strided<double>(op->M, op->planx, op->twx + 2 * op->px, op->twx, 1, op->py, op->px, 3, np, true, s));
+    PBC_TRY(llg::launch_fft_strided<double>(op->M, op->plany, op->twy + 2 * op->py, op->twy, op->px, op->px, 1, 3, np, true, s));
     k_pbc_extract<<<1184, 256, 0, s>>>(op->M, op->nx, op->ny, op->px, op->py, 1.0 / (double)np, d_b_aos);
     PBC_TRY(cudaGetLastError());
     return LLG_OK;
@@ -272,6 +273,8 @@ int llg_demag_op_create(llg_ctx* ctx, const llg_grid* g, int64_t pbc_x, int64_t 
     op->dx = g->dx;
     op->dy = g->dy;
     op->dz = g->dz;
+    op->planx = llg::make_plan(op->px);
+    op->plany = llg::make_plan(op->py);
     const size_t np = (size_t)px * py;
     auto bail = [&](int rc) {
         destroy(op);
@@ -281,11 +284,13 @@ int llg_demag_op_create(llg_ctx* ctx, const llg_grid* g, int64_t pbc_x, int64_t 
     if (cudaMalloc(&op->K, 4 * np * sizeof(cx<double>)) != cudaSuccess ||
         cudaMalloc(&op->M, 3 * np * sizeof(cx<double>)) != cudaSuccess ||
         cudaMalloc(&op->stage, 3 * (size_t)g->nx * g->ny * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&op->twx, 2 * (size_t)px * sizeof(cx<double>)) != cudaSuccess ||
-        cudaMalloc(&op->twy, 2 * (size_t)py * sizeof(cx<double>)) != cudaSuccess)
+        cudaMalloc(&op->twx, 4 * (size_t)px * sizeof(cx<double>)) != cudaSuccess ||
+        cudaMalloc(&op->twy, 4 * (size_t)py * sizeof(cx<double>)) != cudaSuccess)
         return bail(fail(LLG_ERR_OOM, "cudaMalloc failed for a %lldx%lld demag operator", px, py));
     if (llg::launch_twiddles(op->twx, 2 * op->px, true, 0) != cudaSuccess ||
-        llg::launch_twiddles(op->twy, 2 * op->py, true, 0) != cudaSuccess)
+        llg::launch_twiddles(op->twy, 2 * op->py, true, 0) != cudaSuccess ||
+        llg::launch_pass_tables(op->planx, op->twx + 2 * op->px, true, 0) != cudaSuccess ||
+        llg::launch_pass_tables(op->plany, op->twy + 2 * op->py, true, 0) != cudaSuccess)
         return bail(fail(LLG_ERR_CUDA, "twiddle tables"));
     bool hit = cache_path && try_load(op, cache_path);
     if (!hit) {

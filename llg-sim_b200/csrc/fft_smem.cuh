@@ -1,11 +1,21 @@
 // fft_smem.cuh — the project's own shared-memory FFT for sm_100a.
 //
 // Batched complex FFTs of one runtime length L per call, data resident in
-// shared memory, mixed-radix Stockham autosort passes (radix 8/4/2/3/5 in
-// registers, any other prime factor by a direct small DFT), natural-order
-// output.  Twiddles come from a table of exp(-2 pi i k / (2L)), k < 2L, so that
-// the same table serves the zero-padding pre/post twiddles W_{2L}^n of the
-// pruned 2L-point transforms used by the demag convolution.
+// shared memory, mixed-radix Stockham autosort passes (radix 2..16 in registers,
+// any other prime factor by a direct small DFT), natural-order output.  A signal
+// is stored at padded indices (FftPlan::at).  Twiddles of pass s come from a
+// table in [r][k] order (pass_tables), the zero-padding pre/post twiddles
+// W_{2L}^n of the pruned 2L-point transforms from a table of
+// exp(-2 pi i k / (2L)), k < 2L.
+//
+// What bounds it and why it is laid out so: a pass moves every value through
+// shared memory once each way, so the composite radices (16, 12, 10, 6) save whole
+// passes and their barriers (1536 = 16*12*8 is 3 passes instead of 4, 50 = 10*5 is 2
+// instead of 3); the [r][k] tables let a warp read consecutive twiddles (the
+// strided reads of one exp(-2 pi i k / 2L) table cost up to 28 L1 wavefronts per
+// load and more than the data itself); one pad slot per 128 bytes spreads the
+// first pass's stride-P writes over all banks; the runtime divisions by m and ns
+// are multiplications by a reciprocal formed once per pass.
 #pragma once
 #include "types.cuh"
 
@@ -122,41 +132,129 @@ __device__ __forceinline__ void bfly5(cx<R>* v, bool inv) {
     v[3] = p2 - r2;
 }
 
+template <typename R>
+__device__ __forceinline__ void bfly16(cx<R>* v, bool inv) {
+    // 4 x 4: input n = 4 n1 + n2, output k = k1 + 4 k2, internal twiddles W_16^{n2 k1}
+    constexpr double c[10] = {1.0, 0.92387953251128675613, 0.70710678118654752440, 0.38268343236508977173, 0.0,
+                              0.0, -0.70710678118654752440, 0.0, 0.0, -0.92387953251128675613};
+    constexpr double s[10] = {0.0, 0.38268343236508977173, 0.70710678118654752440, 0.92387953251128675613, 1.0,
+                              0.0, 0.70710678118654752440, 0.0, 0.0, -0.38268343236508977173};
+    cx<R> y[16];
+#pragma unroll
+    for (int n2 = 0; n2 < 4; ++n2) {
+        cx<R> a[4] = {v[n2], v[4 + n2], v[8 + n2], v[12 + n2]};
+        bfly4(a, inv);
+#pragma unroll
+        for (int k1 = 0; k1 < 4; ++k1) {
+            const int e = n2 * k1;
+            if (e == 0) y[n2 * 4 + k1] = a[k1];
+            else if (e == 4) y[n2 * 4 + k1] = rot(a[k1], inv);
+            else {
+                const R wr = (R)c[e], wi = inv ? (R)s[e] : (R)-s[e];
+                y[n2 * 4 + k1] = mkc(a[k1].re * wr - a[k1].im * wi, a[k1].re * wi + a[k1].im * wr);
+            }
+        }
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < 4; ++k1) {
+        cx<R> b[4] = {y[k1], y[4 + k1], y[8 + k1], y[12 + k1]};
+        bfly4(b, inv);
+#pragma unroll
+        for (int k2 = 0; k2 < 4; ++k2) v[k1 + 4 * k2] = b[k2];
+    }
+}
+
+__host__ __device__ constexpr int inv_mod(int a, int n) {
+    for (int x = 1; x < n; ++x)
+        if ((a * x) % n == 1) return x;
+    return 1;
+}
+
+// In-register DFT of P points, natural order; coprime composites by the
+// Good-Thomas prime-factor mapping (no internal twiddles).
 template <typename R, int P>
+__device__ __forceinline__ void bfly(cx<R>* v, bool inv);
+template <typename R, int N1, int N2>
+__device__ __forceinline__ void bfly_pfa(cx<R>* v, bool inv) {
+    constexpr int N = N1 * N2, A = N2 * inv_mod(N2 % N1, N1), B = N1 * inv_mod(N1 % N2, N2);
+    cx<R> t[N];
+#pragma unroll
+    for (int n2 = 0; n2 < N2; ++n2) {
+        cx<R> x[N1];
+#pragma unroll
+        for (int n1 = 0; n1 < N1; ++n1) x[n1] = v[(N2 * n1 + N1 * n2) % N];
+        bfly<R, N1>(x, inv);
+#pragma unroll
+        for (int k1 = 0; k1 < N1; ++k1) t[k1 * N2 + n2] = x[k1];
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < N1; ++k1) {
+        cx<R> x[N2];
+#pragma unroll
+        for (int n2 = 0; n2 < N2; ++n2) x[n2] = t[k1 * N2 + n2];
+        bfly<R, N2>(x, inv);
+#pragma unroll
+        for (int k2 = 0; k2 < N2; ++k2) v[(A * k1 + B * k2) % N] = x[k2];
+    }
+}
+template <typename R, int P>
+__device__ __forceinline__ void bfly(cx<R>* v, bool inv) {
+    if constexpr (P == 2) bfly2(v);
+    if constexpr (P == 3) bfly3(v, inv);
+    if constexpr (P == 4) bfly4(v, inv);
+    if constexpr (P == 5) bfly5(v, inv);
+    if constexpr (P == 6) bfly_pfa<R, 2, 3>(v, inv);
+    if constexpr (P == 8) bfly8(v, inv);
+    if constexpr (P == 10) bfly_pfa<R, 2, 5>(v, inv);
+    if constexpr (P == 12) bfly_pfa<R, 4, 3>(v, inv);
+    if constexpr (P == 16) bfly16(v, inv);
+}
+
+// Quotient by a divisor fixed over a loop: exact for value * divisor < 2^32 (both
+// stay far below 2^16 here).
+struct FastDiv {
+    uint32_t mul;
+    int d;
+    __device__ __forceinline__ explicit FastDiv(int div) : mul(0xffffffffu / (uint32_t)div + 1u), d(div) {}
+    __device__ __forceinline__ int quot(int v) const { return d == 1 ? v : (int)__umulhi((uint32_t)v, mul); }
+};
+
+template <typename R, int P, bool INV>
 __device__ __forceinline__ void stockham_pass_fixed(const cx<R>* __restrict__ a, cx<R>* __restrict__ b, int nsig,
-                                                    int L, int ns, const cx<R>* __restrict__ tw2, bool inv) {
-    const int m = L / P;
-    const int tstep = L / (ns * P);
+                                                    const FftPlan& plan, int ns, const cx<R>* __restrict__ tw) {
+    const int m = plan.L / P, LP = plan.stride();
     const int total = nsig * m;
+    const FastDiv dm(m), dns(ns);
     for (int t = threadIdx.x; t < total; t += blockDim.x) {
-        const int sig = t / m;
+        const int sig = dm.quot(t);
         const int j = t - sig * m;
-        const int k = j % ns;
-        const cx<R>* in = a + sig * L;
+        const int q = dns.quot(j);
+        const int k = j - q * ns;
+        const cx<R>* in = a + sig * LP;
         cx<R> v[P];
 #pragma unroll
-        for (int r = 0; r < P; ++r) {
-            cx<R> x = in[j + r * m];
-            if (r > 0 && k > 0) x = cmul(x, twl(tw2, k * r * tstep, inv));
-            v[r] = x;
-        }
-        if (P == 2) bfly2(v);
-        if (P == 3) bfly3(v, inv);
-        if (P == 4) bfly4(v, inv);
-        if (P == 5) bfly5(v, inv);
-        if (P == 8) bfly8(v, inv);
-        cx<R>* out = b + sig * L + (j / ns) * ns * P + k;
+        for (int r = 0; r < P; ++r) v[r] = in[plan.at(j + r * m)];
+        if (ns > 1) {
 #pragma unroll
-        for (int r = 0; r < P; ++r) out[r * ns] = v[r];
+            for (int r = 1; r < P; ++r) {
+                const cx<R> w = tw[r * ns + k];
+                v[r] = INV ? cmulc(v[r], w) : cmul(v[r], w);
+            }
+        }
+        bfly<R, P>(v, INV);
+        cx<R>* out = b + sig * LP;
+        const int o = q * ns * P + k;
+#pragma unroll
+        for (int r = 0; r < P; ++r) out[plan.at(o + r * ns)] = v[r];
     }
 }
 
 // Any prime radix p: one output per thread iteration, direct p-term sum.
-template <typename R>
-__device__ void stockham_pass_generic(const cx<R>* __restrict__ a, cx<R>* __restrict__ b, int nsig, int L, int p,
-                                      int ns, const cx<R>* __restrict__ tw2, bool inv) {
-    const int m = L / p;
-    const int tstep = L / (ns * p);
+template <typename R, bool INV>
+__device__ void stockham_pass_generic(const cx<R>* __restrict__ a, cx<R>* __restrict__ b, int nsig,
+                                      const FftPlan& plan, int p, int ns, const cx<R>* __restrict__ tw,
+                                      const cx<R>* __restrict__ tw2) {
+    const int L = plan.L, m = L / p, LP = plan.stride();
     const int total = nsig * L;
     for (int e = threadIdx.x; e < total; e += blockDim.x) {
         const int sig = e / L;
@@ -164,43 +262,70 @@ __device__ void stockham_pass_generic(const cx<R>* __restrict__ a, cx<R>* __rest
         const int q = rem / m;
         const int j = rem - q * m;
         const int k = j % ns;
-        const cx<R>* in = a + sig * L;
-        cx<R> acc = in[j];
+        const cx<R>* in = a + sig * LP;
+        cx<R> acc = in[plan.at(j)];
+        int qr = 0;   // (q * r) mod p
         for (int r = 1; r < p; ++r) {
-            cx<R> x = in[j + r * m];
-            if (k > 0) x = cmul(x, twl(tw2, k * r * tstep, inv));
-            int qr = (q * r) % p;
-            if (qr) x = cmul(x, twl(tw2, qr * m, inv));
+            cx<R> x = in[plan.at(j + r * m)];
+            if (k > 0) x = INV ? cmulc(x, tw[r * ns + k]) : cmul(x, tw[r * ns + k]);
+            qr += q;
+            if (qr >= p) qr -= p;
+            if (qr) x = cmul(x, twl(tw2, qr * m, INV));
             acc = acc + x;
         }
-        b[sig * L + (j / ns) * ns * p + k + q * ns] = acc;
+        b[sig * LP + plan.at((j / ns) * ns * p + k + q * ns)] = acc;
     }
 }
 
-// Runs the plan on nsig contiguous signals in `a` (scratch `b`, same size).
-// Returns the buffer holding the result.  Ends with __syncthreads().
-template <typename R>
-__device__ cx<R>* fft_smem(cx<R>* a, cx<R>* b, int nsig, const FftPlan& plan, const cx<R>* __restrict__ tw2,
-                           bool inv) {
-    const int L = plan.L;
+// Runs the plan on nsig signals (plan.stride() apart) in `a` (scratch `b`, same
+// size).  `tw` holds the plan's pass tables, `tw2` exp(-2 pi i k / (2L)).  Returns
+// the buffer holding the result.  Ends with __syncthreads().
+template <typename R, bool INV>
+__device__ cx<R>* fft_smem(cx<R>* a, cx<R>* b, int nsig, const FftPlan& plan, const cx<R>* __restrict__ tw,
+                           const cx<R>* __restrict__ tw2) {
     int ns = 1;
     for (int s = 0; s < plan.npass; ++s) {
         const int p = plan.radix[s];
         switch (p) {
-            case 2: stockham_pass_fixed<R, 2>(a, b, nsig, L, ns, tw2, inv); break;
-            case 3: stockham_pass_fixed<R, 3>(a, b, nsig, L, ns, tw2, inv); break;
-            case 4: stockham_pass_fixed<R, 4>(a, b, nsig, L, ns, tw2, inv); break;
-            case 5: stockham_pass_fixed<R, 5>(a, b, nsig, L, ns, tw2, inv); break;
-            case 8: stockham_pass_fixed<R, 8>(a, b, nsig, L, ns, tw2, inv); break;
-            default: stockham_pass_generic<R>(a, b, nsig, L, p, ns, tw2, inv); break;
+            case 2: stockham_pass_fixed<R, 2, INV>(a, b, nsig, plan, ns, tw); break;
+            case 3: stockham_pass_fixed<R, 3, INV>(a, b, nsig, plan, ns, tw); break;
+            case 4: stockham_pass_fixed<R, 4, INV>(a, b, nsig, plan, ns, tw); break;
+            case 5: stockham_pass_fixed<R, 5, INV>(a, b, nsig, plan, ns, tw); break;
+            case 6: stockham_pass_fixed<R, 6, INV>(a, b, nsig, plan, ns, tw); break;
+            case 8: stockham_pass_fixed<R, 8, INV>(a, b, nsig, plan, ns, tw); break;
+            case 10: stockham_pass_fixed<R, 10, INV>(a, b, nsig, plan, ns, tw); break;
+            case 12: stockham_pass_fixed<R, 12, INV>(a, b, nsig, plan, ns, tw); break;
+            case 16: stockham_pass_fixed<R, 16, INV>(a, b, nsig, plan, ns, tw); break;
+            default: stockham_pass_generic<R, INV>(a, b, nsig, plan, p, ns, tw, tw2); break;
         }
         __syncthreads();
         cx<R>* t = a;
         a = b;
         b = t;
+        if (s > 0) tw += p * ns;   // pass 0 has no table
         ns *= p;
     }
     return a;
+}
+
+// Pass tables of a plan: for every pass s >= 1 (radix p, stride ns = product of the
+// earlier radices) W_{ns p}^{k r} at [r * ns + k], r < p, k < ns, pass after pass.
+// Fewer than 2L entries.  Entry e; false past the end.
+__device__ __forceinline__ bool pass_table_entry(const FftPlan& plan, int e, double* c, double* s) {
+    if (plan.npass == 0) return false;
+    int ns = plan.radix[0];
+    for (int q = 1; q < plan.npass; ++q) {
+        const int p = plan.radix[q], n = p * ns;
+        if (e < n) {
+            const long long r = e / ns, k = e % ns;
+            sincospi(2.0 * (double)((k * r) % n) / (double)n, s, c);
+            *s = -*s;
+            return true;
+        }
+        e -= n;
+        ns = n;
+    }
+    return false;
 }
 
 }  // namespace llg

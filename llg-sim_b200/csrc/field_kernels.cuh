@@ -439,9 +439,12 @@ __global__ void __launch_bounds__(256) k_row_forward(const FilmDev* __restrict__
         const R Ms = (R)F.ms;
         const int L = nx;
         const int G = T + (T + 1) / 2;
+        const FftPlan& PL = F.plan_row;
+        const int LP = PL.stride();
         cx<R>* A = sm;
-        cx<R>* B = sm + 2 * G * L;
+        cx<R>* B = sm + 2 * G * LP;
         const cx<R>* __restrict__ tw = reinterpret_cast<const cx<R>*>(F.tw_row);
+        const cx<R>* __restrict__ twg = reinterpret_cast<const cx<R>*>(F.twg_row);
         for (int e = threadIdx.x; e < T * nx; e += blockDim.x) {
             const int r = e / nx, i = e - r * nx, j = j0 + r;
             R v[3] = {(R)0, (R)0, (R)0};
@@ -466,8 +469,8 @@ __global__ void __launch_bounds__(256) k_row_forward(const FilmDev* __restrict__
                 }
             }
             if (do_fft) {
-                A[(2 * r) * L + i] = mkc(Ms * v[0], Ms * v[1]);
-                cx<R>* zp = &A[(2 * (T + r / 2)) * L + i];
+                A[(2 * r) * LP + PL.at(i)] = mkc(Ms * v[0], Ms * v[1]);
+                cx<R>* zp = &A[(2 * (T + r / 2)) * LP + PL.at(i)];
                 if ((r & 1) == 0) {
                     zp->re = Ms * v[2];
                     if (r + 1 >= T) zp->im = (R)0;
@@ -480,10 +483,10 @@ __global__ void __launch_bounds__(256) k_row_forward(const FilmDev* __restrict__
         __syncthreads();
         for (int e = threadIdx.x; e < G * L; e += blockDim.x) {
             const int g = e / L, i = e - g * L;
-            A[(2 * g + 1) * L + i] = cmul(A[(2 * g) * L + i], tw[i]);
+            A[(2 * g + 1) * LP + PL.at(i)] = cmul(A[(2 * g) * LP + PL.at(i)], tw[i]);
         }
         __syncthreads();
-        cx<R>* res = fft_smem<R>(A, B, 2 * G, F.plan_row, tw, false);
+        cx<R>* res = fft_smem<R, false>(A, B, 2 * G, PL, twg, tw);
         cx<R>* __restrict__ X = reinterpret_cast<cx<R>*>(F.X);
         const int K1 = nx + 1;
         const int L2 = 2 * L;
@@ -495,9 +498,9 @@ __global__ void __launch_bounds__(256) k_row_forward(const FilmDev* __restrict__
             int g, half;
             if (c < 2) { g = r; half = c; }
             else { g = T + r / 2; half = r & 1; }
-            const int km = (L2 - k) % L2;
-            cx<R> zk = (k & 1) ? res[(2 * g + 1) * L + (k >> 1)] : res[(2 * g) * L + (k >> 1)];
-            cx<R> zm = (km & 1) ? res[(2 * g + 1) * L + (km >> 1)] : res[(2 * g) * L + (km >> 1)];
+            const int km = k ? L2 - k : 0;
+            cx<R> zk = res[(2 * g + (k & 1)) * LP + PL.at(k >> 1)];
+            cx<R> zm = res[(2 * g + (km & 1)) * LP + PL.at(km >> 1)];
             cx<R> out;
             if (half == 0) out = mkc((R)0.5 * (zk.re + zm.re), (R)0.5 * (zk.im - zm.im));
             else out = mkc((R)0.5 * (zk.im + zm.im), (R)0.5 * (zm.re - zk.re));
@@ -526,33 +529,38 @@ __global__ void __launch_bounds__(256) k_column(const FilmDev* __restrict__ film
         cx<R>* __restrict__ X = reinterpret_cast<cx<R>*>(F.X);
         const r4<R>* __restrict__ Kh = reinterpret_cast<const r4<R>*>(F.Khat) + (size_t)kx * (ny + 1);
         const cx<R>* __restrict__ tw = reinterpret_cast<const cx<R>*>(F.tw_col);
+        const cx<R>* __restrict__ twg = reinterpret_cast<const cx<R>*>(F.twg_col);
+        const FftPlan& PL = F.plan_col;
+        const int LP = PL.stride();
         cx<R>* A = sm;
-        cx<R>* B = sm + 6 * L;
+        cx<R>* B = sm + 6 * LP;
         for (int e = threadIdx.x; e < 3 * L; e += blockDim.x) {
             const int c = e / L, y = e - c * L;
             cx<R> x = X[(c * K1 + kx) * ny + y];
-            A[(2 * c) * L + y] = x;
-            A[(2 * c + 1) * L + y] = cmul(x, tw[y]);
+            A[(2 * c) * LP + PL.at(y)] = x;
+            A[(2 * c + 1) * LP + PL.at(y)] = cmul(x, tw[y]);
         }
         __syncthreads();
-        cx<R>* res = fft_smem<R>(A, B, 6, F.plan_col, tw, false);
+        cx<R>* res = fft_smem<R, false>(A, B, 6, PL, twg, tw);
         for (int e = threadIdx.x; e < 2 * L; e += blockDim.x) {
             const int par = e / L, kk = e - par * L;
             const int ky = 2 * kk + par;
             const int kyf = ky <= ny ? ky : 2 * ny - ky;
             const r4<R> K = Kh[kyf];
             const R kxy = ky <= ny ? K.y : -K.y;
-            cx<R> Mx = res[(0 + par) * L + kk], My = res[(2 + par) * L + kk], Mz = res[(4 + par) * L + kk];
-            res[(0 + par) * L + kk] = mkc(K.x * Mx.re + kxy * My.re, K.x * Mx.im + kxy * My.im);
-            res[(2 + par) * L + kk] = mkc(kxy * Mx.re + K.z * My.re, kxy * Mx.im + K.z * My.im);
-            res[(4 + par) * L + kk] = mkc(K.w * Mz.re, K.w * Mz.im);
+            cx<R>* pr = res + par * LP + PL.at(kk);
+            const cx<R> Mx = pr[0], My = pr[2 * LP], Mz = pr[4 * LP];
+            pr[0] = mkc(K.x * Mx.re + kxy * My.re, K.x * Mx.im + kxy * My.im);
+            pr[2 * LP] = mkc(kxy * Mx.re + K.z * My.re, kxy * Mx.im + K.z * My.im);
+            pr[4 * LP] = mkc(K.w * Mz.re, K.w * Mz.im);
         }
         __syncthreads();
         cx<R>* other = (res == A) ? B : A;
-        cx<R>* res2 = fft_smem<R>(res, other, 6, F.plan_col, tw, true);
+        cx<R>* res2 = fft_smem<R, true>(res, other, 6, PL, twg, tw);
         for (int e = threadIdx.x; e < 3 * L; e += blockDim.x) {
             const int c = e / L, y = e - c * L;
-            X[(c * K1 + kx) * ny + y] = res2[(2 * c) * L + y] + cmulc(res2[(2 * c + 1) * L + y], tw[y]);
+            X[(c * K1 + kx) * ny + y] =
+                res2[(2 * c) * LP + PL.at(y)] + cmulc(res2[(2 * c + 1) * LP + PL.at(y)], tw[y]);
         }
         __syncthreads();
     }
@@ -765,8 +773,11 @@ __global__ void __launch_bounds__(256) k_row_inverse(const FilmDev* __restrict__
         R* D = nullptr;
         if (do_fft) {
             const cx<R>* __restrict__ X = reinterpret_cast<const cx<R>*>(F.X);
+            const cx<R>* __restrict__ twg = reinterpret_cast<const cx<R>*>(F.twg_row);
+            const FftPlan& PL = F.plan_row;
+            const int LP = PL.stride();
             cx<R>* A = sm;
-            cx<R>* B = sm + 2 * G * L;
+            cx<R>* B = sm + 2 * G * LP;
             auto xval = [&](int c, int k, int j) -> cx<R> {
                 if (k <= nx) return X[(c * K1 + k) * ny + j];
                 return conjc(X[(c * K1 + (L2 - k)) * ny + j]);
@@ -778,21 +789,21 @@ __global__ void __launch_bounds__(256) k_row_inverse(const FilmDev* __restrict__
                     cx<R> bx = xval(0, k, j), by = xval(1, k, j);
                     z = mkc(bx.re - by.im, bx.im + by.re);
                 }
-                A[(2 * r + (k & 1)) * L + (k >> 1)] = z;
+                A[(2 * r + (k & 1)) * LP + PL.at(k >> 1)] = z;
             }
             for (int e = threadIdx.x; e < L2 * P; e += blockDim.x) {
                 const int p = e % P, k = e / P;
                 const int ja = j0 + 2 * p, jb = j0 + 2 * p + 1;
                 cx<R> za = (ja < ny) ? xval(2, k, ja) : mkc((R)0, (R)0);
                 cx<R> zb = (2 * p + 1 < T && jb < ny) ? xval(2, k, jb) : mkc((R)0, (R)0);
-                A[(2 * (T + p) + (k & 1)) * L + (k >> 1)] = mkc(za.re - zb.im, za.im + zb.re);
+                A[(2 * (T + p) + (k & 1)) * LP + PL.at(k >> 1)] = mkc(za.re - zb.im, za.im + zb.re);
             }
             __syncthreads();
-            cx<R>* res = fft_smem<R>(A, B, 2 * G, F.plan_row, tw, true);
+            cx<R>* res = fft_smem<R, true>(A, B, 2 * G, PL, twg, tw);
             D = reinterpret_cast<R*>(res == A ? B : A);
             for (int e = threadIdx.x; e < G * L; e += blockDim.x) {
                 const int g = e / L, x = e - g * L;
-                cx<R> z = res[(2 * g) * L + x] + cmulc(res[(2 * g + 1) * L + x], tw[x]);
+                cx<R> z = res[(2 * g) * LP + PL.at(x)] + cmulc(res[(2 * g + 1) * LP + PL.at(x)], tw[x]);
                 if (g < T) {
                     D[(g * 3 + 0) * L + x] = z.re;
                     D[(g * 3 + 1) * L + x] = z.im;

@@ -24,22 +24,31 @@ namespace noalloc {
 
 constexpr size_t kScratchBytes = size_t(32) << 20;  // 32 MiB
 constexpr int kMaxDevices = 64;
+constexpr int kMaxLen = 2048;  // largest nx, ny
 constexpr int kT = 2;          // rows per block
 constexpr int kThreads = 256;
 
 // The shared scratch.  In host code this name is only a stand-in for the
 // device array; kernels receive its device address from cudaGetSymbolAddress.
 static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
+// Pass tables of the two transforms (2 nx and 2 ny entries at most), beside it.
+static __device__ __align__(256) cx<float> g_pass_tables[4 * kMaxLen];
 
 std::mutex g_setup_mutex;
 void* g_scratch_addr[kMaxDevices] = {nullptr};
+void* g_tables_addr[kMaxDevices] = {nullptr};
 
 inline size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
-__global__ void k_na_twiddles(cx<float>* tw_row, int nx, cx<float>* tw_col, int ny) {
+// exp(-2 pi i k / (2L)) of both lengths and the pass tables of both plans.
+__global__ void k_na_twiddles(cx<float>* tw_row, int nx, cx<float>* tw_col, int ny, FftPlan prow, FftPlan pcol,
+                              cx<float>* pass_row, cx<float>* pass_col) {
     const int total = 2 * nx + 2 * ny;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
         const bool row = e < 2 * nx;
+        double pc, ps;
+        if (pass_table_entry(row ? prow : pcol, row ? e : e - 2 * nx, &pc, &ps))
+            (row ? pass_row : pass_col)[row ? e : e - 2 * nx] = mkc((float)pc, (float)ps);
         const int k = row ? e : e - 2 * nx;
         const int L2 = row ? 2 * nx : 2 * ny;
         double s, c;
@@ -51,11 +60,12 @@ __global__ void k_na_twiddles(cx<float>* tw_row, int nx, cx<float>* tw_col, int 
 // Rows j0..j0+kT-1: M = Ms*m, pruned R2C along x, Hermitian bins to X[c][kx][j].
 __global__ void __launch_bounds__(kThreads) k_na_rows_forward(int nx, int ny, float ms, const float* __restrict__ m,
                                                               cx<float>* __restrict__ X,
+                                                              const cx<float>* __restrict__ twp,
                                                               const cx<float>* __restrict__ tw, FftPlan plan) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int L = nx, G = kT + (kT + 1) / 2, n = nx * ny, K1 = nx + 1, L2 = 2 * nx;
+    const int L = nx, G = kT + (kT + 1) / 2, n = nx * ny, K1 = nx + 1, L2 = 2 * nx, LP = plan.stride();
     cx<float>* A = reinterpret_cast<cx<float>*>(smem_raw);
-    cx<float>* B = A + 2 * G * L;
+    cx<float>* B = A + 2 * G * LP;
     const int j0 = blockIdx.x * kT;
     for (int e = threadIdx.x; e < kT * nx; e += blockDim.x) {
         const int r = e / nx, i = e - r * nx, j = j0 + r;
@@ -64,18 +74,18 @@ __global__ void __launch_bounds__(kThreads) k_na_rows_forward(int nx, int ny, fl
             const int idx = j * nx + i;
             v0 = m[idx]; v1 = m[n + idx]; v2 = m[2 * n + idx];
         }
-        A[(2 * r) * L + i] = mkc(ms * v0, ms * v1);
-        cx<float>* zp = &A[(2 * (kT + r / 2)) * L + i];
+        A[(2 * r) * LP + plan.at(i)] = mkc(ms * v0, ms * v1);
+        cx<float>* zp = &A[(2 * (kT + r / 2)) * LP + plan.at(i)];
         if ((r & 1) == 0) zp->re = ms * v2;
         else zp->im = ms * v2;
     }
     __syncthreads();
     for (int e = threadIdx.x; e < G * L; e += blockDim.x) {
         const int g = e / L, i = e - g * L;
-        A[(2 * g + 1) * L + i] = cmul(A[(2 * g) * L + i], tw[i]);
+        A[(2 * g + 1) * LP + plan.at(i)] = cmul(A[(2 * g) * LP + plan.at(i)], tw[i]);
     }
     __syncthreads();
-    cx<float>* res = fft_smem<float>(A, B, 2 * G, plan, tw, false);
+    cx<float>* res = fft_smem<float, false>(A, B, 2 * G, plan, twp, tw);
     for (int e = threadIdx.x; e < 3 * K1 * kT; e += blockDim.x) {
         const int r = e % kT, rest = e / kT;
         const int k = rest % K1, c = rest / K1;
@@ -83,62 +93,84 @@ __global__ void __launch_bounds__(kThreads) k_na_rows_forward(int nx, int ny, fl
         if (j >= ny) continue;
         const int g = c < 2 ? r : kT + r / 2;
         const int half = c < 2 ? c : (r & 1);
-        const int km = (L2 - k) % L2;
-        const cx<float> zk = res[(2 * g + (k & 1)) * L + (k >> 1)];
-        const cx<float> zm = res[(2 * g + (km & 1)) * L + (km >> 1)];
+        const int km = k ? L2 - k : 0;
+        const cx<float> zk = res[(2 * g + (k & 1)) * LP + plan.at(k >> 1)];
+        const cx<float> zm = res[(2 * g + (km & 1)) * LP + plan.at(km >> 1)];
         X[(c * K1 + k) * ny + j] = half == 0 ? mkc(0.5f * (zk.re + zm.re), 0.5f * (zk.im - zm.im))
                                              : mkc(0.5f * (zk.im + zm.im), 0.5f * (zm.re - zk.re));
     }
 }
 
-// One kx column: pruned y transform, kernel multiply, pruned inverse.
-// kp: FP64 kernel planes [4][ny+1][nx+1] (xx, xy, yy, zz), unscaled.
-__global__ void __launch_bounds__(kThreads) k_na_column(int nx, int ny, const double* __restrict__ kp, double scale,
-                                                        cx<float>* __restrict__ X, const cx<float>* __restrict__ tw,
-                                                        FftPlan plan) {
+// NC adjacent kx columns: pruned y transform, kernel multiply, pruned inverse.
+// kp: FP64 kernel planes [4][ny+1][nx+1] (xx, xy, yy, zz), unscaled.  The planes run
+// along kx, so a block of one column reads 8 of every 32-byte sector; with NC = 4
+// columns a block reads whole sectors (columns_per_block: as many as leave two
+// blocks per SM).
+__global__ void __launch_bounds__(kThreads) k_na_column(int nx, int ny, int nc, const double* __restrict__ kp,
+                                                        double scale, cx<float>* __restrict__ X,
+                                                        const cx<float>* __restrict__ twp,
+                                                        const cx<float>* __restrict__ tw, FftPlan plan) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int L = ny, K1 = nx + 1, kx = blockIdx.x;
+    const int L = ny, K1 = nx + 1, kx0 = blockIdx.x * nc, LP = plan.stride();
+    const int nv = min(nc, K1 - kx0);   // columns of this block
     const size_t plane = (size_t)(ny + 1) * (nx + 1);
     cx<float>* A = reinterpret_cast<cx<float>*>(smem_raw);
-    cx<float>* B = A + 6 * L;
-    for (int e = threadIdx.x; e < 3 * L; e += blockDim.x) {
-        const int c = e / L, y = e - c * L;
-        const cx<float> x = X[(c * K1 + kx) * ny + y];
-        A[(2 * c) * L + y] = x;
-        A[(2 * c + 1) * L + y] = cmul(x, tw[y]);
+    cx<float>* B = A + 6 * nc * LP;
+    // signals: column q, component c, parity p at 6 q + 2 c + p
+    for (int e = threadIdx.x; e < 3 * nv * L; e += blockDim.x) {
+        const int cq = e / L, y = e - cq * L, c = cq / nv, q = cq - c * nv;
+        const cx<float> x = X[((size_t)c * K1 + kx0 + q) * ny + y];
+        cx<float>* s = A + (6 * q + 2 * c) * LP + plan.at(y);
+        s[0] = x;
+        s[LP] = cmul(x, tw[y]);
     }
     __syncthreads();
-    cx<float>* res = fft_smem<float>(A, B, 6, plan, tw, false);
-    for (int e = threadIdx.x; e < 2 * L; e += blockDim.x) {
-        const int par = e / L, kk = e - par * L;
-        const int ky = 2 * kk + par;
-        const int kyf = ky <= ny ? ky : 2 * ny - ky;
-        const size_t o = (size_t)kyf * (nx + 1) + kx;
+    cx<float>* res = fft_smem<float, false>(A, B, 6 * nv, plan, twp, tw);
+    // one kernel entry serves both ky and 2 ny - ky (Kxy odd); consecutive threads
+    // take the columns of one ky
+    for (int e = threadIdx.x; e < nv * (ny + 1); e += blockDim.x) {
+        const int kyf = e / nv, q = e - kyf * nv, par = kyf & 1;
+        const size_t o = (size_t)kyf * (nx + 1) + kx0 + q;
         const float kxx = (float)(kp[o] * scale), kyy = (float)(kp[2 * plane + o] * scale);
         const float kzz = (float)(kp[3 * plane + o] * scale);
-        const float kxy = (float)(kp[plane + o] * scale) * (ky <= ny ? 1.f : -1.f);
-        const cx<float> Mx = res[(0 + par) * L + kk], My = res[(2 + par) * L + kk], Mz = res[(4 + par) * L + kk];
-        res[(0 + par) * L + kk] = mkc(kxx * Mx.re + kxy * My.re, kxx * Mx.im + kxy * My.im);
-        res[(2 + par) * L + kk] = mkc(kxy * Mx.re + kyy * My.re, kxy * Mx.im + kyy * My.im);
-        res[(4 + par) * L + kk] = mkc(kzz * Mz.re, kzz * Mz.im);
+        const float kxyf = (float)(kp[plane + o] * scale);
+        for (int h = 0; h < 2; ++h) {
+            const int ky = h ? 2 * ny - kyf : kyf;
+            if (h && (kyf == 0 || kyf == ny)) break;
+            const float kxy = kxyf * (h ? -1.f : 1.f);
+            cx<float>* s = res + (6 * q + par) * LP + plan.at(ky >> 1);
+            const cx<float> Mx = s[0], My = s[2 * LP], Mz = s[4 * LP];
+            s[0] = mkc(kxx * Mx.re + kxy * My.re, kxx * Mx.im + kxy * My.im);
+            s[2 * LP] = mkc(kxy * Mx.re + kyy * My.re, kxy * Mx.im + kyy * My.im);
+            s[4 * LP] = mkc(kzz * Mz.re, kzz * Mz.im);
+        }
     }
     __syncthreads();
     cx<float>* other = res == A ? B : A;
-    cx<float>* res2 = fft_smem<float>(res, other, 6, plan, tw, true);
-    for (int e = threadIdx.x; e < 3 * L; e += blockDim.x) {
-        const int c = e / L, y = e - c * L;
-        X[(c * K1 + kx) * ny + y] = res2[(2 * c) * L + y] + cmulc(res2[(2 * c + 1) * L + y], tw[y]);
+    cx<float>* res2 = fft_smem<float, true>(res, other, 6 * nv, plan, twp, tw);
+    for (int e = threadIdx.x; e < 3 * nv * L; e += blockDim.x) {
+        const int cq = e / L, y = e - cq * L, c = cq / nv, q = cq - c * nv;
+        const cx<float>* s = res2 + (6 * q + 2 * c) * LP + plan.at(y);
+        X[((size_t)c * K1 + kx0 + q) * ny + y] = s[0] + cmulc(s[LP], tw[y]);
     }
+}
+
+int columns_per_block(const FftPlan& plan) {
+    int nc = 1;
+    while (nc < 4 && 12 * (size_t)(2 * nc) * plan.stride() * sizeof(cx<float>) <= 110 * 1024) nc *= 2;
+    return nc;
 }
 
 // Rows: C2R along x keeping nx cells, B_demag to b (SoA FP32).
 __global__ void __launch_bounds__(kThreads) k_na_rows_inverse(int nx, int ny, const cx<float>* __restrict__ X,
+                                                              const cx<float>* __restrict__ twp,
                                                               const cx<float>* __restrict__ tw, FftPlan plan,
                                                               float* __restrict__ b) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int L = nx, K1 = nx + 1, L2 = 2 * nx, G = kT + (kT + 1) / 2, P = (kT + 1) / 2, n = nx * ny;
+    const int LP = plan.stride();
     cx<float>* A = reinterpret_cast<cx<float>*>(smem_raw);
-    cx<float>* B = A + 2 * G * L;
+    cx<float>* B = A + 2 * G * LP;
     const int j0 = blockIdx.x * kT;
     auto xval = [&](int c, int k, int j) -> cx<float> {
         if (k <= nx) return X[(c * K1 + k) * ny + j];
@@ -151,20 +183,20 @@ __global__ void __launch_bounds__(kThreads) k_na_rows_inverse(int nx, int ny, co
             const cx<float> bx = xval(0, k, j), by = xval(1, k, j);
             z = mkc(bx.re - by.im, bx.im + by.re);
         }
-        A[(2 * r + (k & 1)) * L + (k >> 1)] = z;
+        A[(2 * r + (k & 1)) * LP + plan.at(k >> 1)] = z;
     }
     for (int e = threadIdx.x; e < L2 * P; e += blockDim.x) {
         const int p = e % P, k = e / P;
         const int ja = j0 + 2 * p, jb = ja + 1;
         const cx<float> za = ja < ny ? xval(2, k, ja) : mkc(0.f, 0.f);
         const cx<float> zb = (2 * p + 1 < kT && jb < ny) ? xval(2, k, jb) : mkc(0.f, 0.f);
-        A[(2 * (kT + p) + (k & 1)) * L + (k >> 1)] = mkc(za.re - zb.im, za.im + zb.re);
+        A[(2 * (kT + p) + (k & 1)) * LP + plan.at(k >> 1)] = mkc(za.re - zb.im, za.im + zb.re);
     }
     __syncthreads();
-    cx<float>* res = fft_smem<float>(A, B, 2 * G, plan, tw, true);
+    cx<float>* res = fft_smem<float, true>(A, B, 2 * G, plan, twp, tw);
     for (int e = threadIdx.x; e < G * L; e += blockDim.x) {
         const int g = e / L, x = e - g * L;
-        const cx<float> z = res[(2 * g) * L + x] + cmulc(res[(2 * g + 1) * L + x], tw[x]);
+        const cx<float> z = res[(2 * g) * LP + plan.at(x)] + cmulc(res[(2 * g + 1) * LP + plan.at(x)], tw[x]);
         if (g < kT) {
             const int j = j0 + g;
             if (j < ny) {
@@ -185,13 +217,14 @@ __global__ void __launch_bounds__(kThreads) k_na_rows_inverse(int nx, int ny, co
 // cudaDeviceReset the device has a new context: the static array is reloaded,
 // possibly at another address, and the kernels' attributes are back at their
 // defaults), so a cached address never outlives the context it came from.
-int setup(int dev, void** out) {
+int setup(int dev, void** out, void** tables) {
     std::lock_guard<std::mutex> lock(g_setup_mutex);
     const int smax = 227 * 1024;
     if (g_scratch_addr[dev]) {
         cudaFuncAttributes fa;
         if (cudaFuncGetAttributes(&fa, k_na_rows_forward) == cudaSuccess && fa.maxDynamicSharedSizeBytes >= smax) {
             *out = g_scratch_addr[dev];
+            *tables = g_tables_addr[dev];
             return LLG_OK;
         }
         cudaGetLastError();
@@ -200,12 +233,17 @@ int setup(int dev, void** out) {
     void* ptr = nullptr;
     cudaError_t e = cudaGetSymbolAddress(&ptr, g_scratch);
     if (e != cudaSuccess || !ptr) return LLG_ERR_CUDA;
+    void* tab = nullptr;
+    e = cudaGetSymbolAddress(&tab, g_pass_tables);
+    if (e != cudaSuccess || !tab) return LLG_ERR_CUDA;
     if (cudaFuncSetAttribute(k_na_rows_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, smax) != cudaSuccess ||
         cudaFuncSetAttribute(k_na_rows_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, smax) != cudaSuccess ||
         cudaFuncSetAttribute(k_na_column, cudaFuncAttributeMaxDynamicSharedMemorySize, smax) != cudaSuccess)
         return LLG_ERR_CUDA;
     g_scratch_addr[dev] = ptr;
+    g_tables_addr[dev] = tab;
     *out = ptr;
+    *tables = tab;
     return LLG_OK;
 }
 
@@ -233,23 +271,30 @@ extern "C" int llg_demag_field_noalloc(int64_t nx, int64_t ny, double ms, const 
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices)
         return fail(LLG_ERR_CUDA, "no current CUDA device");
     void* base = nullptr;
-    if (setup(dev, &base) != LLG_OK) return fail(LLG_ERR_CUDA, "static scratch set-up failed");
+    void* tables = nullptr;
+    if (setup(dev, &base, &tables) != LLG_OK) return fail(LLG_ERR_CUDA, "static scratch set-up failed");
     unsigned char* b8 = static_cast<unsigned char*>(base);
     cx<float>* X = reinterpret_cast<cx<float>*>(b8);
     cx<float>* tw_row = reinterpret_cast<cx<float>*>(b8 + xbytes);
     cx<float>* tw_col = reinterpret_cast<cx<float>*>(b8 + xbytes + twr);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const int inx = (int)nx, iny = (int)ny;
-    const FftPlan prow = make_plan(inx), pcol = make_plan(iny);
     const int G = kT + (kT + 1) / 2;
-    const size_t smem_row = 4 * (size_t)G * inx * sizeof(cx<float>);
-    const size_t smem_col = 12 * (size_t)iny * sizeof(cx<float>);
+    const FftPlan prow = padded_plan(make_plan(inx), false, 4 * G, 227 * 1024);
+    const FftPlan pcol = padded_plan(make_plan(iny), false, 12, 227 * 1024);
+    cx<float>* pass_row = static_cast<cx<float>*>(tables);
+    cx<float>* pass_col = pass_row + 2 * kMaxLen;
+    const int nc = columns_per_block(pcol);
+    const size_t smem_row = 4 * (size_t)G * prow.stride() * sizeof(cx<float>);
+    const size_t smem_col = 12 * (size_t)nc * pcol.stride() * sizeof(cx<float>);
     const int row_blocks = (iny + kT - 1) / kT;
-    k_na_twiddles<<<(2 * inx + 2 * iny + 255) / 256, 256, 0, s>>>(tw_row, inx, tw_col, iny);
-    k_na_rows_forward<<<row_blocks, kThreads, smem_row, s>>>(inx, iny, (float)ms, m, X, tw_row, prow);
-    k_na_column<<<inx + 1, kThreads, smem_col, s>>>(inx, iny, kernel_planes, 1.0 / (4.0 * (double)nx * (double)ny),
-                                                    X, tw_col, pcol);
-    k_na_rows_inverse<<<row_blocks, kThreads, smem_row, s>>>(inx, iny, X, tw_row, prow, b_out);
+    k_na_twiddles<<<(2 * inx + 2 * iny + 255) / 256, 256, 0, s>>>(tw_row, inx, tw_col, iny, prow, pcol, pass_row,
+                                                                 pass_col);
+    k_na_rows_forward<<<row_blocks, kThreads, smem_row, s>>>(inx, iny, (float)ms, m, X, pass_row, tw_row, prow);
+    k_na_column<<<(inx + nc) / nc, kThreads, smem_col, s>>>(inx, iny, nc, kernel_planes,
+                                                            1.0 / (4.0 * (double)nx * (double)ny), X, pass_col, tw_col,
+                                                            pcol);
+    k_na_rows_inverse<<<row_blocks, kThreads, smem_row, s>>>(inx, iny, X, pass_row, tw_row, prow, b_out);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         std::snprintf(msg, sizeof(msg), "llg_demag_field_noalloc: launch failed: %s", cudaGetErrorString(e));

@@ -393,6 +393,11 @@ struct Engine final : EngineBase {
         if (own_stream) cudaStreamDestroy(own_stream);
     }
 
+    // Signal buffers of a generic row or column block (six signals, two buffers each:
+    // two rows, or one column), and the plan that pads them where they fit.
+    static constexpr int kGenBuffers = 12;
+    static FftPlan generic_plan(const FftPlan& p) { return padded_plan(p, sizeof(R) == 8, kGenBuffers, 200 * 1024); }
+
     template <typename T>
     int dalloc(T** p, size_t bytes) {
         void* q = nullptr;
@@ -472,8 +477,10 @@ struct Engine final : EngineBase {
         size_t smem_row = 0, smem_col = 0;   // generic kernels
         for (int f = 0; f < nf; ++f) {
             if (!m[f].demag) continue;
-            if (!frow[f]) smem_row = std::max(smem_row, 4 * (size_t)3 * g[f].nx * sizeof(cx<R>));
-            if (!fcol[f]) smem_col = std::max(smem_col, 12 * (size_t)g[f].ny * sizeof(cx<R>));
+            if (!frow[f])
+                smem_row = std::max(smem_row, kGenBuffers * generic_plan(make_plan((int)g[f].nx)).stride() * sizeof(cx<R>));
+            if (!fcol[f])
+                smem_col = std::max(smem_col, kGenBuffers * generic_plan(make_plan((int)g[f].ny)).stride() * sizeof(cx<R>));
         }
         const size_t smem_max = 227 * 1024;
         if (smem_row > smem_max || smem_col > smem_max)
@@ -515,8 +522,8 @@ struct Engine final : EngineBase {
             F.half_inv_dy = 0.5 / g[f].dy;
             for (int c = 0; c < 3; ++c) F.u[c] = m[f].easy_axis[c];
             F.demag_mat = m[f].demag ? 1 : 0;
-            F.plan_row = make_plan(nx);
-            F.plan_col = make_plan(ny);
+            F.plan_row = generic_plan(make_plan(nx));
+            F.plan_col = generic_plan(make_plan(ny));
             for (int b = 0; b < 2; ++b) {
                 if ((rc = dalloc(&F.m[b], plane))) return rc;
                 if ((rc = dalloc(&F.ms_buf[b], plane))) return rc;
@@ -548,6 +555,14 @@ struct Engine final : EngineBase {
                 CUDA_TRY(launch_twiddles(tw_col, 2 * ny, sizeof(R) == 8, stream));
                 F.tw_row = tw_row;
                 F.tw_col = tw_col;
+                if (!frow[f]) {
+                    if ((rc = dalloc(&F.twg_row, sizeof(cx<R>) * 2 * (size_t)nx))) return rc;
+                    CUDA_TRY(launch_pass_tables(F.plan_row, F.twg_row, sizeof(R) == 8, stream));
+                }
+                if (!fcol[f]) {
+                    if ((rc = dalloc(&F.twg_col, sizeof(cx<R>) * 2 * (size_t)ny))) return rc;
+                    CUDA_TRY(launch_pass_tables(F.plan_col, F.twg_col, sizeof(R) == 8, stream));
+                }
                 // register-FFT pass tables of every radix plan the film's lengths have
                 const FastCfg& fc = fcs[f];
                 for (int v = 0; v < 2; ++v) {
@@ -919,10 +934,13 @@ struct Engine final : EngineBase {
                 lengths.erase(std::unique(lengths.begin(), lengths.end()), lengths.end());
                 for (int L : lengths) {
                     const std::vector<FftPlan> cand = plan_candidates(L);
-                    auto apply = [&](const FftPlan& pl) {
+                    auto apply = [&](const FftPlan& pl) -> int {
                         for (int f : films[i]) {
                             if ((kind == 0 ? fh[f].nx : fh[f].ny) != L) continue;
-                            (kind == 0 ? fh[f].plan_row : fh[f].plan_col) = pl;
+                            FftPlan& dst = kind == 0 ? fh[f].plan_row : fh[f].plan_col;
+                            void* tab = kind == 0 ? fh[f].twg_row : fh[f].twg_col;
+                            dst = generic_plan(pl);
+                            if (tab) CUDA_TRY(launch_pass_tables(dst, tab, sizeof(R) == 8, stream));
                         }
                         return upload_films();
                     };

@@ -15,11 +15,15 @@ namespace llg {
 
 constexpr int kMaxRadices = 24;
 
-// Radix plan for a shared-memory FFT of length L (product of radices).
+// Radix plan for a shared-memory FFT of length L (product of radices).  Element i
+// of a signal sits at i + (i >> sh): one pad slot per 2^sh elements (sh = 30: none).
 struct FftPlan {
     int L;
     int npass;
+    int sh;
     int radix[kMaxRadices];
+    __host__ __device__ int at(int i) const { return i + (i >> sh); }
+    __host__ __device__ int stride() const { return L + (L >> sh); }   // slots per signal
 };
 
 // Logical buffer ids resolved per film at run time (parity `cur` swaps the
@@ -95,6 +99,8 @@ struct FilmDev {
     const uint8_t* mask;
     const void* tw_row;           // exp(-2 pi i k / (2nx)), k < 2nx
     const void* tw_col;           // exp(-2 pi i k / (2ny)), k < 2ny
+    void* twg_row;                // pass tables of plan_row (generic row kernels)
+    void* twg_col;                // pass tables of plan_col (generic column kernel)
     const void* twp_row[2];       // register-FFT pass tables for length nx, per radix plan (fast path)
     const void* twp_col[2];       // register-FFT pass tables for length ny, per radix plan (fast path)
     double* red_part;             // [nblk][RED_NSLOT] per-block partial reductions
