@@ -23,7 +23,7 @@
 
 #include "../../include/llg_b200.h"
 #include "build_api.h"
-#include "fft_smem.cuh"
+#include "field_kernels.cuh"
 
 namespace llg {
 int ctx_device(const llg_ctx* c);
@@ -39,6 +39,12 @@ struct llg_demag_op {
     llg::cx<double>* twx = nullptr;  // [2 px] exp(-2 pi i k / (2 px)), then [2 px] pass tables of planx
     llg::cx<double>* twy = nullptr;
     llg::FftPlan planx{}, plany{};
+    // open boundaries in both directions: the folded real kernel of the pruned path
+    // (nullptr: general path), and the plans / pass tables of lengths nx and ny
+    llg::r4<double>* Kf = nullptr;   // [nx+1][ny+1] (xx, xy, yy, zz) / (px py)
+    llg::FftPlan plan_nx{}, plan_ny{};
+    llg::cx<double>* tab_nx = nullptr;   // [2 nx] pass tables, then [2 nx] exp(-2 pi i k / (2 nx))
+    llg::cx<double>* tab_ny = nullptr;
 };
 
 namespace {
@@ -102,12 +108,249 @@ __global__ void k_pbc_extract(const cx<double>* __restrict__ M, int nx, int ny, 
     }
 }
 
+// ---------------------------------------------------------------------------
+// Open boundaries in both directions: the same convolution with its zeros and its
+// symmetries left out.  A 2n-point transform whose upper half is zero is two
+// n-point transforms (even and odd bins, the odd input multiplied by W_{2n}^i); two
+// real signals share one complex transform, so only the nx+1 Hermitian bins of x
+// are kept; the kernel spectrum of an open grid is real, even in kx and ky (Kxy odd
+// in ky), so a quarter of it serves all bins; forward transform, kernel product and
+// inverse of a column are one kernel.
+//
+// What bounds it: HBM.  At 1536 x 1536 cells the general path moves about 5.8 GB
+// (its padded planes are 453 MB and cross HBM twice in every pass), this one about
+// 0.8 GB: m in (56 MB), the spectrum [3][nx+1][ny] out and in twice (113 MB each
+// way), the odd-bin half of the columns through scratch (mostly L2), the folded
+// kernel (75 MB), the field out.
+constexpr int kOpenThreads = 256;
+
+// Signal w of a row pair p (rows j0 = 2p, j0+1): w = 0, 1: x + i y of row j0 + w;
+// w = 2: z of row j0 + i z of row j0 + 1.  One signal per block: two transforms
+// in 4 padded buffers, so that two blocks fit an SM at nx = 1536.
+__global__ void __launch_bounds__(kOpenThreads) k_open_rows_forward(int nx, int ny, double ms,
+                                                                    const double* __restrict__ m,
+                                                                    cx<double>* __restrict__ X, llg::FftPlan plan,
+                                                                    const cx<double>* __restrict__ tab,
+                                                                    const cx<double>* __restrict__ tw) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int L = nx, LP = plan.stride(), K1 = nx + 1;
+    cx<double>* A = reinterpret_cast<cx<double>*>(smem_raw);
+    cx<double>* B = A + 2 * LP;
+    const int p = blockIdx.x / 3, w = blockIdx.x - 3 * p;
+    const int ja = w < 2 ? 2 * p + w : 2 * p, jb = 2 * p + 1;
+    if (ja >= ny) return;
+    const bool second = w < 2 || jb < ny;
+    for (int i = threadIdx.x; i < L; i += kOpenThreads) {
+        const double* a = m + ((long long)ja * nx + i) * 3;
+        cx<double> v;
+        if (w < 2) v = mkc(ms * a[0], ms * a[1]);
+        else v = mkc(ms * a[2], second ? ms * m[((long long)jb * nx + i) * 3 + 2] : 0.0);
+        A[plan.at(i)] = v;
+        A[LP + plan.at(i)] = llg::cmul(v, tw[i]);
+    }
+    __syncthreads();
+    const cx<double>* res = llg::fft_smem<double, false>(A, B, 2, plan, tab, tw);
+    const int c0 = w < 2 ? 0 : 2;
+    cx<double>* xa = X + (long long)c0 * K1 * ny + ja;
+    cx<double>* xb = w < 2 ? X + (long long)K1 * ny + ja : X + (long long)2 * K1 * ny + jb;
+    for (int k = threadIdx.x; k < K1; k += kOpenThreads) {
+        const int km = k ? 2 * L - k : 0;
+        const cx<double> zk = res[(k & 1) * LP + plan.at(k >> 1)], zm = res[(km & 1) * LP + plan.at(km >> 1)];
+        xa[(long long)k * ny] = mkc(0.5 * (zk.re + zm.re), 0.5 * (zk.im - zm.im));
+        if (second) xb[(long long)k * ny] = mkc(0.5 * (zk.im + zm.im), 0.5 * (zm.re - zk.re));
+    }
+}
+
+// One kx column: the odd and then the even ky bins of the three components (six
+// padded buffers at a time, so that ny = 2048 fits), product with the folded kernel
+// and inverse.  The odd half waits in O, the even half adds it and replaces X.
+__global__ void __launch_bounds__(kOpenThreads) k_open_column(int nx, int ny, const llg::r4<double>* __restrict__ Kf,
+                                                              cx<double>* __restrict__ X, cx<double>* __restrict__ O,
+                                                              llg::FftPlan plan, const cx<double>* __restrict__ tab,
+                                                              const cx<double>* __restrict__ tw) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int L = ny, LP = plan.stride(), kx = blockIdx.x;
+    const long long plane = (long long)(nx + 1) * ny, col = (long long)kx * ny;
+    cx<double>* A = reinterpret_cast<cx<double>*>(smem_raw);
+    cx<double>* B = A + 3 * LP;
+    const llg::r4<double>* kc = Kf + (long long)kx * (ny + 1);
+    for (int par = 1; par >= 0; --par) {
+        for (int c = 0; c < 3; ++c)
+            for (int y = threadIdx.x; y < L; y += kOpenThreads) {
+                const cx<double> x = X[c * plane + col + y];
+                A[c * LP + plan.at(y)] = par ? llg::cmul(x, tw[y]) : x;
+            }
+        __syncthreads();
+        cx<double>* res = llg::fft_smem<double, false>(A, B, 3, plan, tab, tw);
+        for (int kk = threadIdx.x; kk < L; kk += kOpenThreads) {
+            const int ky = 2 * kk + par;
+            const llg::r4<double> K = kc[ky <= ny ? ky : 2 * ny - ky];
+            const double kxy = ky <= ny ? K.y : -K.y;
+            cx<double>* s = res + plan.at(kk);
+            const cx<double> Mx = s[0], My = s[LP], Mz = s[2 * LP];
+            s[0] = mkc(K.x * Mx.re + kxy * My.re, K.x * Mx.im + kxy * My.im);
+            s[LP] = mkc(kxy * Mx.re + K.z * My.re, kxy * Mx.im + K.z * My.im);
+            s[2 * LP] = mkc(K.w * Mz.re, K.w * Mz.im);
+        }
+        __syncthreads();
+        const cx<double>* r2 = llg::fft_smem<double, true>(res, res == A ? B : A, 3, plan, tab, tw);
+        for (int c = 0; c < 3; ++c)
+            for (int y = threadIdx.x; y < L; y += kOpenThreads) {
+                const cx<double> v = r2[c * LP + plan.at(y)];
+                const long long o = c * plane + col + y;   // every y by the same thread in both rounds
+                if (par) O[o] = llg::cmulc(v, tw[y]);
+                else X[o] = v + O[o];
+            }
+        __syncthreads();
+    }
+}
+
+// Signals as in the forward pass; the field goes to the AoS output.
+__global__ void __launch_bounds__(kOpenThreads) k_open_rows_inverse(int nx, int ny, const cx<double>* __restrict__ X,
+                                                                    llg::FftPlan plan,
+                                                                    const cx<double>* __restrict__ tab,
+                                                                    const cx<double>* __restrict__ tw,
+                                                                    double* __restrict__ b) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int L = nx, LP = plan.stride(), K1 = nx + 1;
+    cx<double>* A = reinterpret_cast<cx<double>*>(smem_raw);
+    cx<double>* B = A + 2 * LP;
+    const int p = blockIdx.x / 3, w = blockIdx.x - 3 * p;
+    const int ja = w < 2 ? 2 * p + w : 2 * p, jb = 2 * p + 1;
+    if (ja >= ny) return;
+    const bool second = w < 2 || jb < ny;
+    const int c0 = w < 2 ? 0 : 2;
+    const cx<double>* xa = X + (long long)c0 * K1 * ny + ja;
+    const cx<double>* xb = w < 2 ? X + (long long)K1 * ny + ja : X + (long long)2 * K1 * ny + jb;
+    for (int k = threadIdx.x; k < K1; k += kOpenThreads) {
+        const cx<double> u = xa[(long long)k * ny];
+        const cx<double> v = second ? xb[(long long)k * ny] : mkc(0.0, 0.0);
+        A[(k & 1) * LP + plan.at(k >> 1)] = mkc(u.re - v.im, u.im + v.re);
+        const int km = 2 * L - k;   // conjugate bins: conj(u) + i conj(v)
+        if (k > 0 && k < L) A[(km & 1) * LP + plan.at(km >> 1)] = mkc(u.re + v.im, v.re - u.im);
+    }
+    __syncthreads();
+    const cx<double>* res = llg::fft_smem<double, true>(A, B, 2, plan, tab, tw);
+    for (int i = threadIdx.x; i < L; i += kOpenThreads) {
+        const cx<double> z = res[plan.at(i)] + llg::cmulc(res[LP + plan.at(i)], tw[i]);
+        double* o = b + ((long long)ja * nx + i) * 3;
+        if (w < 2) {
+            o[0] = z.re;
+            o[1] = z.im;
+        } else {
+            o[2] = z.re;
+            if (second) b[((long long)jb * nx + i) * 3 + 2] = z.im;
+        }
+    }
+}
+
+// Folded kernel of an open grid, scaled by 1/(px py), and in dev[0] the largest
+// deviation of the planes from being real and even (Kxy odd in ky and in kx), in
+// dev[1] the largest magnitude (bit patterns of non-negative doubles order like the
+// values; a NaN ends up above every number).
+__global__ void k_open_fold(const cx<double>* __restrict__ K, int nx, int ny, double scale,
+                            llg::r4<double>* __restrict__ Kf, unsigned long long* __restrict__ dev) {
+    const int px = 2 * nx, py = 2 * ny;
+    const long long np = (long long)px * py;
+    double worst = 0.0, big = 0.0;
+    bool nan = false;
+    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < (long long)(nx + 1) * (ny + 1);
+         e += (long long)gridDim.x * blockDim.x) {
+        const int kx = (int)(e / (ny + 1)), ky = (int)(e % (ny + 1));
+        const int mx = kx ? px - kx : 0, my = ky ? py - ky : 0;
+        double v[4];
+        for (int c = 0; c < 4; ++c) {
+            const cx<double>* P = K + c * np;
+            const double sg = c == 1 ? -1.0 : 1.0;
+            const cx<double> a = P[(long long)ky * px + kx], q[3] = {P[(long long)ky * px + mx],
+                                                                    P[(long long)my * px + kx],
+                                                                    P[(long long)my * px + mx]};
+            v[c] = a.re;
+            const double d[7] = {a.im, q[0].re - sg * a.re, q[0].im, q[1].re - sg * a.re, q[1].im, q[2].re - a.re,
+                                 q[2].im};
+            for (int t = 0; t < 7; ++t) {
+                nan |= d[t] != d[t];
+                worst = fmax(worst, fabs(d[t]));
+            }
+            big = fmax(big, fabs(a.re));
+        }
+        llg::r4<double> o;
+        o.x = v[0] * scale;
+        o.y = v[1] * scale;
+        o.z = v[2] * scale;
+        o.w = v[3] * scale;
+        Kf[e] = o;
+    }
+    atomicMax(dev, nan ? 0x7ff8000000000000ull : (unsigned long long)__double_as_longlong(worst));
+    atomicMax(dev + 1, (unsigned long long)__double_as_longlong(big));
+}
+
+// Sets the pruned path of an open operator up.  The planes qualify when they are
+// real and even to kOpenTol of their largest value: a built kernel is to a few
+// 1e-16, and dropping what is below 1e-13 changes the field by less than the
+// transforms' own rounding.  A cache file may hold any planes: others keep the
+// general path, and so does an operator for which the extra buffers do not fit.
+constexpr double kOpenTol = 1e-13;
+void open_path_create(llg_demag_op* op) {
+    const size_t nk = (size_t)(op->nx + 1) * (op->ny + 1);
+    unsigned long long* dev = nullptr;
+    unsigned long long h[2] = {~0ull, 0};
+    bool ok = cudaMalloc(&op->Kf, nk * sizeof(llg::r4<double>)) == cudaSuccess &&
+              cudaMalloc(&op->tab_nx, 4 * (size_t)op->nx * sizeof(cx<double>)) == cudaSuccess &&
+              cudaMalloc(&op->tab_ny, 4 * (size_t)op->ny * sizeof(cx<double>)) == cudaSuccess &&
+              cudaMalloc(&dev, sizeof(h)) == cudaSuccess && cudaMemset(dev, 0, sizeof(h)) == cudaSuccess;
+    if (ok) {
+        k_open_fold<<<1184, 256>>>(op->K, op->nx, op->ny, 1.0 / ((double)op->px * op->py), op->Kf, dev);
+        ok = cudaGetLastError() == cudaSuccess && cudaMemcpy(h, dev, sizeof(h), cudaMemcpyDeviceToHost) == cudaSuccess;
+    }
+    if (ok) {
+        double d[2];
+        std::memcpy(d, h, sizeof(d));
+        ok = d[0] <= kOpenTol * d[1];
+    }
+    constexpr size_t kMax = 227 * 1024;
+    op->plan_nx = llg::padded_plan(llg::make_plan(op->nx), true, 4, kMax);
+    op->plan_ny = llg::padded_plan(llg::make_plan(op->ny), true, 6, kMax);
+    auto attr = [&](const void* f) {
+        return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax) == cudaSuccess;
+    };
+    ok = ok && attr((const void*)k_open_rows_forward) && attr((const void*)k_open_column) &&
+         attr((const void*)k_open_rows_inverse) &&
+         llg::launch_pass_tables(op->plan_nx, op->tab_nx, true, 0) == cudaSuccess &&
+         llg::launch_pass_tables(op->plan_ny, op->tab_ny, true, 0) == cudaSuccess &&
+         llg::launch_twiddles(op->tab_nx + 2 * op->nx, 2 * op->nx, true, 0) == cudaSuccess &&
+         llg::launch_twiddles(op->tab_ny + 2 * op->ny, 2 * op->ny, true, 0) == cudaSuccess;
+    if (dev) cudaFree(dev);
+    if (!ok) {
+        cudaGetLastError();
+        for (void* p : {(void*)op->Kf, (void*)op->tab_nx, (void*)op->tab_ny})
+            if (p) cudaFree(p);
+        op->Kf = nullptr;
+        op->tab_nx = op->tab_ny = nullptr;
+    }
+}
+
 }  // namespace
 
 namespace llg {
 
 int demag_op_apply_device(llg_demag_op* op, double ms, const double* d_m_aos, double* d_b_aos, cudaStream_t s) {
     const long long np = (long long)op->px * op->py;
+    if (op->Kf) {
+        cx<double>* X = op->M;
+        cx<double>* O = op->M + 3 * (long long)(op->nx + 1) * op->ny;   // 6 (nx+1) ny <= 3 px py = 12 nx ny
+        const cx<double>* twx = op->tab_nx + 2 * op->nx;
+        const cx<double>* twy = op->tab_ny + 2 * op->ny;
+        const size_t row = 4 * (size_t)op->plan_nx.stride() * sizeof(cx<double>);
+        const size_t col = 6 * (size_t)op->plan_ny.stride() * sizeof(cx<double>);
+        const int rows = 3 * ((op->ny + 1) / 2);
+        k_open_rows_forward<<<rows, kOpenThreads, row, s>>>(op->nx, op->ny, ms, d_m_aos, X, op->plan_nx, op->tab_nx,
+                                                            twx);
+        k_open_column<<<op->nx + 1, kOpenThreads, col, s>>>(op->nx, op->ny, op->Kf, X, O, op->plan_ny, op->tab_ny, twy);
+        k_open_rows_inverse<<<rows, kOpenThreads, row, s>>>(op->nx, op->ny, X, op->plan_nx, op->tab_nx, twx, d_b_aos);
+        PBC_TRY(cudaGetLastError());
+        return LLG_OK;
+    }
     k_pbc_pack<<<1184, 256, 0, s>>>(d_m_aos, op->nx, op->ny, op->px, op->py, ms, op->M);
     PBC_TRY(cudaGetLastError());
     PBC_TRY(llg::launch_fft_strided<double>(op->M, op->planx, op->twx + 2 * op->px, op->twx, 1, op->py, op->px, 3, np, false, s));
@@ -233,6 +476,9 @@ void destroy(llg_demag_op* op) {
     cudaFree(op->stage);
     cudaFree(op->twx);
     cudaFree(op->twy);
+    cudaFree(op->Kf);
+    cudaFree(op->tab_nx);
+    cudaFree(op->tab_ny);
     delete op;
 }
 
@@ -301,6 +547,7 @@ int llg_demag_op_create(llg_ctx* ctx, const llg_grid* g, int64_t pbc_x, int64_t 
             // like the reference, a cache that cannot be written is not an error
         }
     }
+    if (pbc_x == 0 && pbc_y == 0) open_path_create(op);
     if (cudaDeviceSynchronize() != cudaSuccess) return bail(fail(LLG_ERR_CUDA, "demag operator set-up"));
     if (loaded) *loaded = hit ? 1 : 0;
     *out = op;
