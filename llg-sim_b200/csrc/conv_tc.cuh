@@ -319,6 +319,7 @@ __device__ __forceinline__ void conv_epilogue(const float (&acc)[NCOL], long lon
 // while the tensor cores work on tile k.  The MMA sequence of a tile is the one
 // of k_conv3x3_tc (same operands, same order), so both kernels give the same bits.
 constexpr int kHaloW = 256;
+constexpr int kPipeThreads = 2 * kTile;   // two threads per cell build the im2col rows
 constexpr int kHaloCells = kTile + 2 * kHaloW + 2;
 
 template <int CIN>
@@ -327,8 +328,8 @@ __host__ __device__ constexpr size_t conv_pipe_smem_bytes(int npad) {
 }
 
 template <int NCOL, int EPI, typename R, int CIN>
-__global__ void __launch_bounds__(kTile) k_conv3x3_pipe(const __nv_bfloat16* __restrict__ x, int nimg, int H, int W,
-                                                        Layer L, __nv_bfloat16* __restrict__ y,
+__global__ void __launch_bounds__(kPipeThreads) k_conv3x3_pipe(const __nv_bfloat16* __restrict__ x, int nimg, int H,
+                                                               int W, Layer L, __nv_bfloat16* __restrict__ y,
                                                         R* __restrict__ m_out, float* __restrict__ out32,
                                                         const uint8_t* __restrict__ mask,
                                                         const __nv_bfloat16* __restrict__ act, int* err,
@@ -355,7 +356,7 @@ __global__ void __launch_bounds__(kTile) k_conv3x3_pipe(const __nv_bfloat16* __r
         mbar_init_fence();
     }
     // weights, K-major core matrices
-    for (int c = t; c < L.npad * (K / 8); c += kTile) {
+    for (int c = t; c < L.npad * (K / 8); c += kPipeThreads) {
         const int n = c / (K / 8), kc = c - n * (K / 8);
         const uint4 v = reinterpret_cast<const uint4*>(L.w + (size_t)n * K)[kc];
         *reinterpret_cast<uint4*>(Bs + (size_t)(n >> 3) * sbo + (size_t)kc * 128 + (size_t)(n & 7) * 16) = v;
@@ -414,25 +415,33 @@ __global__ void __launch_bounds__(kTile) k_conv3x3_pipe(const __nv_bfloat16* __r
             }
             halo_pending[hb ^ 1] = ((k + 1) >> 1) & 1;
         }
-        // im2col row of cell p from the halo (zero outside the image)
+        // im2col row of cell p from the halo (zero outside the image): threads t and
+        // t + 128 share a cell, 4 taps and 5 taps (the first 128 also run the epilogue).
+        // Lanes start at different 8-channel groups, so the eight lanes of a 16-byte
+        // access phase, whose cells are CIN * 2 bytes apart, cover all banks.
         {
             long long lo, cnt;
             halo_range(tile, &lo, &cnt);
             const unsigned char* hsrc = Hs + (size_t)hb * kHaloCells * CIN * 2;
-            const long long p = tile * kTile + t;
+            const int cell = t & (kTile - 1), half = t >> 7;
+            const long long p = tile * kTile + cell;
             const bool valid = p < total;
             const int img = valid ? (int)(p / hw) : 0;
             const int rem = valid ? (int)(p - (long long)img * hw) : 0;
             const int yy = rem / W, xx = rem - (rem / W) * W;
-            unsigned char* arow = As + (size_t)(t >> 3) * sbo + (size_t)(t & 7) * 16;
+            unsigned char* arow = As + (size_t)(cell >> 3) * sbo + (size_t)(cell & 7) * 16;
+            const int rot = CIN == 32 ? cell >> 1 : cell >> 2;
 #pragma unroll
-            for (int tap = 0; tap < 9; ++tap) {
-                const int sy = yy + tap / 3 - 1, sx = xx + tap % 3 - 1;
-                const bool in = valid && sy >= 0 && sy < H && sx >= 0 && sx < W;
-                const long long q = p + (long long)(tap / 3 - 1) * W + (tap % 3 - 1);
-                const uint4* src = reinterpret_cast<const uint4*>(hsrc + (in ? (q - lo) : 0) * CIN * 2);
+            for (int q = 0; q < 5; ++q) {
+                const int tap = half ? 4 + q : q;
+                if (!half && q == 4) continue;
+                const int dy = tap / 3 - 1, dx = tap - (dy + 1) * 3 - 1;
+                const bool in = valid && yy + dy >= 0 && yy + dy < H && xx + dx >= 0 && xx + dx < W;
+                const long long src_cell = in ? p + (long long)dy * W + dx - lo : 0;
+                const uint4* src = reinterpret_cast<const uint4*>(hsrc + src_cell * CIN * 2);
 #pragma unroll
-                for (int g = 0; g < CIN / 8; ++g) {
+                for (int gi = 0; gi < CIN / 8; ++gi) {
+                    const int g = (gi + rot) & (CIN / 8 - 1);
                     const uint4 v = in ? src[g] : make_uint4(0u, 0u, 0u, 0u);
                     *reinterpret_cast<uint4*>(arow + (size_t)((tap * CIN + g * 8) >> 3) * 128) = v;
                 }
@@ -452,7 +461,7 @@ __global__ void __launch_bounds__(kTile) k_conv3x3_pipe(const __nv_bfloat16* __r
         }
         mma_pending = k & 1;
         // epilogue of the previous tile while the tensor cores work on this one
-        if (prev >= 0) {
+        if (prev >= 0 && t < kTile) {
             float acc[NCOL];
             tmem_ld<NCOL>(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(hb ^ 1) * kAcc, acc);
             const long long p = prev * kTile + t;
@@ -463,8 +472,8 @@ __global__ void __launch_bounds__(kTile) k_conv3x3_pipe(const __nv_bfloat16* __r
     if (ok && mma_pending >= 0) {
         ok = mbar_wait_n(&bar_mma, (uint32_t)mma_pending, spin);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (ok) {
-            mma_pending = -1;
+        if (ok) mma_pending = -1;
+        if (ok && t < kTile) {
             float acc[NCOL];
             tmem_ld<NCOL>(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((k - 1) & 1) * kAcc, acc);
             const long long p = prev * kTile + t;
@@ -509,14 +518,14 @@ cudaError_t conv_launch(const __nv_bfloat16* x, int nimg, int H, int W, const La
             cudaError_t e = cudaFuncSetAttribute(k_conv3x3_pipe<NCOL, EPI, R, 32>,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (e != cudaSuccess) return e;
-            k_conv3x3_pipe<NCOL, EPI, R, 32><<<grid, kTile, smem, s>>>(x, nimg, H, W, L, y, m_out, out32, mask, act,
+            k_conv3x3_pipe<NCOL, EPI, R, 32><<<grid, kPipeThreads, smem, s>>>(x, nimg, H, W, L, y, m_out, out32, mask, act,
                                                                         err, spin);
         } else {
             const size_t smem = conv_pipe_smem_bytes<16>(L.npad);
             cudaError_t e = cudaFuncSetAttribute(k_conv3x3_pipe<NCOL, EPI, R, 16>,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (e != cudaSuccess) return e;
-            k_conv3x3_pipe<NCOL, EPI, R, 16><<<grid, kTile, smem, s>>>(x, nimg, H, W, L, y, m_out, out32, mask, act,
+            k_conv3x3_pipe<NCOL, EPI, R, 16><<<grid, kPipeThreads, smem, s>>>(x, nimg, H, W, L, y, m_out, out32, mask, act,
                                                                         err, spin);
         }
         return cudaGetLastError();

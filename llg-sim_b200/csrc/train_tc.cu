@@ -36,11 +36,15 @@ constexpr int kRedThreads = 256;
 // Both operands MN-major, no swizzle: element (mn, k) of a tile sits at byte
 // (k / 8) * LBO + (mn / 8) * SBO + (k % 8) * 16 + (mn % 8) * 2 with SBO = 128
 // (the 8-channel groups of one cell group are adjacent) and LBO = (MN / 8) * 128.
-template <int NT, int NN>
-__global__ void __launch_bounds__(128) k_wgrad_tc(const __nv_bfloat16* __restrict__ x, int cin,
+// Measured at 16 films of 128 x 128 cells, 32 channels: 127 us per layer with one
+// 64-bit division per 16-byte chunk of the gather (a thread's time went into index
+// arithmetic).
+template <int CIN, int NN>
+__global__ void __launch_bounds__(128) k_wgrad_tc(const __nv_bfloat16* __restrict__ x,
                                                   const __nv_bfloat16* __restrict__ g, int nimg, int H, int W,
                                                   long long cells_per_cta, float* __restrict__ part, int* err,
                                                   long long spin) {
+    constexpr int GROUPS = CIN / 8, NT = (9 * CIN + kTile - 1) / kTile;
     constexpr int A_TILE = kTile * kWgKC * 2;           // bytes per M tile and chunk
     constexpr uint32_t A_LBO = (kTile / 8) * 128, B_LBO = (NN / 8) * 128;
     constexpr uint32_t kCols = NT * NN <= 32 ? 32 : NT * NN <= 64 ? 64 : NT * NN <= 128 ? 128 : 256;
@@ -53,7 +57,7 @@ __global__ void __launch_bounds__(128) k_wgrad_tc(const __nv_bfloat16* __restric
     const long long hw = (long long)H * W, total = (long long)nimg * hw;
     const long long c_begin = (long long)blockIdx.x * cells_per_cta;
     const long long c_end = min(total, c_begin + cells_per_cta);
-    const int M = 9 * cin, groups = cin / 8;
+    constexpr int M = 9 * CIN;
 
     if (warp == 0) tmem_alloc(&tmem_base, kCols);
     if (t == 0) {
@@ -68,20 +72,32 @@ __global__ void __launch_bounds__(128) k_wgrad_tc(const __nv_bfloat16* __restric
     uint32_t phase = 0;
     bool ok = true, first = true;
     for (long long c0 = c_begin; c0 < c_end; c0 += kWgKC) {
-        // A: (cell k, tap, 8-channel group) -> one 16-byte chunk
-        for (int e = t; e < kWgKC * 9 * groups; e += 128) {
-            const int k = e / (9 * groups), r = e - k * (9 * groups), tap = r / groups, cg = r - tap * groups;
+        // A: (cell k, tap, 8-channel group) -> one 16-byte chunk.  Thread t takes cell
+        // t % 64 and half of the groups: the image position is formed once per chunk, a
+        // thread's groups of a tap are one 32-byte sector (16 bytes for 16 channels), and
+        // eight neighbouring lanes store the 128 consecutive bytes of a core matrix.
+        {
+            const int k = t & (kWgKC - 1), half = t >> 6;
             const long long p = c0 + k;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (p < c_end) {
-                const int img = (int)(p / hw);
-                const int rem = (int)(p - (long long)img * hw);
-                const int sy = rem / W + tap / 3 - 1, sx = rem % W + tap % 3 - 1;
-                if (sy >= 0 && sy < H && sx >= 0 && sx < W)
-                    v = reinterpret_cast<const uint4*>(x + (((long long)img * H + sy) * W + sx) * cin)[cg];
+            const bool valid = p < c_end;
+            const unsigned pu = valid ? (unsigned)p : 0u;   // fewer than 2^28 cells
+            const unsigned rem = pu % (unsigned)hw;
+            const int yy = (int)(rem / (unsigned)W), xx = (int)(rem % (unsigned)W);
+            const __nv_bfloat16* xc = x + (long long)pu * CIN;
+            unsigned char* ak = As + (k >> 3) * A_LBO + (k & 7) * 16;
+#pragma unroll
+            for (int tap = 0; tap < 9; ++tap) {
+                const int dy = tap / 3 - 1, dx = tap % 3 - 1;
+                const bool in = valid && yy + dy >= 0 && yy + dy < H && xx + dx >= 0 && xx + dx < W;
+                const uint4* src = reinterpret_cast<const uint4*>(xc + ((long long)dy * W + dx) * CIN);
+#pragma unroll
+                for (int q = 0; q < GROUPS / 2; ++q) {
+                    const int cg = half * (GROUPS / 2) + q;
+                    const uint4 v = in ? src[cg] : make_uint4(0u, 0u, 0u, 0u);
+                    const int m = tap * CIN + cg * 8;
+                    *reinterpret_cast<uint4*>(ak + (m / kTile) * A_TILE + ((m % kTile) >> 3) * 128) = v;
+                }
             }
-            const int m = tap * cin + cg * 8, tile = m / kTile, mm = m - tile * kTile;
-            *reinterpret_cast<uint4*>(As + tile * A_TILE + (k >> 3) * A_LBO + (mm >> 3) * 128 + (k & 7) * 16) = v;
         }
         // B: (cell k, 8-channel group of the output gradient)
         for (int e = t; e < kWgKC * (NN / 8); e += 128) {
@@ -192,54 +208,87 @@ __global__ void __launch_bounds__(kRedThreads) k_cos_loss(const float* __restric
     }
 }
 
-// Sum of the loss partials in block order: red[0] = mean loss, red[1] = 1 / inside cells.
+// Sum of the loss partials: lane l of one warp adds blocks l, l + 32, ... in order,
+// then a fixed butterfly (deterministic).  red[0] = mean loss, red[1] = 1 / inside
+// cells.  One thread walking the 592 partials took 41 us of dependent loads.
 __global__ void k_loss_finalize(const double* __restrict__ part, int nblocks, double* __restrict__ red) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
     double l = 0.0, c = 0.0;
-    for (int b = 0; b < nblocks; ++b) {
+    for (int b = threadIdx.x; b < nblocks; b += 32) {
         l += part[2 * b];
         c += part[2 * b + 1];
     }
-    red[0] = c > 0.0 ? l / c : 0.0;
-    red[1] = c > 0.0 ? 1.0 / c : 0.0;
-}
-
-// Per-block column sums of g [P][NN] (bias gradient), FP32 partials [block][NN].
-template <int NN>
-__global__ void __launch_bounds__(kRedThreads) k_bias_part(const __nv_bfloat16* __restrict__ g, long long total,
-                                                           float* __restrict__ part) {
-    __shared__ float s[kRedThreads / NN][NN];
-    constexpr int ROWS = kRedThreads / NN;
-    const int c = threadIdx.x % NN, r = threadIdx.x / NN;
-    float acc = 0.0f;
-    for (long long p = (long long)blockIdx.x * ROWS + r; p < total; p += (long long)gridDim.x * ROWS)
-        acc += __bfloat162float(g[p * NN + c]);
-    s[r][c] = acc;
-    __syncthreads();
-    if (r == 0) {
-        float v = 0.0f;
-        for (int q = 0; q < ROWS; ++q) v += s[q][c];
-        part[blockIdx.x * NN + c] = v;
+    for (int o = 16; o > 0; o >>= 1) {
+        l += __shfl_xor_sync(0xffffffffu, l, o);
+        c += __shfl_xor_sync(0xffffffffu, c, o);
+    }
+    if (threadIdx.x == 0) {
+        red[0] = c > 0.0 ? l / c : 0.0;
+        red[1] = c > 0.0 ? 1.0 / c : 0.0;
     }
 }
 
-// Gradient of one layer in the flat parameter layout (W[cout][3][3][cin_real] then
-// b[cout_real]) from the CTA partials, summed in CTA order.
-__global__ void k_grad_reduce(const float* __restrict__ wpart, int nwb, int rows_per_cta, int nn,
-                              const float* __restrict__ bpart, int nbb, int cin_pad, int cin_real, int cout_real,
-                              float* __restrict__ grad) {
-    const int nw = cout_real * 9 * cin_real;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nw + cout_real; i += gridDim.x * blockDim.x) {
-        float s = 0.0f;
-        if (i < nw) {
-            const int co = i / (9 * cin_real), r = i - co * 9 * cin_real, tap = r / cin_real, ci = r - tap * cin_real;
-            const int m = tap * cin_pad + ci;
-            for (int b = 0; b < nwb; ++b) s += wpart[((size_t)b * rows_per_cta + m) * nn + co];
-        } else {
-            const int co = i - nw;
-            for (int b = 0; b < nbb; ++b) s += bpart[b * nn + co];
+// Per-block column sums of g [P][NN] (bias gradient), FP32 partials [block][NN].  A
+// thread adds 8 channels (one 16-byte load) of every ROWS-th row; bound by reading g.
+template <int NN>
+__global__ void __launch_bounds__(kRedThreads) k_bias_part(const __nv_bfloat16* __restrict__ g, long long total,
+                                                           float* __restrict__ part) {
+    constexpr int LANES = NN / 8, ROWS = kRedThreads / LANES;
+    __shared__ float s[ROWS][NN + 1];
+    const int c = threadIdx.x % LANES, r = threadIdx.x / LANES;
+    float acc[8] = {};
+    for (long long p = (long long)blockIdx.x * ROWS + r; p < total; p += (long long)gridDim.x * ROWS) {
+        const uint4 v = reinterpret_cast<const uint4*>(g + p * NN)[c];
+        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float2 f = __bfloat1622float2(h[q]);
+            acc[2 * q] += f.x;
+            acc[2 * q + 1] += f.y;
         }
-        grad[i] = s;
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) s[r][c * 8 + q] = acc[q];
+    __syncthreads();
+    for (int o = ROWS / 2; o > 0; o >>= 1) {
+        for (int e = threadIdx.x; e < o * NN; e += kRedThreads) s[e / NN][e % NN] += s[e / NN + o][e % NN];
+        __syncthreads();
+    }
+    if (threadIdx.x < NN) part[blockIdx.x * NN + threadIdx.x] = s[0][threadIdx.x];
+}
+
+// Gradient of one layer in the flat parameter layout (W[cout][3][3][cin_real] then
+// b[cout_real]) from the CTA partials.  Block = one (tap, input channel), the last
+// one the bias: a row of NN output channels is contiguous in every partial, so the
+// lanes read whole rows; the 256 / NN row slots of the block take partials slot,
+// slot + SLOTS, ... (four running sums each) and are added in slot order
+// (deterministic).  One thread per weight walking all 586 partials in series, at a
+// stride of one row between lanes, took 98 us per layer.
+template <int NN>
+__global__ void __launch_bounds__(kRedThreads) k_grad_reduce(const float* __restrict__ wpart, int nwb,
+                                                             int rows_per_cta, const float* __restrict__ bpart,
+                                                             int nbb, int cin_pad, int cin_real, int cout_real,
+                                                             float* __restrict__ grad) {
+    constexpr int SLOTS = kRedThreads / NN;
+    __shared__ float s[SLOTS][NN];
+    const int co = threadIdx.x % NN, slot = threadIdx.x / NN;
+    const bool bias = blockIdx.x == 9u * cin_real;
+    const int tap = blockIdx.x / cin_real, ci = blockIdx.x % cin_real;
+    const float* src = bias ? bpart + co : wpart + (size_t)(tap * cin_pad + ci) * NN + co;
+    const size_t stride = bias ? NN : (size_t)rows_per_cta * NN;
+    const int n = bias ? nbb : nwb;
+    float a[4] = {};
+    int b = slot;
+    for (; b + 3 * SLOTS < n; b += 4 * SLOTS) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) a[q] += src[(size_t)(b + q * SLOTS) * stride];
+    }
+    for (; b < n; b += SLOTS) a[0] += src[(size_t)b * stride];
+    s[slot][co] = (a[0] + a[1]) + (a[2] + a[3]);
+    __syncthreads();
+    if (slot == 0 && co < cout_real) {
+        float v = 0.0f;
+        for (int q = 0; q < SLOTS; ++q) v += s[q][co];
+        grad[bias ? cout_real * 9 * cin_real + co : (co * 9 + tap) * cin_real + ci] = v;
     }
 }
 
@@ -361,9 +410,9 @@ static cudaError_t trainer_set_attrs() {
     set((const void*)k_conv3x3_tc<kNout, EPI_FINAL_RAW, float>, smax);
     set((const void*)k_conv3x3_tc<kCh, EPI_DGRAD, float>, smax);
     const int wg3 = 3 * kTile * kWgKC * 2 + 32 * kWgKC * 2;
-    set((const void*)k_wgrad_tc<3, 32>, wg3);
-    set((const void*)k_wgrad_tc<3, 16>, wg3);
-    set((const void*)k_wgrad_tc<2, 32>, wg3);
+    set((const void*)k_wgrad_tc<kCh, 32>, wg3);
+    set((const void*)k_wgrad_tc<kCh, 16>, wg3);
+    set((const void*)k_wgrad_tc<kCin0, 32>, wg3);
     return e;
 }
 
@@ -480,7 +529,7 @@ cudaError_t trainer_backprop(Trainer* tr, int nimg, int ny, int nx, const float*
     }
     // loss and its gradient (layer 5 output gradient, 16 channels, in g[0])
     k_cos_loss<<<tr->loss_blocks, kRedThreads, 0, s>>>(tr->out32, target, mask, nimg, hw, tr->g[0], tr->lpart);
-    k_loss_finalize<<<1, 1, 0, s>>>(tr->lpart, tr->loss_blocks, tr->red);
+    k_loss_finalize<<<1, 32, 0, s>>>(tr->lpart, tr->loss_blocks, tr->red);
     // backward
     const long long per_cta = ((P + tr->wg_ctas - 1) / tr->wg_ctas + kWgKC - 1) / kWgKC * kWgKC;
     const int wg_grid = (int)((P + per_cta - 1) / per_cta);
@@ -491,22 +540,26 @@ cudaError_t trainer_backprop(Trainer* tr, int nimg, int ny, int nx, const float*
         const __nv_bfloat16* a = l == 0 ? tr->x0 : tr->h[l - 1];
         const __nv_bfloat16* gl = tr->g[gi];
         const int nt = (9 * D.cin_pad + kTile - 1) / kTile;
-        if (D.cout_pad == 32 && nt == 3)
-            k_wgrad_tc<3, 32><<<wg_grid, 128, wg_smem, s>>>(a, D.cin_pad, gl, nimg, ny, nx, per_cta, tr->wpart,
-                                                            tr->err, tr->spin);
-        else if (D.cout_pad == 16 && nt == 3)
-            k_wgrad_tc<3, 16><<<wg_grid, 128, wg_smem, s>>>(a, D.cin_pad, gl, nimg, ny, nx, per_cta, tr->wpart,
-                                                            tr->err, tr->spin);
+        if (D.cin_pad == kCh && D.cout_pad == 32)
+            k_wgrad_tc<kCh, 32><<<wg_grid, 128, wg_smem, s>>>(a, gl, nimg, ny, nx, per_cta, tr->wpart, tr->err,
+                                                              tr->spin);
+        else if (D.cin_pad == kCh)
+            k_wgrad_tc<kCh, 16><<<wg_grid, 128, wg_smem, s>>>(a, gl, nimg, ny, nx, per_cta, tr->wpart, tr->err,
+                                                              tr->spin);
         else
-            k_wgrad_tc<2, 32><<<wg_grid, 128, wg_smem, s>>>(a, D.cin_pad, gl, nimg, ny, nx, per_cta, tr->wpart,
-                                                            tr->err, tr->spin);
-        if (D.cout_pad == 32)
+            k_wgrad_tc<kCin0, 32><<<wg_grid, 128, wg_smem, s>>>(a, gl, nimg, ny, nx, per_cta, tr->wpart, tr->err,
+                                                                tr->spin);
+        if (D.cout_pad == 32) {
             k_bias_part<32><<<tr->bias_blocks, kRedThreads, 0, s>>>(gl, P, tr->bpart);
-        else
+            k_grad_reduce<32><<<9 * D.cin_real + 1, kRedThreads, 0, s>>>(tr->wpart, wg_grid, nt * kTile, tr->bpart,
+                                                                         tr->bias_blocks, D.cin_pad, D.cin_real,
+                                                                         D.cout_real, tr->graw + D.off);
+        } else {
             k_bias_part<16><<<tr->bias_blocks, kRedThreads, 0, s>>>(gl, P, tr->bpart);
-        k_grad_reduce<<<(D.cout_real * 9 * D.cin_real + D.cout_real + 255) / 256, 256, 0, s>>>(
-            tr->wpart, wg_grid, nt * kTile, D.cout_pad, tr->bpart, tr->bias_blocks, D.cin_pad, D.cin_real,
-            D.cout_real, tr->graw + D.off);
+            k_grad_reduce<16><<<9 * D.cin_real + 1, kRedThreads, 0, s>>>(tr->wpart, wg_grid, nt * kTile, tr->bpart,
+                                                                         tr->bias_blocks, D.cin_pad, D.cin_real,
+                                                                         D.cout_real, tr->graw + D.off);
+        }
         if (l > 0) {
             // g_{l-1} = conv(g_l, W_l transposed / flipped) * (h_{l-1} > 0)
             const Layer Ld{tr->wd[l], nullptr, D.cout_pad, D.cin_pad, D.cin_pad, 0};
