@@ -91,6 +91,7 @@ cudaError_t build_pass_tables(void* out, int L, int v, cudaStream_t s);
 // Whether stage si's row inverse and stage sf's row forward can run as one fused
 // row pass on segment g (register-FFT rows, lean epilogue, sf's combination ends
 // with si's torque).
+template <typename R>
 bool can_fuse(const EvalSpec& si, const EvalSpec& sf, const LaunchGeom& g);
 template <typename R>
 cudaError_t launch_fused(const EvalSpec& si, const EvalSpec& sf, const LaunchGeom& g, cudaStream_t s,

@@ -1,6 +1,8 @@
-// eval_kernels.cu — instantiation and launch of the per-evaluation kernels for
-// FP32 and FP64: register-FFT kernels for power-of-two sizes, generic
-// shared-memory Stockham kernels otherwise.
+// eval_kernels.cuh — instantiation and launch of the per-evaluation kernels:
+// register-FFT kernels for power-of-two sizes, generic shared-memory Stockham
+// kernels otherwise.  Included by one compilation unit per precision
+// (eval_f32.cu, eval_f64.cu), which the build compiles side by side.
+#pragma once
 #include "build_api.h"
 #include "fast_kernels.cuh"
 #include "fused_kernels.cuh"
@@ -145,6 +147,14 @@ cudaError_t prepare_eval_kernels(size_t smem_row, size_t smem_col) {
 template <typename R>
 cudaError_t launch_one(int which, const EvalSpec& spec, const LaunchGeom& g, cudaStream_t s, int* nk) {
     int count = 0;
+    auto row = [&](auto kernel, int grid, int block, size_t smem) {
+        kernel<<<grid, block, smem, s>>>(g.films, g.row_items, g.n_row_items, spec);
+        ++count;
+    };
+    auto col = [&](auto kernel, int block, size_t smem) {
+        kernel<<<g.grid_col, block, smem, s>>>(g.films, g.col_items, g.n_col_items, spec);
+        ++count;
+    };
     if (which == 0 || which == 2) {
         if (g.fast_row) {
             dispatch_LV<R>(g.fast_row, g.row_var, [&](auto LC, auto VC) {
@@ -152,70 +162,47 @@ cudaError_t launch_one(int which, const EvalSpec& spec, const LaunchGeom& g, cud
                 if constexpr (RowCfg<R, L, V>::SMEM <= kSmemMax) {
                     using C = RowCfg<R, L, V>;
                     if (which == 0) {
-                        k_row_forward_fast<R, L, V><<<g.grid_row, C::THREADS, C::SMEM, s>>>(g.films, g.row_items,
-                                                                                           g.n_row_items, spec);
-                        ++count;
+                        row(k_row_forward_fast<R, L, V>, g.grid_row, C::THREADS, C::SMEM);
                     } else if (lean_epilogue(spec) || lean_err45_epilogue(spec)) {
                         // transform only, then the torque epilogue as a streaming kernel
                         constexpr int CPI = C::T * L;
-                        const long long cells = (long long)g.n_row_items * CPI;
-                        k_row_inverse_fast<R, L, 1, V><<<g.grid_rinv, C::THREADS, C::SMEM, s>>>(
-                            g.films, g.row_items, g.n_row_items, spec);
-                        if (lean_err45_epilogue(spec))
-                            k_stage_torque<R, true><<<stage_grid(cells), 256, 0, s>>>(g.films, g.row_items,
-                                                                                        g.n_row_items, CPI, spec);
-                        else
-                            k_stage_torque<R, false><<<stage_grid(cells), 256, 0, s>>>(g.films, g.row_items,
-                                                                                         g.n_row_items, CPI, spec);
-                        count += 2;
+                        row(k_row_inverse_fast<R, L, 1, V>, g.grid_rinv, C::THREADS, C::SMEM);
+                        const int grid = stage_grid((long long)g.n_row_items * CPI);
+                        auto torque = lean_err45_epilogue(spec) ? k_stage_torque<R, true> : k_stage_torque<R, false>;
+                        torque<<<grid, 256, 0, s>>>(g.films, g.row_items, g.n_row_items, CPI, spec);
+                        ++count;
                     } else if (spec.rhs == RHS_MINIMIZE) {
-                        k_row_inverse_fast<R, L, 2, V><<<g.grid_rfull, C::THREADS, C::SMEM, s>>>(
-                            g.films, g.row_items, g.n_row_items, spec);
-                        ++count;
+                        row(k_row_inverse_fast<R, L, 2, V>, g.grid_rfull, C::THREADS, C::SMEM);
                     } else {
-                        k_row_inverse_fast<R, L, 0, V><<<g.grid_rfull, C::THREADS, C::SMEM, s>>>(
-                            g.films, g.row_items, g.n_row_items, spec);
-                        ++count;
+                        row(k_row_inverse_fast<R, L, 0, V>, g.grid_rfull, C::THREADS, C::SMEM);
                     }
                 }
             });
         } else if (which == 0) {
-            k_row_forward<R><<<g.grid_row, 256, g.smem_row, s>>>(g.films, g.row_items, g.n_row_items, spec);
-            ++count;
+            row(k_row_forward<R>, g.grid_row, 256, g.smem_row);
         } else {
-            if (spec.rhs == RHS_MINIMIZE)
-                k_row_inverse<R, true><<<g.grid_row, 256, g.smem_row, s>>>(g.films, g.row_items, g.n_row_items,
-                                                                           spec);
-            else
-                k_row_inverse<R, false><<<g.grid_row, 256, g.smem_row, s>>>(g.films, g.row_items, g.n_row_items,
-                                                                            spec);
-            ++count;
+            row(spec.rhs == RHS_MINIMIZE ? k_row_inverse<R, true> : k_row_inverse<R, false>, g.grid_row, 256,
+                g.smem_row);
         }
+    } else if (g.fast_col) {
+        // col_var = 2 * radix plan + lean form
+        dispatch_LV<R>(g.fast_col, g.col_var / 2, [&](auto LC, auto VC) {
+            constexpr int L = decltype(LC)::value, V = decltype(VC)::value;
+            if constexpr (ColCfg<R, L, V>::SMEM + kStaticSmemCol <= kSmemMax) {
+                using Staged = ColCfg<R, L, V, false>;
+                using Lean = ColCfg<R, L, V, true>;
+                if (g.col_var % 2) col(k_column_fast<R, L, V, true>, Lean::THREADS, Lean::SMEM);
+                else col(k_column_fast<R, L, V, false>, Staged::THREADS, Staged::SMEM);
+            }
+        });
     } else {
-        if (g.fast_col) {
-            // col_var = 2 * radix plan + lean form
-            dispatch_LV<R>(g.fast_col, g.col_var / 2, [&](auto LC, auto VC) {
-                constexpr int L = decltype(LC)::value, V = decltype(VC)::value;
-                if constexpr (ColCfg<R, L, V>::SMEM + kStaticSmemCol <= kSmemMax) {
-                    if (g.col_var % 2)
-                        k_column_fast<R, L, V, true><<<g.grid_col, ColCfg<R, L, V, true>::THREADS,
-                                                       ColCfg<R, L, V, true>::SMEM, s>>>(g.films, g.col_items,
-                                                                                         g.n_col_items, spec);
-                    else
-                        k_column_fast<R, L, V, false><<<g.grid_col, ColCfg<R, L, V, false>::THREADS,
-                                                        ColCfg<R, L, V, false>::SMEM, s>>>(g.films, g.col_items,
-                                                                                           g.n_col_items, spec);
-                }
-            });
-        } else {
-            k_column<R><<<g.grid_col, 256, g.smem_col, s>>>(g.films, g.col_items, g.n_col_items, spec);
-        }
-        ++count;
+        col(k_column<R>, 256, g.smem_col);
     }
     if (nk) *nk += count;
     return cudaGetLastError();
 }
 
+template <typename R>
 bool can_fuse(const EvalSpec& si, const EvalSpec& sf, const LaunchGeom& g) {
     return g.fast_row != 0 && g.fuse_rows && lean_epilogue(si) && si.k_out != KB_NONE && !si.skip_if_fsal &&
            !sf.skip_if_fsal && sf.nterm >= 1 && sf.nterm <= 6 && sf.kidx[sf.nterm - 1] == si.k_out &&
@@ -282,19 +269,5 @@ void fast_occupancy(int nx, int ny, int row_var, int col_var, int* fwd_blocks_pe
         }
     });
 }
-template void fast_occupancy<float>(int, int, int, int, int*, int*, int*, int*, int*);
-template void fast_occupancy<double>(int, int, int, int, int*, int*, int*, int*, int*);
-template FastCfg fast_config<float>(int, int);
-template FastCfg fast_config<double>(int, int);
-template cudaError_t build_pass_tables<float>(void*, int, int, cudaStream_t);
-template cudaError_t build_pass_tables<double>(void*, int, int, cudaStream_t);
-template cudaError_t launch_one<float>(int, const EvalSpec&, const LaunchGeom&, cudaStream_t, int*);
-template cudaError_t launch_one<double>(int, const EvalSpec&, const LaunchGeom&, cudaStream_t, int*);
-template cudaError_t launch_fused<float>(const EvalSpec&, const EvalSpec&, const LaunchGeom&, cudaStream_t, int*);
-template cudaError_t launch_fused<double>(const EvalSpec&, const EvalSpec&, const LaunchGeom&, cudaStream_t, int*);
-template cudaError_t prepare_eval_kernels<float>(size_t, size_t);
-template cudaError_t prepare_eval_kernels<double>(size_t, size_t);
-template cudaError_t launch_eval<float>(const EvalSpec&, const LaunchGeom&, cudaStream_t);
-template cudaError_t launch_eval<double>(const EvalSpec&, const LaunchGeom&, cudaStream_t);
 
 }  // namespace llg

@@ -433,7 +433,7 @@ struct Engine final : EngineBase {
             if (e.demag && geom.any_demag)
                 for (auto& sg : cseg) CUDA_TRY(launch_one<R>(1, e, sg, stream, &nk));
             for (size_t q = 0; q < rseg.size(); ++q) {
-                if (i + 1 < n && can_fuse(e, v[i + 1], rseg[q])) {
+                if (i + 1 < n && can_fuse<R>(e, v[i + 1], rseg[q])) {
                     CUDA_TRY(launch_fused<R>(e, v[i + 1], rseg[q], stream, &nk));
                     fwd_done[q] = 1;
                 } else {
@@ -1798,7 +1798,7 @@ struct Engine final : EngineBase {
             for (auto& sg : rseg) CUDA_TRY(launch_one<R>(2, e, sg, stream));
             CUDA_TRY(cudaEventRecord(ev[3], stream));
             for (auto& sg : rseg)
-                if (can_fuse(e, f, sg)) {
+                if (can_fuse<R>(e, f, sg)) {
                     CUDA_TRY(launch_fused<R>(e, f, sg, stream));
                     any_fused = true;
                 }
