@@ -74,7 +74,7 @@ __device__ __forceinline__ void normalize3(R* v) {
 __device__ __forceinline__ bool skip_item(const EvalSpec& spec, const StepState* st) {
     if (!st->active) return true;
     if (spec.skip_if_fsal && st->fsal_valid) return true;
-    if (spec.req && st->req != spec.req) return true;
+    if (spec.req && !req_matches(spec.req, st->req)) return true;
     return false;
 }
 
@@ -577,6 +577,7 @@ __device__ __forceinline__ void row_epilogue(const FilmDev& F, const EvalSpec& s
     const int nx = F.nx, ny = F.ny, n = nx * ny;
     const int j0 = blk * T;
     const int cur = st->cur;
+    const int rhs = spec.rhs != RHS_REQUEST ? spec.rhs : st->req == REQ_ENERGY ? RHS_ENERGY : RHS_TORQUE;
         const R* __restrict__ msb = mbuf<R>(F, spec.m_in, cur);
         R* __restrict__ kout = spec.k_out != KB_NONE ? kbuf<R>(F, spec.k_out, cur) : nullptr;
         R* __restrict__ bout = reinterpret_cast<R*>(F.bout);
@@ -595,7 +596,7 @@ __device__ __forceinline__ void row_epilogue(const FilmDev& F, const EvalSpec& s
             R mc[3];
             ld3(msb, n, idx, mc);
             R b[3];
-            if (spec.rhs == RHS_ENERGY) {
+            if (rhs == RHS_ENERGY) {
                 double bd[3] = {0.0, 0.0, 0.0};
                 if (do_fft) {
                     bd[0] = (double)dfield(r, i, 0);
@@ -615,14 +616,14 @@ __device__ __forceinline__ void row_epilogue(const FilmDev& F, const EvalSpec& s
                 b[1] += dfield(r, i, 1);
                 b[2] += dfield(r, i, 2);
             }
-            if (spec.rhs == RHS_FIELD) {
+            if (rhs == RHS_FIELD) {
                 bout[idx] = b[0]; bout[n + idx] = b[1]; bout[2 * n + idx] = b[2];
             }
             // torque m x B and m x (m x B) (llg.rs:20-32, 38-50)
             R k[3] = {(R)0, (R)0, (R)0};
-            if (spec.rhs == RHS_LLG || spec.rhs == RHS_RELAX) {
+            if (rhs == RHS_LLG || rhs == RHS_RELAX) {
                 const R denom = (R)1 + alp * alp;
-                const bool llg = spec.rhs == RHS_LLG;
+                const bool llg = rhs == RHS_LLG;
                 torque_cell<R>(mc, b, llg ? -gam / denom : -gam * alp / denom, llg ? (R)1 : (R)0, llg ? alp : (R)1, k);
                 kout[idx] = k[0]; kout[n + idx] = k[1]; kout[2 * n + idx] = k[2];
             }

@@ -5,8 +5,8 @@
 // RhsMode RHS_MINIMIZE (the effective field, the damping-only update of every
 // cell written to the other parity buffer, the FP64 block reductions of
 // max |m x B| and sum |m x B|, and max |m' - m| through the film's error-norm
-// accumulator), the deterministic per-film finalisation of the
-// reductions, and k_minimize_control, which adopts the update and runs the
+// accumulator), and k_finalize, which sums the reductions of a film
+// (deterministic), adopts the update and runs the
 // iteration's decisions: torque threshold, the dM stop with its torque gates,
 // the lambda controller and the stall counter.  A finished film drops its
 // REQ_MINIMIZE request, so the rest of the graph skips it.
@@ -145,13 +145,8 @@ __global__ void k_minimize_begin(FilmDev* films, const MinimizeStateDev* ms_all,
     st->lam = M.lambda;
 }
 
-// One thread per film, after the RHS_MINIMIZE evaluation and k_finalize.
-__global__ void k_minimize_control(FilmDev* films, MinimizeStateDev* ms_all, int nfilms, MinimizeSettingsDev S) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= nfilms) return;
-    StepState* st = films[f].st;
-    if (!st->active || st->req != REQ_MINIMIZE) return;
-    MinimizeStateDev& M = ms_all[f];
+// After the RHS_MINIMIZE evaluation and the reductions of one film.
+__device__ inline void minimize_control_film(StepState* st, MinimizeStateDev& M, const MinimizeSettingsDev& S) {
     st->cur ^= 1;  // the updated state is the film's state from here on
     // max |m' - m| arrives in the error-norm accumulator (max of non-negative bit patterns)
     const double dmx = __longlong_as_double((long long)st->err_bits);

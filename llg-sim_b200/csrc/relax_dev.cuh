@@ -1,12 +1,12 @@
 // relax_dev.cuh — relax_with_report (relax.rs:334-768) as a per-film device
 // state machine.
 //
-// Each relax iteration of the replayed graph executes at most one request per
-// film — an energy evaluation (compute_total_energy, energy.rs:287), a torque
-// rebuild (torque_metric_rebuild, relax.rs:192) or one RK23 relax attempt
-// (llg.rs:278) — gated by StepState::req, and then runs k_relax_control, which
-// consumes the result and advances the film's program counter to the next
-// request.  Films advance independently; a finished film goes inactive.
+// Each relax iteration of the replayed graph executes a film's requested
+// evaluation, if any — the energy (compute_total_energy, energy.rs:287) or a torque
+// rebuild (torque_metric_rebuild, relax.rs:192) — and then, if it asks for one, one
+// RK23 relax attempt (llg.rs:278), gated by StepState::req.  After either,
+// relax_control_core consumes the result and advances the film's program counter to
+// the next request (at the end of k_finalize; k_relax_control issues the first).  Films advance independently; a finished film goes inactive.
 #pragma once
 #include <cmath>
 

@@ -111,13 +111,9 @@ __global__ void k_set_control(FilmDev* films, int nfilms, Control c, const FilmC
     }
 }
 
-// Step-size controller (llg.rs:997-1025 for order 5, llg.rs:401-435 for order 3).
-__global__ void k_controller(FilmDev* films, int nfilms, int order, int req) {
-    int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= nfilms) return;
-    StepState* st = films[f].st;
-    if (!st->active) return;
-    if (req && st->req != req) return;
+// Step-size controller of one film (llg.rs:997-1025 for order 5, llg.rs:401-435 for
+// order 3).
+__device__ void controller_core(StepState* st, int order) {
     const unsigned long long bits = st->err_bits;
     st->err_bits = 0ull;
     const double err = __longlong_as_double((long long)bits);
@@ -137,16 +133,15 @@ __global__ void k_controller(FilmDev* films, int nfilms, int order, int req) {
     const bool acc = (eps <= st->max_err) || (dt0 <= st->dt_min * 1.0000000001);
     if (acc) {
         st->cur ^= 1;
-        st->fsal_valid = 1;
         st->n_acc += 1;
         st->t += dt0;
     } else {
-        // RK45: k1 of the unchanged state stays valid (its buffer is not written by
-        // the rejected attempt, and the run / step calls evaluate it before their
-        // first attempt); RK23 re-evaluates it, as the relax loop expects
-        st->fsal_valid = order == 5 ? 1 : 0;
         st->n_rej += 1;
     }
+    // an accepted step flips k7 into k1; a rejected attempt leaves the state and k1's
+    // buffer untouched: k1 = f(m0) holds either way, and is evaluated once, before the
+    // first attempt of a call
+    st->fsal_valid = 1;
     st->accepted = acc ? 1 : 0;
     st->dt = dt_next;
     if (st->attempts_left > 0) st->attempts_left -= 1;
@@ -159,16 +154,18 @@ __global__ void k_controller(FilmDev* films, int nfilms, int order, int req) {
     if (stop) st->active = 0;
 }
 
-// Sum the per-block partial reductions of each film in block order (deterministic).
-// One warp per film: lane l sums blocks l, l + 32, ... in order, then a fixed
-// butterfly combines the lanes (deterministic; the loads of the 32 lanes overlap).
-constexpr int kFinalizeFilmsPerBlock = 4;
-__global__ void k_finalize(FilmDev* films, int nfilms, int req) {
-    const int f = blockIdx.x * kFinalizeFilmsPerBlock + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (f >= nfilms) return;   // uniform over the warp
-    const FilmDev& F = films[f];
-    if (req && (!F.st->active || F.st->req != req)) return;
-    double acc[RED_NSLOT];
+__global__ void k_controller(FilmDev* films, int nfilms, int order) {
+    int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= nfilms) return;
+    StepState* st = films[f].st;
+    if (st->active) controller_core(st, order);
+}
+
+// Sums the per-block partial reductions of one film (deterministic) into every
+// lane of its warp: lane l sums blocks l, l + 32, ... in order, then a fixed butterfly
+// combines the lanes (the loads of the 32 lanes overlap).
+__device__ __forceinline__ void finalize_film(const FilmDev& F, double* acc) {
+    const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int s = 0; s < RED_NSLOT; ++s) acc[s] = 0.0;
     for (int b = lane; b < F.nblk; b += 32) {
@@ -177,13 +174,48 @@ __global__ void k_finalize(FilmDev* films, int nfilms, int req) {
         for (int s = 0; s < RED_NSLOT; ++s) acc[s] = (s == RED_TMAX) ? fmax(acc[s], p[s]) : acc[s] + p[s];
     }
 #pragma unroll
-    for (int s = 0; s < RED_NSLOT; ++s)
-        for (int o = 16; o > 0; o >>= 1) {
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int s = 0; s < RED_NSLOT; ++s) {
             const double w = __shfl_xor_sync(0xffffffffu, acc[s], o);
             acc[s] = (s == RED_TMAX) ? fmax(acc[s], w) : acc[s] + w;
         }
-    if (lane == 0)
-        for (int s = 0; s < RED_NSLOT; ++s) F.st->red[s] = acc[s];
+}
+
+// End of an evaluation with reductions, one warp per film: the sums into
+// StepState::red and then, in the same kernel, what consumes them — one launch and
+// one round of dependent loads instead of two or three per iteration.
+//   END_RED   nothing more (films matching req; 0: all)
+//   END_EVAL  the relax controller takes the requested energy or torque
+//   END_STEP  the RK23 controller, then the relax controller takes the attempt
+//   END_MIN   the minimiser's controller takes the update
+enum EndMode { END_RED = 0, END_EVAL = 1, END_STEP = 2, END_MIN = 3 };
+constexpr int kFinalizeFilmsPerBlock = 4;
+template <int MODE, typename STATE, typename SETTINGS>
+__global__ void k_finalize(FilmDev* films, int nfilms, int req, STATE* ctl, SETTINGS S) {
+    const int f = blockIdx.x * kFinalizeFilmsPerBlock + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (f >= nfilms) return;   // uniform over the warp
+    const FilmDev& F = films[f];
+    StepState* st = F.st;
+    if constexpr (MODE == END_EVAL) {
+        // a controller call bounds its transitions and may end without a request: go on
+        if (st->active && st->req == REQ_NONE) {
+            if (lane == 0) relax_control_core(st, ctl[f], S);
+            return;
+        }
+    }
+    if (req && (!st->active || !req_matches(req, st->req))) return;
+    double acc[RED_NSLOT];
+    finalize_film(F, acc);
+    if (lane != 0) return;
+    if constexpr (MODE == END_STEP) {
+        controller_core(st, 3);
+        if (!st->active) return;   // non-finite: the host finds err_code
+    }
+#pragma unroll
+    for (int s = 0; s < RED_NSLOT; ++s) st->red[s] = acc[s];
+    if constexpr (MODE == END_EVAL || MODE == END_STEP) relax_control_core(st, ctl[f], S);
+    if constexpr (MODE == END_MIN) minimize_control_film(st, ctl[f], S);
 }
 
 // <m> partial sums per row block of every film.
@@ -1132,10 +1164,8 @@ struct Engine final : EngineBase {
     int mean_m(double* out3n) override {
         k_mean_m<R><<<std::min(geom.n_row_items, 148 * 8), 256, 0, stream>>>(d_films, d_row_items, geom.n_row_items);
         CUDA_TRY(cudaGetLastError());
-        k_finalize<<<(nf + kFinalizeFilmsPerBlock - 1) / kFinalizeFilmsPerBlock, 32 * kFinalizeFilmsPerBlock, 0,
-                     stream>>>(d_films, nf, 0);
-        CUDA_TRY(cudaGetLastError());
         int rc;
+        if ((rc = finalize<END_RED>(0, (char*)nullptr, 0))) return rc;
         if ((rc = read_states())) return rc;
         for (int f = 0; f < nf; ++f)
             for (int c = 0; c < 3; ++c) out3n[3 * f + c] = h_states[f].red[RED_MX + c] / (double)cells(f);
@@ -1180,9 +1210,10 @@ struct Engine final : EngineBase {
         for (double a : as) s.a[q++] = a;
     }
 
-    int finalize(int req) {
-        k_finalize<<<(nf + kFinalizeFilmsPerBlock - 1) / kFinalizeFilmsPerBlock, 32 * kFinalizeFilmsPerBlock, 0,
-                     stream>>>(d_films, nf, req);
+    template <int MODE, typename STATE, typename SETTINGS>
+    int finalize(int req, STATE* ctl, const SETTINGS& S) {
+        k_finalize<MODE><<<(nf + kFinalizeFilmsPerBlock - 1) / kFinalizeFilmsPerBlock, 32 * kFinalizeFilmsPerBlock, 0,
+                           stream>>>(d_films, nf, req, ctl, S);
         CUDA_TRY(cudaGetLastError());
         launches += 1;
         return LLG_OK;
@@ -1199,15 +1230,15 @@ struct Engine final : EngineBase {
         return e;
     }
 
-    // One integrator attempt: stages 1 (unless with_stage1 is false: RK45 graphs,
-    // whose callers evaluate stage 1 once before their first attempt, since after
-    // any attempt k1 of the film's state is valid) to s, then the controller; req
-    // gates every kernel on StepState::req (relax).
-    int launch_attempt(int kind, int fmask, int req, bool with_stage1 = true) {
+    // Stages 2 to s of one integrator attempt and, for a run or a single step, the
+    // controller (relax runs it at the end of its iteration).  Stage 1 is not among
+    // them: the caller evaluates it once before its first attempt, since after any
+    // attempt k1 of the film's state is valid.  req gates every kernel on
+    // StepState::req (relax).
+    int launch_attempt(int kind, int fmask, int req, bool control = true) {
         int rc;
         std::vector<EvalSpec> ch;
         EvalSpec e = stage1_spec(kind, fmask, req);
-        if (with_stage1) ch.push_back(e);
         e.skip_if_fsal = 0;
         if (kind == KIND_RK45) {
             using namespace dp5;
@@ -1234,10 +1265,6 @@ struct Engine final : EngineBase {
             std::memcpy(e.wb, wb, sizeof(wb));
             std::memcpy(e.wh, wh, sizeof(wh));
             ch.push_back(e);
-            if ((rc = eval_chain(ch))) return rc;
-            k_controller<<<(nf + 127) / 128, 128, 0, stream>>>(d_films, nf, 5, req);
-            CUDA_TRY(cudaGetLastError());
-            launches += 1;
         } else {
             using namespace bs3;
             combo(e, MB_S0, {KB_K1}, {A21});
@@ -1255,36 +1282,42 @@ struct Engine final : EngineBase {
             std::memcpy(e.wb, wb, sizeof(wb));
             std::memcpy(e.wh, wh, sizeof(wh));
             ch.push_back(e);
-            if ((rc = eval_chain(ch))) return rc;
-            k_controller<<<(nf + 127) / 128, 128, 0, stream>>>(d_films, nf, 3, req);
+        }
+        if ((rc = eval_chain(ch))) return rc;
+        if (control) {
+            k_controller<<<(nf + 127) / 128, 128, 0, stream>>>(d_films, nf, kind == KIND_RK45 ? 5 : 3);
             CUDA_TRY(cudaGetLastError());
             launches += 1;
-            if ((rc = finalize(req))) return rc;
         }
         return LLG_OK;
     }
 
-    // One relax iteration: the request-gated energy, torque and RK23 step, then the controller.
+    // One relax iteration: the requested evaluations (energy or torque) and the
+    // controller that consumes them, then one RK23 attempt of the films that ask for it
+    // by now and its controllers — a film that has its energy goes on with its next
+    // step in the same iteration.  With the full field mask energy and torque need the
+    // same passes and share them.
     int launch_relax_iteration(int fmask, const RelaxSettingsDev& S) {
         int rc;
         EvalSpec en = base_spec(LLG_FIELD_FULL);
-        en.req = REQ_ENERGY;
         en.rhs = RHS_ENERGY;
+        en.req = REQ_ENERGY;
         en.reduce = 1;
         en.demag = 1;  // the energy includes demag iff Material::demag (energy.rs:117-121)
+        if (fmask == LLG_FIELD_FULL) {
+            en.rhs = RHS_REQUEST;
+            en.req = REQ_EVAL;
+        } else {
+            EvalSpec tq = base_spec(fmask);
+            tq.req = REQ_TORQUE;
+            tq.rhs = RHS_TORQUE;
+            tq.reduce = 1;
+            if ((rc = eval(tq))) return rc;
+        }
         if ((rc = eval(en))) return rc;
-        if ((rc = finalize(REQ_ENERGY))) return rc;
-        EvalSpec tq = base_spec(fmask);
-        tq.req = REQ_TORQUE;
-        tq.rhs = RHS_TORQUE;
-        tq.reduce = 1;
-        if ((rc = eval(tq))) return rc;
-        if ((rc = finalize(REQ_TORQUE))) return rc;
-        if ((rc = launch_attempt(KIND_RK23, fmask, REQ_STEP))) return rc;
-        k_relax_control<<<(nf + 127) / 128, 128, 0, stream>>>(d_films, d_relax, nf, S);
-        CUDA_TRY(cudaGetLastError());
-        launches += 1;
-        return LLG_OK;
+        if ((rc = finalize<END_EVAL>(REQ_EVAL, d_relax, S))) return rc;
+        if ((rc = launch_attempt(KIND_RK23, fmask, REQ_STEP, false))) return rc;
+        return finalize<END_STEP>(REQ_STEP, d_relax, S);
     }
 
     // One minimiser iteration: the RHS_MINIMIZE evaluation, the reductions, the controller.
@@ -1295,11 +1328,7 @@ struct Engine final : EngineBase {
         e.rhs = RHS_MINIMIZE;
         e.reduce = 1;
         if ((rc = eval(e))) return rc;
-        if ((rc = finalize(REQ_MINIMIZE))) return rc;
-        k_minimize_control<<<(nf + 127) / 128, 128, 0, stream>>>(d_films, d_min, nf, S);
-        CUDA_TRY(cudaGetLastError());
-        launches += 1;
-        return LLG_OK;
+        return finalize<END_MIN>(REQ_MINIMIZE, d_min, S);
     }
 
     int graph_launch(long long key, cudaGraphExec_t ge) {
@@ -1348,7 +1377,7 @@ struct Engine final : EngineBase {
 
     int attempt_graph(int kind, int fmask, int reps, cudaGraphExec_t* out) {
         return get_graph(graph_key(kind, fmask, reps), reps,
-                         [&]() { return launch_attempt(kind, fmask, 0, kind != KIND_RK45); }, out);
+                         [&]() { return launch_attempt(kind, fmask, 0); }, out);
     }
 
     // FSAL validity across calls (llg.rs:854-867, 317-330): same kind, mask and b_ext.
@@ -1383,7 +1412,7 @@ struct Engine final : EngineBase {
         if ((rc = set_control(c, p, inv.get(), false))) return rc;
         cudaGraphExec_t ge = nullptr;
         if ((rc = attempt_graph(kind, fmask, 1, &ge))) return rc;
-        if (kind == KIND_RK45 && (rc = eval(stage1_spec(kind, fmask, 0)))) return rc;
+        if ((rc = eval(stage1_spec(kind, fmask, 0)))) return rc;
         if ((rc = graph_launch(graph_key(kind, fmask, 1), ge))) return rc;
         if ((rc = read_states())) return rc;
         for (int f = 0; f < nf; ++f) {
@@ -1433,7 +1462,7 @@ struct Engine final : EngineBase {
         const int reps = 8;
         cudaGraphExec_t ge = nullptr, ge1 = nullptr;
         if ((rc = attempt_graph(kind, fmask, reps, &ge))) return rc;
-        if (kind == KIND_RK45 && (rc = eval(stage1_spec(kind, fmask, 0)))) return rc;
+        if ((rc = eval(stage1_spec(kind, fmask, 0)))) return rc;
         long long launched = 0;
         const long long limit = max_attempts > 0 ? max_attempts : (1LL << 40);
         long long round = 32;
@@ -1525,6 +1554,7 @@ struct Engine final : EngineBase {
         for (int f = 0; f < nf; ++f) inv[f] = true;  // scratch.invalidate_last_b_eff() (relax.rs:374)
         invalidate_fsal_host();
         if ((rc = set_control(c, p, inv.get(), false))) return rc;
+        if ((rc = eval(stage1_spec(KIND_RK23, fmask, 0)))) return rc;
         // issue the first requests
         k_relax_control<<<(nf + 127) / 128, 128, 0, stream>>>(d_films, d_relax, nf, S);
         CUDA_TRY(cudaGetLastError());
@@ -1679,7 +1709,7 @@ struct Engine final : EngineBase {
         int rc;
         if ((rc = set_control(idle_control(), nullptr, nullptr, true))) return rc;
         if ((rc = eval(e))) return rc;
-        if (e.reduce && (rc = finalize(0))) return rc;
+        if (e.reduce && (rc = finalize<END_RED>(0, (char*)nullptr, 0))) return rc;
         return LLG_OK;
     }
 

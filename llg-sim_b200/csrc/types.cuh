@@ -33,10 +33,14 @@ enum KBuf : int { KB_NONE = 0, KB_K1 = 1, KB_K2, KB_K3, KB_K4, KB_K5, KB_K6, KB_
 
 // RHS_MINIMIZE: one damping-only descent update m' = normalize(m + lambda (m x B) x m)
 // written to the other parity buffer (minimize.rs:216-256)
-enum RhsMode : int { RHS_LLG = 0, RHS_RELAX = 1, RHS_FIELD = 2, RHS_ENERGY = 3, RHS_TORQUE = 4, RHS_MINIMIZE = 5 };
+// RHS_REQUEST: RHS_ENERGY or RHS_TORQUE, whichever the film requested
+enum RhsMode : int {
+    RHS_LLG = 0, RHS_RELAX = 1, RHS_FIELD = 2, RHS_ENERGY = 3, RHS_TORQUE = 4, RHS_MINIMIZE = 5, RHS_REQUEST = 6
+};
 enum ErrMode : int { ERR_NONE = 0, ERR_RK45 = 1, ERR_RK23 = 2 };
 // Requests of the device-side relax and minimiser controllers.
-enum ReqKind : int { REQ_NONE = 0, REQ_ENERGY = 1, REQ_TORQUE = 2, REQ_STEP = 3, REQ_MINIMIZE = 4 };
+// REQ_EVAL names no request: it gates a kernel on either evaluation (energy or torque).
+enum ReqKind : int { REQ_NONE = 0, REQ_ENERGY = 1, REQ_TORQUE = 2, REQ_STEP = 3, REQ_MINIMIZE = 4, REQ_EVAL = 5 };
 
 // Slots of the per-block FP64 partial reductions.
 enum RedSlot : int {
@@ -44,6 +48,11 @@ enum RedSlot : int {
     RED_TSUM, RED_TSUM2, RED_TMAX, RED_MX, RED_MY, RED_MZ,
     RED_NSLOT
 };
+
+// Whether a film that requested `have` takes part in a kernel gated on `gate`.
+__host__ __device__ inline bool req_matches(int gate, int have) {
+    return gate == REQ_EVAL ? have == REQ_ENERGY || have == REQ_TORQUE : gate == have;
+}
 
 // Per-film integrator / controller state (device resident, FP64).
 struct StepState {
@@ -121,7 +130,7 @@ struct EvalSpec {
     int local;                    // include the local terms (0: demag field only)
     int skip_if_fsal;             // skip when the film's FSAL torque is valid
     int reduce;                   // write per-block reductions (torque / energy / mean m)
-    int req;                      // run only for films whose StepState::req equals this (0: always)
+    int req;                      // run only for films whose StepState::req matches this (0: always)
     // Error-norm weights over k1..k7: wb = solution weights b_q, wh = embedded
     // weights bhat_q (RK45: torques, llg.rs:948-997; RK23: states, llg.rs:356-401)
     double wb[8];
