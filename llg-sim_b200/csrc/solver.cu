@@ -399,6 +399,9 @@ struct Engine final : EngineBase {
     // launch segments: films grouped by the row (rseg) / column (cseg) kernel they use,
     // with the resident blocks per SM of each segment's kernels
     std::vector<LaunchGeom> rseg, cseg;
+    std::vector<cudaStream_t> side;          // streams of the second, third, ... segment of a pass
+    std::vector<cudaEvent_t> side_event;
+    cudaEvent_t fork_event = nullptr;
     // each segment's geometry under radix plan 0 / 1 (where the plan exists) and
     // the resident blocks per SM of its kernels; the autotuner picks one
     // (a column segment has 4 forms: 2 * plan + lean)
@@ -422,6 +425,11 @@ struct Engine final : EngineBase {
         if (h_relax) cudaFreeHost(h_relax);
         if (h_min) cudaFreeHost(h_min);
         if (h_ctl) cudaFreeHost(h_ctl);
+        for (cudaStream_t x : side)
+            if (x) cudaStreamDestroy(x);
+        for (cudaEvent_t x : side_event)
+            if (x) cudaEventDestroy(x);
+        if (fork_event) cudaEventDestroy(fork_event);
         if (own_stream) cudaStreamDestroy(own_stream);
     }
 
@@ -440,13 +448,46 @@ struct Engine final : EngineBase {
         return LLG_OK;
     }
 
-    // One evaluation: row forward, column (with demag), row inverse, one launch per segment.
+    // The launches of one pass, one per segment.  Segments hold different films, so
+    // their launches are independent and run side by side on streams forked from and
+    // joined to the engine's: a pass takes as long as its slowest segment instead of
+    // the sum (each of them leaves most of the machine idle in a mixed batch).
+    template <typename Body>
+    int each_segment(size_t n, Body body) {
+        if (n > 1) CUDA_TRY(cudaEventRecord(fork_event, stream));
+        for (size_t q = 0; q < n; ++q) {
+            cudaStream_t s = q == 0 ? stream : side[q - 1];
+            if (q > 0) CUDA_TRY(cudaStreamWaitEvent(s, fork_event, 0));
+            CUDA_TRY(body(q, s));
+            if (q > 0) CUDA_TRY(cudaEventRecord(side_event[q - 1], s));
+        }
+        for (size_t q = 1; q < n; ++q) CUDA_TRY(cudaStreamWaitEvent(stream, side_event[q - 1], 0));
+        return LLG_OK;
+    }
+
+    int create_side_streams() {
+        const size_t n = std::max(rseg.size(), cseg.size());
+        if (n > 1) CUDA_TRY(cudaEventCreateWithFlags(&fork_event, cudaEventDisableTiming));
+        for (size_t q = 1; q < n; ++q) {
+            side.push_back(nullptr);
+            side_event.push_back(nullptr);
+            CUDA_TRY(cudaStreamCreateWithFlags(&side.back(), cudaStreamNonBlocking));
+            CUDA_TRY(cudaEventCreateWithFlags(&side_event.back(), cudaEventDisableTiming));
+        }
+        return LLG_OK;
+    }
+
+    // One evaluation: row forward, column (with demag), row inverse.
     int eval(const EvalSpec& e) {
-        int nk = 0;
-        for (auto& sg : rseg) CUDA_TRY(launch_one<R>(0, e, sg, stream, &nk));
-        if (e.demag && geom.any_demag)
-            for (auto& sg : cseg) CUDA_TRY(launch_one<R>(1, e, sg, stream, &nk));
-        for (auto& sg : rseg) CUDA_TRY(launch_one<R>(2, e, sg, stream, &nk));
+        int nk = 0, rc;
+        auto pass = [&](int which) {
+            auto& segs = which == 1 ? cseg : rseg;
+            return each_segment(segs.size(),
+                                [&](size_t q, cudaStream_t s) { return launch_one<R>(which, e, segs[q], s, &nk); });
+        };
+        if ((rc = pass(0))) return rc;
+        if (e.demag && geom.any_demag && (rc = pass(1))) return rc;
+        if ((rc = pass(2))) return rc;
         launches += nk;
         return LLG_OK;
     }
@@ -455,24 +496,23 @@ struct Engine final : EngineBase {
     // rows, a lean stage followed by a combination that ends with its torque),
     // stage i's row inverse and stage i+1's row forward run as one fused row pass.
     int eval_chain(const std::vector<EvalSpec>& v) {
-        int nk = 0;
+        int nk = 0, rc;
         const int n = (int)v.size();
-        std::vector<char> fwd_done(rseg.size(), 0);
-        for (int i = 0; i < n; ++i) {
-            const EvalSpec& e = v[i];
-            for (size_t q = 0; q < rseg.size(); ++q)
-                if (!fwd_done[q]) CUDA_TRY(launch_one<R>(0, e, rseg[q], stream, &nk));
-            if (e.demag && geom.any_demag)
-                for (auto& sg : cseg) CUDA_TRY(launch_one<R>(1, e, sg, stream, &nk));
-            for (size_t q = 0; q < rseg.size(); ++q) {
-                if (i + 1 < n && can_fuse<R>(e, v[i + 1], rseg[q])) {
-                    CUDA_TRY(launch_fused<R>(e, v[i + 1], rseg[q], stream, &nk));
-                    fwd_done[q] = 1;
-                } else {
-                    CUDA_TRY(launch_one<R>(2, e, rseg[q], stream, &nk));
-                    fwd_done[q] = 0;
-                }
-            }
+        auto fused = [&](int i, size_t q) { return i >= 0 && i + 1 < n && can_fuse<R>(v[i], v[i + 1], rseg[q]); };
+        for (int i = 0; i <= n; ++i) {
+            // rows: the end of stage i - 1 and the start of stage i, segment by segment
+            rc = each_segment(rseg.size(), [&](size_t q, cudaStream_t s) -> cudaError_t {
+                if (fused(i - 1, q)) return launch_fused<R>(v[i - 1], v[i], rseg[q], s, &nk);
+                cudaError_t e = i > 0 ? launch_one<R>(2, v[i - 1], rseg[q], s, &nk) : cudaSuccess;
+                if (e == cudaSuccess && i < n) e = launch_one<R>(0, v[i], rseg[q], s, &nk);
+                return e;
+            });
+            if (rc) return rc;
+            if (i < n && v[i].demag && geom.any_demag)
+                if ((rc = each_segment(cseg.size(), [&](size_t q, cudaStream_t s) {
+                         return launch_one<R>(1, v[i], cseg[q], s, &nk);
+                     })))
+                    return rc;
         }
         launches += nk;
         return LLG_OK;
@@ -755,6 +795,7 @@ struct Engine final : EngineBase {
                 }
             }
         }
+        if ((rc = create_side_streams())) return rc;
         if (any_demag && nf == 1) set_l2_window();
         if ((rc = autotune_grids(nsm_count()))) return rc;
         CUDA_TRY(cudaStreamSynchronize(stream));
@@ -1458,7 +1499,9 @@ struct Engine final : EngineBase {
         // Poll the device every 32 attempts.  With a step-count target no film can
         // finish in fewer attempts than its remaining steps, so a round launches at
         // most the smallest remaining count (graphs of 8 attempts, then single ones)
-        // and no attempt is launched after every film is done.
+        // and no attempt is launched after every film is done.  With an end time a round
+        // is no longer than the steps of the current size that are left of it (an idle
+        // attempt costs its launches, 25 to 45 us).
         const int reps = 8;
         cudaGraphExec_t ge = nullptr, ge1 = nullptr;
         if ((rc = attempt_graph(kind, fmask, reps, &ge))) return rc;
@@ -1468,12 +1511,20 @@ struct Engine final : EngineBase {
         long long round = 32;
         bool first = true;   // h_states predates set_control: every film is active in the first round
         for (;;) {
+            round = 32;
             if (n_acc > 0) {
-                round = 32;
                 for (int f = 0; f < nf; ++f)
                     if (first || h_states[f].active)
                         round = std::min(round, n_acc - (h_states[f].n_acc - acc0[f]));
                 round = std::max(round, 1LL);
+            } else if (std::isfinite(t_end)) {
+                double need = 1.0;
+                for (int f = 0; f < nf; ++f)
+                    if (first || h_states[f].active) {
+                        const double rem = t_end - (first ? 0.0 : h_states[f].t), dt = first ? p[f].dt : h_states[f].dt;
+                        need = std::max(need, dt > 0.0 ? std::floor(rem / dt) + 1.0 : 32.0);
+                    }
+                if (need < 32.0) round = (long long)need;
             }
             first = false;
             round = std::min(round, limit - launched);
