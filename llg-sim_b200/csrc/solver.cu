@@ -1100,6 +1100,10 @@ struct Engine final : EngineBase {
         return LLG_OK;
     }
 
+    // Blocks of the layout conversions: four per SM for a large film, no idle ones for a
+    // small one (a batch converts its films one by one).
+    int convert_grid(int f) const { return (int)std::min<int64_t>(592, (cells(f) + 255) / 256); }
+
     int ensure_stage() {
         if (!d_stage) return dalloc(&d_stage, sizeof(double) * 3 * (size_t)max_cells);
         return LLG_OK;
@@ -1147,11 +1151,11 @@ struct Engine final : EngineBase {
         int rc;
         if ((rc = ensure_stage())) return rc;
         CUDA_TRY(cudaMemcpyAsync(d_stage, m, sizeof(double) * 3 * (size_t)cells(f), cudaMemcpyHostToDevice, stream));
-        k_aos_to_soa<R><<<592, 256, 0, stream>>>(d_films, f, d_stage);
+        // FSAL validity of film f is decided on the device by k_aos_to_soa; the rest of
+        // the film's control state is set by every call that reads it
+        k_aos_to_soa<R><<<convert_grid(f), 256, 0, stream>>>(d_films, f, d_stage);
         CUDA_TRY(cudaGetLastError());
         launches += 1;
-        // FSAL validity of film f is decided on the device by k_aos_to_soa
-        if ((rc = set_control(idle_control(), nullptr, nullptr, true))) return rc;
         CUDA_TRY(cudaStreamSynchronize(stream));
         return LLG_OK;
     }
@@ -1183,7 +1187,7 @@ struct Engine final : EngineBase {
         if (format != LLG_OVF_BINARY4) return set_error(LLG_ERR_INVALID, "unknown OVF format %d", format);
         int rc;
         if ((rc = ensure_stage())) return rc;
-        k_soa_to_aos_f32<R><<<592, 256, 0, stream>>>(d_films, f, reinterpret_cast<float*>(d_stage));
+        k_soa_to_aos_f32<R><<<convert_grid(f), 256, 0, stream>>>(d_films, f, reinterpret_cast<float*>(d_stage));
         CUDA_TRY(cudaGetLastError());
         std::vector<float> payload(3 * (size_t)cells(f));
         CUDA_TRY(cudaMemcpyAsync(payload.data(), d_stage, sizeof(float) * payload.size(), cudaMemcpyDeviceToHost,
@@ -1195,7 +1199,7 @@ struct Engine final : EngineBase {
     int get_state(int f, double* m) override {
         int rc;
         if ((rc = ensure_stage())) return rc;
-        k_soa_to_aos<R><<<592, 256, 0, stream>>>(d_films, f, 0, d_stage);
+        k_soa_to_aos<R><<<convert_grid(f), 256, 0, stream>>>(d_films, f, 0, d_stage);
         CUDA_TRY(cudaGetLastError());
         CUDA_TRY(cudaMemcpyAsync(m, d_stage, sizeof(double) * 3 * (size_t)cells(f), cudaMemcpyDeviceToHost, stream));
         CUDA_TRY(cudaStreamSynchronize(stream));
@@ -1498,12 +1502,12 @@ struct Engine final : EngineBase {
         if ((rc = set_control(c, p, inv.get(), false))) return rc;
         // Poll the device every 32 attempts.  With a step-count target no film can
         // finish in fewer attempts than its remaining steps, so a round launches at
-        // most the smallest remaining count (graphs of 8 attempts, then single ones)
+        // most the smallest remaining count (graphs of 8 attempts, the rest one by one)
         // and no attempt is launched after every film is done.  With an end time a round
         // is no longer than the steps of the current size that are left of it (an idle
         // attempt costs its launches, 25 to 45 us).
         const int reps = 8;
-        cudaGraphExec_t ge = nullptr, ge1 = nullptr;
+        cudaGraphExec_t ge = nullptr;
         if ((rc = attempt_graph(kind, fmask, reps, &ge))) return rc;
         if ((rc = eval(stage1_spec(kind, fmask, 0)))) return rc;
         long long launched = 0;
@@ -1531,9 +1535,8 @@ struct Engine final : EngineBase {
             long long q = 0;
             for (; q + reps <= round; q += reps)
                 if ((rc = graph_launch(graph_key(kind, fmask, reps), ge))) return rc;
-            if (q < round && !ge1 && (rc = attempt_graph(kind, fmask, 1, &ge1))) return rc;
-            for (; q < round; ++q)
-                if ((rc = graph_launch(graph_key(kind, fmask, 1), ge1))) return rc;
+            for (; q < round; ++q)   // a single attempt is not worth a graph of its own
+                if ((rc = launch_attempt(kind, fmask, 0))) return rc;
             launched += round;
             if ((rc = read_states())) return rc;
             bool any = false;
@@ -1627,17 +1630,25 @@ struct Engine final : EngineBase {
         // of rejections, so this bound is only a safety net against a stuck film.
         const long long max_iters = 16 * std::max<long long>(st->max_accepted_steps, 1) + 1000000;
         long long iters = 0;
+        int per_poll = 4;
         for (;;) {
-            for (int q = 0; q < 4; ++q)
+            for (int q = 0; q < per_poll; ++q)
                 if ((rc = graph_launch(key, ge))) return rc;
-            iters += 4 * reps;
+            iters += per_poll * reps;
             if (iters > max_iters)
                 return set_error(LLG_ERR_TIMEOUT, "relax did not finish within %lld iterations", max_iters);
             CUDA_TRY(cudaMemcpyAsync(h_relax, d_relax, sizeof(RelaxStateDev) * nf, cudaMemcpyDeviceToHost, stream));
             if ((rc = read_states())) return rc;
             bool all = true;
-            for (int f = 0; f < nf; ++f) all &= (h_relax[f].done != 0) || h_states[f].err_code != 0;
+            // poll earlier where max_accepted_steps leaves fewer steps than a round
+            long long left = 1;
+            for (int f = 0; f < nf; ++f) {
+                const bool done = (h_relax[f].done != 0) || h_states[f].err_code != 0;
+                all &= done;
+                if (!done) left = std::max(left, st->max_accepted_steps - h_relax[f].accepted + 1);
+            }
             if (all) break;
+            per_poll = (int)std::min<long long>(4, (left + reps - 1) / reps);
         }
         for (int f = 0; f < nf; ++f) {
             const RelaxStateDev& Q = h_relax[f];
@@ -1719,7 +1730,9 @@ struct Engine final : EngineBase {
             for (int q = 0; q < per_poll; ++q)
                 if ((rc = graph_launch(key, ge))) return rc;
             iters += (long long)per_poll * reps;
-            per_poll = std::min(per_poll * 2, 8);
+            // no more than max_iters leaves to do: a finished film's iteration still costs its launches
+            per_poll = (int)std::max<long long>(
+                1, std::min<long long>(std::min(per_poll * 2, 8), (st->max_iters - iters + reps - 1) / reps));
             CUDA_TRY(cudaMemcpyAsync(h_min, d_min, sizeof(MinimizeStateDev) * nf, cudaMemcpyDeviceToHost, stream));
             CUDA_TRY(cudaStreamSynchronize(stream));
             all = true;
@@ -1773,7 +1786,7 @@ struct Engine final : EngineBase {
         EvalSpec e = base_spec(fmask);
         e.rhs = RHS_FIELD;
         if ((rc = eval_resident(e))) return rc;
-        k_soa_to_aos<R><<<592, 256, 0, stream>>>(d_films, f, 1, d_stage);
+        k_soa_to_aos<R><<<convert_grid(f), 256, 0, stream>>>(d_films, f, 1, d_stage);
         CUDA_TRY(cudaGetLastError());
         CUDA_TRY(cudaMemcpyAsync(b, d_stage, sizeof(double) * 3 * (size_t)cells(f), cudaMemcpyDeviceToHost, stream));
         CUDA_TRY(cudaStreamSynchronize(stream));
@@ -1792,7 +1805,7 @@ struct Engine final : EngineBase {
         e.rhs = RHS_FIELD;
         e.local = 0;
         if ((rc = eval_resident(e))) return rc;
-        k_soa_to_aos<R><<<592, 256, 0, stream>>>(d_films, f, 1, d_stage);
+        k_soa_to_aos<R><<<convert_grid(f), 256, 0, stream>>>(d_films, f, 1, d_stage);
         CUDA_TRY(cudaGetLastError());
         CUDA_TRY(cudaMemcpyAsync(b, d_stage, sizeof(double) * 3 * (size_t)cells(f), cudaMemcpyDeviceToHost, stream));
         CUDA_TRY(cudaStreamSynchronize(stream));
