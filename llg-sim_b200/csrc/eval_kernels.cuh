@@ -115,6 +115,8 @@ cudaError_t prepare_eval_kernels(size_t smem_row, size_t smem_col) {
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k_row_inverse<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row);
     if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(k_row_fused_generic<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row);
+    if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k_column<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_col);
     if (e != cudaSuccess) return e;
     // fast kernels: every instantiation whose shared memory fits; the whole unified
@@ -204,13 +206,15 @@ cudaError_t launch_one(int which, const EvalSpec& spec, const LaunchGeom& g, cud
 
 template <typename R>
 bool can_fuse(const EvalSpec& si, const EvalSpec& sf, const LaunchGeom& g) {
-    return g.fast_row != 0 && g.fuse_rows && lean_epilogue(si) && si.k_out != KB_NONE && !si.skip_if_fsal &&
+    return g.fuse_rows && lean_epilogue(si) && si.k_out != KB_NONE && !si.skip_if_fsal &&
            !sf.skip_if_fsal && sf.nterm >= 1 && sf.nterm <= 6 && sf.kidx[sf.nterm - 1] == si.k_out &&
            sf.req == si.req && sf.demag == si.demag && sf.m_in != si.m_in;
 }
 
 template <typename R>
 cudaError_t launch_fused(const EvalSpec& si, const EvalSpec& sf, const LaunchGeom& g, cudaStream_t s, int* nk) {
+    if (!g.fast_row)
+        k_row_fused_generic<R><<<g.grid_row, 256, g.smem_row, s>>>(g.films, g.row_items, g.n_row_items, si, sf);
     dispatch_LV<R>(g.fast_row, g.row_var, [&](auto LC, auto VC) {
         constexpr int L = decltype(LC)::value, V = decltype(VC)::value;
         if constexpr (RowCfg<R, L, V>::SMEM <= kSmemMax) {

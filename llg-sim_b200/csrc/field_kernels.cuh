@@ -410,10 +410,105 @@ __device__ __forceinline__ double warp_max(double v) {
 }
 
 // ---------------------------------------------------------------------------
+// Transforms of a row block of the generic kernels.  Signals: x + i y of row r in
+// buffer 2r, z of rows 2p, 2p+1 in buffer 2(T + p); the odd-bin half of each in the
+// buffer after it.
+// ---------------------------------------------------------------------------
+// Zero-padded R2C along x of the signals in A (even buffers filled) to X; B scratch.
+template <typename R>
+__device__ __forceinline__ void generic_rows_forward(const FilmDev& F, cx<R>* A, cx<R>* B, int j0) {
+    const int nx = F.nx, ny = F.ny, T = F.rows_per_block, L = nx;
+    const int G = T + (T + 1) / 2;
+    const FftPlan& PL = F.plan_row;
+    const int LP = PL.stride();
+    const cx<R>* __restrict__ tw = reinterpret_cast<const cx<R>*>(F.tw_row);
+    const cx<R>* __restrict__ twg = reinterpret_cast<const cx<R>*>(F.twg_row);
+    for (int e = threadIdx.x; e < G * L; e += blockDim.x) {
+        const int g = e / L, i = e - g * L;
+        A[(2 * g + 1) * LP + PL.at(i)] = cmul(A[(2 * g) * LP + PL.at(i)], tw[i]);
+    }
+    __syncthreads();
+    cx<R>* res = fft_smem<R, false>(A, B, 2 * G, PL, twg, tw);
+    cx<R>* __restrict__ X = reinterpret_cast<cx<R>*>(F.X);
+    const int K1 = nx + 1;
+    const int L2 = 2 * L;
+    for (int e = threadIdx.x; e < 3 * K1 * T; e += blockDim.x) {
+        const int r = e % T, rest = e / T;
+        const int c = rest / K1, k = rest - c * K1;
+        const int j = j0 + r;
+        if (j >= ny) continue;
+        int g, half;
+        if (c < 2) { g = r; half = c; }
+        else { g = T + r / 2; half = r & 1; }
+        const int km = k ? L2 - k : 0;
+        cx<R> zk = res[(2 * g + (k & 1)) * LP + PL.at(k >> 1)];
+        cx<R> zm = res[(2 * g + (km & 1)) * LP + PL.at(km >> 1)];
+        cx<R> out;
+        if (half == 0) out = mkc((R)0.5 * (zk.re + zm.re), (R)0.5 * (zk.im - zm.im));
+        else out = mkc((R)0.5 * (zk.im + zm.im), (R)0.5 * (zm.re - zk.re));
+        X[(c * K1 + k) * ny + j] = out;
+    }
+}
+
+// C2R along x of the block's rows of X, keeping nx cells: D[(r * 3 + c) * nx + i].
+// D lies in one half of the block's buffers; *spare receives the other half.
+template <typename R>
+__device__ __forceinline__ R* generic_rows_inverse(const FilmDev& F, cx<R>* sm, int j0, cx<R>** spare) {
+    const int nx = F.nx, ny = F.ny, T = F.rows_per_block;
+    const int L = nx, K1 = nx + 1, L2 = 2 * nx;
+    const int G = T + (T + 1) / 2, P = (T + 1) / 2;
+    const cx<R>* __restrict__ tw = reinterpret_cast<const cx<R>*>(F.tw_row);
+    const cx<R>* __restrict__ X = reinterpret_cast<const cx<R>*>(F.X);
+    const cx<R>* __restrict__ twg = reinterpret_cast<const cx<R>*>(F.twg_row);
+    const FftPlan& PL = F.plan_row;
+    const int LP = PL.stride();
+    cx<R>* A = sm;
+    cx<R>* B = sm + 2 * G * LP;
+    auto xval = [&](int c, int k, int j) -> cx<R> {
+        if (k <= nx) return X[(c * K1 + k) * ny + j];
+        return conjc(X[(c * K1 + (L2 - k)) * ny + j]);
+    };
+    for (int e = threadIdx.x; e < L2 * T; e += blockDim.x) {
+        const int r = e % T, k = e / T, j = j0 + r;
+        cx<R> z = mkc((R)0, (R)0);
+        if (j < ny) {
+            cx<R> bx = xval(0, k, j), by = xval(1, k, j);
+            z = mkc(bx.re - by.im, bx.im + by.re);
+        }
+        A[(2 * r + (k & 1)) * LP + PL.at(k >> 1)] = z;
+    }
+    for (int e = threadIdx.x; e < L2 * P; e += blockDim.x) {
+        const int p = e % P, k = e / P;
+        const int ja = j0 + 2 * p, jb = j0 + 2 * p + 1;
+        cx<R> za = (ja < ny) ? xval(2, k, ja) : mkc((R)0, (R)0);
+        cx<R> zb = (2 * p + 1 < T && jb < ny) ? xval(2, k, jb) : mkc((R)0, (R)0);
+        A[(2 * (T + p) + (k & 1)) * LP + PL.at(k >> 1)] = mkc(za.re - zb.im, za.im + zb.re);
+    }
+    __syncthreads();
+    cx<R>* res = fft_smem<R, true>(A, B, 2 * G, PL, twg, tw);
+    R* D = reinterpret_cast<R*>(res == A ? B : A);
+    for (int e = threadIdx.x; e < G * L; e += blockDim.x) {
+        const int g = e / L, x = e - g * L;
+        cx<R> z = res[(2 * g) * LP + PL.at(x)] + cmulc(res[(2 * g + 1) * LP + PL.at(x)], tw[x]);
+        if (g < T) {
+            D[(g * 3 + 0) * L + x] = z.re;
+            D[(g * 3 + 1) * L + x] = z.im;
+        } else {
+            const int p = g - T;
+            D[((2 * p) * 3 + 2) * L + x] = z.re;
+            if (2 * p + 1 < T) D[((2 * p + 1) * 3 + 2) * L + x] = z.im;
+        }
+    }
+    __syncthreads();
+    *spare = res;
+    return D;
+}
+
+// ---------------------------------------------------------------------------
 // Pass 1: stage combination + zero-padded R2C along x.
 // ---------------------------------------------------------------------------
 template <typename R>
-__global__ void __launch_bounds__(256) k_row_forward(const FilmDev* __restrict__ films,
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 0 : 2) k_row_forward(const FilmDev* __restrict__ films,
                                                      const WorkItem* __restrict__ items, int nitems, EvalSpec spec) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cx<R>* sm = reinterpret_cast<cx<R>*>(smem_raw);
@@ -437,14 +532,11 @@ __global__ void __launch_bounds__(256) k_row_forward(const FilmDev* __restrict__
         }
         const bool do_fft = spec.demag && F.demag_mat;
         const R Ms = (R)F.ms;
-        const int L = nx;
         const int G = T + (T + 1) / 2;
         const FftPlan& PL = F.plan_row;
         const int LP = PL.stride();
         cx<R>* A = sm;
         cx<R>* B = sm + 2 * G * LP;
-        const cx<R>* __restrict__ tw = reinterpret_cast<const cx<R>*>(F.tw_row);
-        const cx<R>* __restrict__ twg = reinterpret_cast<const cx<R>*>(F.twg_row);
         for (int e = threadIdx.x; e < T * nx; e += blockDim.x) {
             const int r = e / nx, i = e - r * nx, j = j0 + r;
             R v[3] = {(R)0, (R)0, (R)0};
@@ -481,31 +573,7 @@ __global__ void __launch_bounds__(256) k_row_forward(const FilmDev* __restrict__
         }
         if (!do_fft) continue;
         __syncthreads();
-        for (int e = threadIdx.x; e < G * L; e += blockDim.x) {
-            const int g = e / L, i = e - g * L;
-            A[(2 * g + 1) * LP + PL.at(i)] = cmul(A[(2 * g) * LP + PL.at(i)], tw[i]);
-        }
-        __syncthreads();
-        cx<R>* res = fft_smem<R, false>(A, B, 2 * G, PL, twg, tw);
-        cx<R>* __restrict__ X = reinterpret_cast<cx<R>*>(F.X);
-        const int K1 = nx + 1;
-        const int L2 = 2 * L;
-        for (int e = threadIdx.x; e < 3 * K1 * T; e += blockDim.x) {
-            const int r = e % T, rest = e / T;
-            const int k = rest % K1, c = rest / K1;
-            const int j = j0 + r;
-            if (j >= ny) continue;
-            int g, half;
-            if (c < 2) { g = r; half = c; }
-            else { g = T + r / 2; half = r & 1; }
-            const int km = k ? L2 - k : 0;
-            cx<R> zk = res[(2 * g + (k & 1)) * LP + PL.at(k >> 1)];
-            cx<R> zm = res[(2 * g + (km & 1)) * LP + PL.at(km >> 1)];
-            cx<R> out;
-            if (half == 0) out = mkc((R)0.5 * (zk.re + zm.re), (R)0.5 * (zk.im - zm.im));
-            else out = mkc((R)0.5 * (zk.im + zm.im), (R)0.5 * (zm.re - zk.re));
-            X[(c * K1 + k) * ny + j] = out;
-        }
+        generic_rows_forward<R>(F, A, B, j0);
         __syncthreads();
     }
 }
@@ -514,7 +582,7 @@ __global__ void __launch_bounds__(256) k_row_forward(const FilmDev* __restrict__
 // Pass 2: y transform, kernel multiply, inverse y transform (one kx column).
 // ---------------------------------------------------------------------------
 template <typename R>
-__global__ void __launch_bounds__(256) k_column(const FilmDev* __restrict__ films, const WorkItem* __restrict__ items,
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 0 : 2) k_column(const FilmDev* __restrict__ films, const WorkItem* __restrict__ items,
                                                 int nitems, EvalSpec spec) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cx<R>* sm = reinterpret_cast<cx<R>*>(smem_raw);
@@ -765,57 +833,10 @@ __global__ void __launch_bounds__(256) k_row_inverse(const FilmDev* __restrict__
         const FilmDev& F = films[w.film];
         StepState* st = F.st;
         if (skip_item(spec, st)) continue;
-        const int nx = F.nx, ny = F.ny, T = F.rows_per_block;
-        const int j0 = w.blk * T;
-        const int L = nx, K1 = nx + 1, L2 = 2 * nx;
-        const int G = T + (T + 1) / 2, P = (T + 1) / 2;
+        const int T = F.rows_per_block, L = F.nx;
         const bool do_fft = spec.demag && F.demag_mat;
-        const cx<R>* __restrict__ tw = reinterpret_cast<const cx<R>*>(F.tw_row);
-        R* D = nullptr;
-        if (do_fft) {
-            const cx<R>* __restrict__ X = reinterpret_cast<const cx<R>*>(F.X);
-            const cx<R>* __restrict__ twg = reinterpret_cast<const cx<R>*>(F.twg_row);
-            const FftPlan& PL = F.plan_row;
-            const int LP = PL.stride();
-            cx<R>* A = sm;
-            cx<R>* B = sm + 2 * G * LP;
-            auto xval = [&](int c, int k, int j) -> cx<R> {
-                if (k <= nx) return X[(c * K1 + k) * ny + j];
-                return conjc(X[(c * K1 + (L2 - k)) * ny + j]);
-            };
-            for (int e = threadIdx.x; e < L2 * T; e += blockDim.x) {
-                const int r = e % T, k = e / T, j = j0 + r;
-                cx<R> z = mkc((R)0, (R)0);
-                if (j < ny) {
-                    cx<R> bx = xval(0, k, j), by = xval(1, k, j);
-                    z = mkc(bx.re - by.im, bx.im + by.re);
-                }
-                A[(2 * r + (k & 1)) * LP + PL.at(k >> 1)] = z;
-            }
-            for (int e = threadIdx.x; e < L2 * P; e += blockDim.x) {
-                const int p = e % P, k = e / P;
-                const int ja = j0 + 2 * p, jb = j0 + 2 * p + 1;
-                cx<R> za = (ja < ny) ? xval(2, k, ja) : mkc((R)0, (R)0);
-                cx<R> zb = (2 * p + 1 < T && jb < ny) ? xval(2, k, jb) : mkc((R)0, (R)0);
-                A[(2 * (T + p) + (k & 1)) * LP + PL.at(k >> 1)] = mkc(za.re - zb.im, za.im + zb.re);
-            }
-            __syncthreads();
-            cx<R>* res = fft_smem<R, true>(A, B, 2 * G, PL, twg, tw);
-            D = reinterpret_cast<R*>(res == A ? B : A);
-            for (int e = threadIdx.x; e < G * L; e += blockDim.x) {
-                const int g = e / L, x = e - g * L;
-                cx<R> z = res[(2 * g) * LP + PL.at(x)] + cmulc(res[(2 * g + 1) * LP + PL.at(x)], tw[x]);
-                if (g < T) {
-                    D[(g * 3 + 0) * L + x] = z.re;
-                    D[(g * 3 + 1) * L + x] = z.im;
-                } else {
-                    const int p = g - T;
-                    D[((2 * p) * 3 + 2) * L + x] = z.re;
-                    if (2 * p + 1 < T) D[((2 * p + 1) * 3 + 2) * L + x] = z.im;
-                }
-            }
-            __syncthreads();
-        }
+        cx<R>* spare;
+        const R* D = do_fft ? generic_rows_inverse<R>(F, sm, w.blk * T, &spare) : nullptr;
         auto dfield = [&](int r, int i, int c) -> R { return D[(r * 3 + c) * L + i]; };
         row_epilogue<R, MIN>(F, spec, st, w.blk, T, do_fft, dfield, sm_red);
         __syncthreads();

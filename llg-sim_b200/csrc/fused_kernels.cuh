@@ -296,4 +296,108 @@ __global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS) __maxnreg__((RowCfg<
     }
 }
 
+// The same row pass for films whose nx has no register FFT: the transforms of the
+// generic kernels (shared-memory Stockham) around one cell per thread and step.  It
+// replaces two launches by one; its loads of a step are all in flight together, and
+// the field and torque arithmetic needs neither the reductions nor the FP64 of the
+// full epilogue.  Same operations in the same order as the unfused kernels.
+template <typename R>
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) k_row_fused_generic(const FilmDev* __restrict__ films,
+                                                              const WorkItem* __restrict__ items, int nitems,
+                                                              EvalSpec si, EvalSpec sf) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    cx<R>* sm = reinterpret_cast<cx<R>*>(smem_raw);
+    for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
+        const WorkItem w = items[it];
+        const FilmDev& F = films[w.film];
+        const StepState* st = F.st;
+        if (skip_item(si, st)) continue;   // uniform over the block
+        const bool do_fft = si.demag && F.demag_mat;
+        const int nx = F.nx, ny = F.ny, n = nx * ny, T = F.rows_per_block, j0 = w.blk * T;
+        const int cur = st->cur;
+        const FftPlan& PL = F.plan_row;
+        const int LP = PL.stride();
+        cx<R>* A = nullptr;   // signals of the forward transform, in the half D does not use
+        const R* D = do_fft ? generic_rows_inverse<R>(F, sm, j0, &A) : nullptr;
+        const R* __restrict__ msb = mbuf<R>(F, si.m_in, cur);
+        const R* __restrict__ m0 = mbuf<R>(F, MB_M0, cur);
+        R* __restrict__ kout = kbuf<R>(F, si.k_out, cur);
+        R* __restrict__ mnext = mbuf<R>(F, sf.m_in, cur);
+        const double dt = st->dt;
+        const R gam = (R)F.gamma, alp = (R)F.alpha;
+        const R denom = (R)1 + alp * alp;
+        const R pref = si.rhs == RHS_LLG ? -gam / denom : -gam * alp / denom;
+        const R c1 = si.rhs == RHS_LLG ? (R)1 : (R)0;
+        const R c2 = si.rhs == RHS_LLG ? alp : (R)1;
+        const int nq = sf.nterm - 1;   // terms read from HBM; the last one is k_s
+        const R* kp[5];
+        R cq[5];
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+            kp[q] = q < nq ? kbuf<R>(F, sf.kidx[q], cur) : nullptr;
+            cq[q] = q < nq ? (R)(dt * sf.a[q]) : (R)0;
+        }
+        const R cs = (R)(dt * sf.a[nq]);
+        const R Ms = (R)F.ms;
+        const LocalCoef<R> cf = local_coef<R>(F, si.dmi != 0);
+        for (int e = threadIdx.x; e < T * nx; e += blockDim.x) {
+            const int r = e / nx, i = e - r * nx, j = j0 + r;
+            R v[3] = {(R)0, (R)0, (R)0};   // rows past the film are zero in the forward transform
+            if (j < ny) {
+                const int idx = j * nx + i;
+                R a[3], kq[5][3], mc[3], b[3], k[3];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) a[c] = m0[c * n + idx];
+#pragma unroll
+                for (int q = 0; q < 5; ++q)
+                    if (q < nq)
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) kq[q][c] = kp[q][c * n + idx];
+                ld3(msb, n, idx, mc);
+                local_field_c<R>(
+                    cf,
+                    [&](int d, R* o) {
+                        ld3(msb, n, d == 0 ? idx - 1 : d == 1 ? idx + 1 : d == 2 ? idx - nx : idx + nx, o);
+                    },
+                    i, j, mc, b);
+                if (do_fft) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) b[c] += D[(r * 3 + c) * nx + i];
+                }
+                torque_cell<R>(mc, b, pref, c1, c2, k);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    kout[c * n + idx] = k[c];
+                    v[c] = a[c];
+                }
+#pragma unroll
+                for (int q = 0; q < 5; ++q)
+                    if (q < nq)
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) v[c] = v[c] + cq[q] * kq[q][c];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) v[c] = v[c] + cs * k[c];
+                if (coef_inside(cf, idx)) normalize3(v);
+                else { v[0] = (R)0; v[1] = (R)0; v[2] = (R)0; }   // vacuum pinned at m = 0
+#pragma unroll
+                for (int c = 0; c < 3; ++c) mnext[c * n + idx] = v[c];
+            }
+            if (do_fft) {
+                A[(2 * r) * LP + PL.at(i)] = mkc(Ms * v[0], Ms * v[1]);
+                cx<R>* zp = &A[(2 * (T + r / 2)) * LP + PL.at(i)];
+                if ((r & 1) == 0) {
+                    zp->re = Ms * v[2];
+                    if (r + 1 >= T) zp->im = (R)0;
+                } else {
+                    zp->im = Ms * v[2];
+                }
+            }
+        }
+        if (!do_fft) continue;
+        __syncthreads();
+        generic_rows_forward<R>(F, A, A == sm ? sm + 2 * (T + (T + 1) / 2) * LP : sm, j0);
+        __syncthreads();
+    }
+}
+
 }  // namespace llg

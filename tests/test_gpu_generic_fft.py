@@ -9,7 +9,7 @@ from helpers import case, gpu_solver, oracle_solver, random_m, rel_err
 pytestmark = pytest.mark.gpu
 TOL = {0: 2e-5, 1: 1e-9}   # the parity tests' bounds for demag fields
 
-# radices 2..16 alone and combined; 7 and 13 as passes of their own; 1200 in FP64 is
+# radices 2..16 alone and combined; 7 and 13 as passes of their own; 1152 in FP64 is
 # too long for padded signals
 SHAPES = [(6, 10), (12, 5), (48, 60), (80, 36), (144, 15), (240, 14), (7, 26), (192, 20), (250, 9)]
 
@@ -26,7 +26,7 @@ def test_demag_field_of_generic_lengths(orc, gpu, nx, ny, prec):
 
 
 def test_longest_double_precision_rows(orc, gpu):
-    nx, ny = 1200, 2
+    nx, ny = 1152, 2
     c = case(nx, ny)
     o, g = oracle_solver(orc, c), gpu_solver(gpu, c, 1)
     m = random_m(orc, nx * ny, 5)
