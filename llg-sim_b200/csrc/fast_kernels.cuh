@@ -83,15 +83,16 @@ struct ColCfg {
 };
 
 // Staged spectrum of a row block, [c][k][r] in 16-byte pieces (PER complex values).
-// With two rows per block a warp of the inverse transform reads every other piece,
-// which put its lanes on a quarter of the shared-memory banks; the piece slot is
-// XOR-swizzled within each group of eight so that the lanes spread over all of
-// them.  The slots of a group stay in the group, so the staging area needs the
-// piece count rounded up to a multiple of eight.
+// A warp of the inverse transform reads one row of every other k, pieces 2 T / PER
+// slots apart: without more, 8 (two rows per block in FP32) to all 32 of its lanes
+// (eight rows and more) fall on the same banks.  The slot of a piece is XOR-swizzled
+// within its group of eight by bits of the group's number, as many as it takes: one
+// or two for two rows, three for more, which leaves at most 4 wavefronts.  The slots of
+// a group stay in the group, so the staging area needs the piece count rounded up to
+// a multiple of eight.
 template <typename R, int T>
 __host__ __device__ __forceinline__ int stage_slot(int p) {
-    if constexpr (T == 2) return p ^ ((p >> 3) & (sizeof(R) == 4 ? 1 : 3));
-    else return p;
+    return p ^ ((p >> 3) & (T > 2 ? 7 : sizeof(R) == 4 ? 1 : 3));
 }
 template <typename R, int T>
 __host__ __device__ __forceinline__ int stage_index(int e) {
@@ -503,17 +504,13 @@ __global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS) __maxnreg__((MODE ==
             }
             cp_async_wait_all();
             __syncthreads();
-            static_assert(T != 2 || (2 * G * T / PER) % 32 == 0, "swizzle needs 32-piece strides");
+            static_assert((2 * G * T / PER) % (T == 2 ? 32 : 64) == 0, "swizzle strides");
             const int kb = 2 * t + par;
             auto xval = [&](int c, int rr, int k, int r) -> cx<R> {
                 // k = kb + 2*G*rr: the swizzle of a slot depends only on the bits below
                 // 2*G*T/PER pieces, so the slots of a thread are its slot at rr = 0 plus
                 // a constant per rr (immediate offsets, no per-value swizzle)
                 const int off = 2 * G * rr * T;
-                if constexpr (T != 2) {   // identity slots
-                    if (k <= L) return stg[(c * K1 + k) * T + r];
-                    return conjc(stg[(c * K1 + (L2 - k)) * T + r]);
-                }
                 if (k <= L) return stg[stage_index<R, T>((c * K1 + kb) * T + r) + off];
                 return conjc(stg[stage_index<R, T>((c * K1 + (L2 - kb)) * T + r) - off]);
             };

@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS) __maxnreg__((RowCfg<
             }
             cp_async_wait_all();
             __syncthreads();
-            static_assert(T != 2 || (2 * G * T / PER) % 32 == 0, "swizzle needs 32-piece strides");
+            static_assert((2 * G * T / PER) % (T == 2 ? 32 : 64) == 0, "swizzle strides");
             const int kb = 2 * t + par;
             auto xval = [&](int c, int rr, int k, int r) -> cx<R> {
                 // k = kb + 2*G*rr: the swizzle of a slot depends only on the bits below
