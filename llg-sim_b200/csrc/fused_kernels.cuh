@@ -33,14 +33,15 @@ __global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS) __maxnreg__((RowCfg<
     using FF = GroupFFT<R, L, false, V>;
     using FI = GroupFFT<R, L, true, V>;
     constexpr int G = C::G, E = C::E, T = C::T, BUF = C::BUF;
-    // phase 2 takes W = 2 cells per step of its loop: the stencil (and, with EARLY,
-    // m0 and the previous torques) of both cells are loaded before any arithmetic
-    constexpr int W = 2, NV = T * L / W;
+    // phase 2 takes W cells per step of its loop, two in FP32 and one in FP64 (the same
+    // registers): with EARLY the stencil, m0 and the previous torques of a step are all
+    // loaded before any arithmetic, one memory round trip per step instead of one per
+    // term.  Plan 1 and the 384-thread FP64 blocks have too few registers for that: they
+    // load the torques where they are used and take the general path for interior
+    // cells too.
+    constexpr int W = sizeof(R) == 4 ? 2 : 1, NV = T * L / W;
     using VW = VecW<R, W>;
-    // the early loads of the combination's torques and the ghost-free path of
-    // interior cells need the registers of the FP32 plan-0 budget; the other
-    // instantiations load the torques where they are used and take the general path
-    constexpr bool EARLY = sizeof(R) == 4 && V == 0;
+    constexpr bool EARLY = V == 0 && (sizeof(R) == 4 || C::REG2 > 200);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cx<R>* buf = reinterpret_cast<cx<R>*>(smem_raw);
     cx<R>* twp = buf + C::NSIG * BUF;
