@@ -74,12 +74,11 @@ struct ColCfg {
     static constexpr size_t OFF_XST = al16(OFF_PRE + (LEAN ? 0 : sizeof(cx<R>) * (size_t)L));
     static constexpr size_t OFF_KST = al16(OFF_XST + sizeof(cx<R>) * 3 * (size_t)NC * L);
     static constexpr size_t SMEM = al16(OFF_KST + (LEAN ? 0 : sizeof(r4<R>) * (size_t)NC * (L + 1)));
-    // register cap: plan 1 (half the registers per thread) for two resident blocks,
-    // the lean FP32 form of 192-thread blocks for three (its shared memory allows
-    // three), one block otherwise
-    static constexpr int MAXREG = V == 1 ? regs_for_blocks(THREADS, 2)
-                                         : (LEAN && sizeof(R) == 4 && THREADS <= 192) ? regs_for_blocks(THREADS, 3)
-                                                                                      : regs_for_blocks(THREADS, 1);
+    // register cap: two resident blocks for plan 1 (half the registers per thread) and
+    // for the 192-thread FP32 blocks (three for their lean form; their shared memory
+    // allows as many), one block otherwise
+    static constexpr int MAXREG =
+        regs_for_blocks(THREADS, V == 1 ? 2 : (sizeof(R) == 4 && THREADS <= 192) ? (LEAN ? 3 : 2) : 1);
 };
 
 // Staged spectrum of a row block, [c][k][r] in 16-byte pieces (PER complex values).
@@ -417,13 +416,13 @@ __global__ void __launch_bounds__(ColCfg<R, L, V, LEAN>::THREADS) __maxnreg__((C
                 cx<R> out;
                 if (comp == 0) {
                     const cx<R> Mx = sx[pi], My = sy[pi];
-                    out = mkc(K.x * Mx.re + kxy * My.re, K.x * Mx.im + kxy * My.im);
+                    out = cmix(K.x, Mx, kxy, My);
                 } else if (comp == 1) {
                     const cx<R> Mx = sx[pi], My = sy[pi];
-                    out = mkc(kxy * Mx.re + K.z * My.re, kxy * Mx.im + K.z * My.im);
+                    out = cmix(kxy, Mx, K.z, My);
                 } else {
                     const cx<R> Mz = sz[pi];
-                    out = mkc(K.w * Mz.re, K.w * Mz.im);
+                    out = cscale(Mz, K.w);
                 }
                 v[r] = out;
             }

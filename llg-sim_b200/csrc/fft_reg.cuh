@@ -48,7 +48,7 @@ __device__ __forceinline__ cx<R> twc(cx<R> x) {
     } else {
         constexpr double c = kCos64[j];
         constexpr double s = INV ? kCos64[(j + 48) % 64] : -kCos64[(j + 48) % 64];  // +/- sin(2 pi j/64)
-        return mkc((R)c * x.re - (R)s * x.im, (R)c * x.im + (R)s * x.re);
+        return cmul(x, mkc((R)c, (R)s));
     }
 }
 

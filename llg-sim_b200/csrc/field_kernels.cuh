@@ -60,7 +60,7 @@ __device__ __forceinline__ R* kbuf(const FilmDev& F, int id, int cur) {
 template <typename R>
 __device__ __forceinline__ void normalize3(R* v) {
     // vec3::normalize (vec3.rs:21-28): zero maps to +z
-    R n2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
+    const R n2 = fma_rn(v[2], v[2], fma_rn(v[1], v[1], mul_rn(v[0], v[0])));
     if (n2 == (R)0) {
         v[0] = (R)0; v[1] = (R)0; v[2] = (R)1;
         return;
@@ -153,18 +153,6 @@ template <typename R>
 __device__ __forceinline__ bool coef_inside(const LocalCoef<R>& c, int idx) {
     return c.mask == nullptr || c.mask[idx] != 0;
 }
-
-// Rounded operations that the compiler may not fuse or reorder: the cores below
-// spell out every product, sum and fused multiply-add, so a cell's field has the
-// same bits whichever kernel (and whichever surrounding code) evaluates it.
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
-__device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
-__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
 
 // Arithmetic of the exchange (exchange.rs:45-222), anisotropy (anisotropy.rs:10-26)
 // and DMI (dmi.rs:67-209) terms of one cell from its four neighbour values (real
@@ -618,9 +606,9 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 0 : 2) k_column(const Fi
             const R kxy = ky <= ny ? K.y : -K.y;
             cx<R>* pr = res + par * LP + PL.at(kk);
             const cx<R> Mx = pr[0], My = pr[2 * LP], Mz = pr[4 * LP];
-            pr[0] = mkc(K.x * Mx.re + kxy * My.re, K.x * Mx.im + kxy * My.im);
-            pr[2 * LP] = mkc(kxy * Mx.re + K.z * My.re, kxy * Mx.im + K.z * My.im);
-            pr[4 * LP] = mkc(K.w * Mz.re, K.w * Mz.im);
+            pr[0] = cmix(K.x, Mx, kxy, My);
+            pr[2 * LP] = cmix(kxy, Mx, K.z, My);
+            pr[4 * LP] = cscale(Mz, K.w);
         }
         __syncthreads();
         cx<R>* other = (res == A) ? B : A;
