@@ -106,6 +106,103 @@ __device__ __forceinline__ void load_tables(cx<R>* twp, const cx<R>* __restrict_
     for (int i = threadIdx.x; i < L; i += blockDim.x) pre[i] = gpre[i];
 }
 
+// Stages the spectrum of a block's rows, [c][k][r] in swizzled 16-byte pieces with
+// contiguous T-row chunks per (c, k), into the signal buffers (free here).
+template <typename R, int L, int V>
+__device__ __forceinline__ void row_stage_spectrum(const cx<R>* __restrict__ X, cx<R>* stg, int ny, int j0) {
+    using C = RowCfg<R, L, V>;
+    constexpr int T = C::T, PER = 16 / (int)sizeof(cx<R>), TP = T / PER;
+    for (int p = threadIdx.x; p < 3 * (L + 1) * TP; p += C::THREADS) {
+        const int ck = p / TP, r = p % TP * PER;
+        cx<R>* dst = stg + stage_slot<R, T>(p) * PER;
+        if (j0 + r < ny) {
+            cp_async16(dst, X + (size_t)ck * ny + j0 + r);
+        } else {
+#pragma unroll
+            for (int q = 0; q < PER; ++q) dst[q] = mkc((R)0, (R)0);
+        }
+    }
+    cp_async_wait_all();
+}
+
+// Inputs of a group's inverse transform from the staged spectrum: signal g < T is
+// x + i y of row g, the others z of two rows; the group of parity par takes the bins
+// k = 2 (t + G r) + par.  Bins up to L are stored, the ones above are conjugates of
+// bin 2L - k: r < E / 2 lies below L for every thread and r >= E / 2 above, but for
+// k = L itself (r = E / 2, t = 0, even bins), whose mirror image it is, unconjugated.
+// So each r has one address, a constant away from the thread's first (the swizzle of
+// a slot depends on the bits below 2 G T / PER pieces only).
+template <typename R, int L, int V>
+__device__ __forceinline__ void row_load_inverse(const cx<R>* stg, cx<R> (&v)[RowCfg<R, L, V>::E], int t, int g, int par) {
+    using C = RowCfg<R, L, V>;
+    constexpr int G = C::G, E = C::E, T = C::T, K1 = L + 1, PER = 16 / (int)sizeof(cx<R>);
+    static_assert((2 * G * T / PER) % (T == 2 ? 32 : 64) == 0, "swizzle strides");
+    static_assert(E >= 2 && G * E == L, "bins of a thread");
+    const int kb = 2 * t + par;
+    const int ca = g < T ? 0 : 2, cb = g < T ? 1 : 2;             // the two real fields of the signal
+    const int ra = g < T ? g : 2 * (g - T), rb = g < T ? g : ra + 1;
+    const cx<R>* lo_a = stg + stage_index<R, T>((ca * K1 + kb) * T + ra);
+    const cx<R>* lo_b = stg + stage_index<R, T>((cb * K1 + kb) * T + rb);
+    const cx<R>* hi_a = stg + stage_index<R, T>((ca * K1 + (2 * L - kb)) * T + ra);
+    const cx<R>* hi_b = stg + stage_index<R, T>((cb * K1 + (2 * L - kb)) * T + rb);
+#pragma unroll
+    for (int r = 0; r < E; ++r) {
+        const int off = 2 * G * r * T;
+        cx<R> a, b;
+        if (r < E / 2) {
+            a = lo_a[off];
+            b = lo_b[off];
+        } else {
+            a = hi_a[-off];
+            b = hi_b[-off];
+            if (!(r == E / 2 && kb == 0)) {   // above the last stored bin
+                a = conjc(a);
+                b = conjc(b);
+            }
+        }
+        v[r] = mkc(a.re - b.im, a.im + b.re);
+    }
+}
+
+// Hermitian bins of the block's rows from the forward transforms in the signal
+// buffers.  The two real fields of a signal come from the same two values, so each
+// value is read once; PER consecutive rows of one (component, kx) make one 16-byte
+// store into the column-major spectrum.
+template <typename R, int L, int V>
+__device__ __forceinline__ void row_store_spectrum(const cx<R>* buf, cx<R>* __restrict__ X, int ny, int j0) {
+    using C = RowCfg<R, L, V>;
+    constexpr int T = C::T, E = C::E, BUF = C::BUF, K1 = L + 1;
+    constexpr int PER = 16 / (int)sizeof(cx<R>), TP = T / PER;
+    const size_t plane = (size_t)K1 * ny;
+    for (int e = threadIdx.x; e < K1 * TP; e += C::THREADS) {
+        const int k = e / TP, r0 = e % TP * PER;
+        if (j0 + r0 >= ny) continue;
+        // bins k and 2L - k (mod 2L) have the parity of k
+        const int km = k ? 2 * L - k : 0;
+        const cx<R>* bk = buf + (k & 1) * BUF + padi<E>(k >> 1);
+        const cx<R>* bm = buf + (k & 1) * BUF + padi<E>(km >> 1);
+        auto first = [](cx<R> zk, cx<R> zm) { return mkc((R)0.5 * (zk.re + zm.re), (R)0.5 * (zk.im - zm.im)); };
+        auto second = [](cx<R> zk, cx<R> zm) { return mkc((R)0.5 * (zk.im + zm.im), (R)0.5 * (zm.re - zk.re)); };
+        cx<R>* dst = X + (size_t)k * ny + j0 + r0;
+        Vec16<R> px, py, pz;
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            const int r = r0 + q;
+            const cx<R> zk = bk[2 * r * BUF], zm = bm[2 * r * BUF];
+            const cx<R> x = first(zk, zm), y = second(zk, zm);
+            px.v[2 * q] = x.re; px.v[2 * q + 1] = x.im;
+            py.v[2 * q] = y.re; py.v[2 * q + 1] = y.im;
+            // z of rows 2p, 2p + 1 share a signal (and, with PER = 2, this iteration)
+            const cx<R> wk = bk[2 * (T + r / 2) * BUF], wm = bm[2 * (T + r / 2) * BUF];
+            const cx<R> z = (r & 1) ? second(wk, wm) : first(wk, wm);
+            pz.v[2 * q] = z.re; pz.v[2 * q + 1] = z.im;
+        }
+        stv(reinterpret_cast<R*>(dst), px);
+        stv(reinterpret_cast<R*>(dst + plane), py);
+        stv(reinterpret_cast<R*>(dst + 2 * plane), pz);
+    }
+}
+
 // ---------------------------------------------------------------------------
 template <typename R, int L, int V>
 __global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS) __maxnreg__((RowCfg<R, L, V>::MAXREG)) k_row_forward_fast(const FilmDev* __restrict__ films,
@@ -236,33 +333,7 @@ __global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS) __maxnreg__((RowCfg<
         for (int i = 0; i < E; ++i) buf[s * BUF + padi<E>(FFT::out_index(t, i))] = v[i];
         __syncthreads();
         cx<R>* __restrict__ X = reinterpret_cast<cx<R>*>(F.X);
-        constexpr int K1 = L + 1, L2 = 2 * L;
-        // unpack the two real rows of each transform; PER consecutive rows of one
-        // (component, kx) make one 16-byte store into the column-major spectrum
-        constexpr int PER = 16 / (int)sizeof(cx<R>), TP = T / PER;
-        for (int e = tid; e < 3 * K1 * TP; e += C::THREADS) {
-            const int rp = e % TP, rest = e / TP;
-            const int k = rest % K1, c = rest / K1;
-            const int r0 = rp * PER;
-            if (j0 + r0 >= ny) continue;
-            const int km = (L2 - k) % L2;
-            cx<R> out[PER];
-#pragma unroll
-            for (int q = 0; q < PER; ++q) {
-                const int r = r0 + q;
-                int gg, half;
-                if (c < 2) { gg = r; half = c; }
-                else { gg = T + r / 2; half = r & 1; }
-                const cx<R> zk = buf[(2 * gg + (k & 1)) * BUF + padi<E>(k >> 1)];
-                const cx<R> zm = buf[(2 * gg + (km & 1)) * BUF + padi<E>(km >> 1)];
-                if (half == 0) out[q] = mkc((R)0.5 * (zk.re + zm.re), (R)0.5 * (zk.im - zm.im));
-                else out[q] = mkc((R)0.5 * (zk.im + zm.im), (R)0.5 * (zm.re - zk.re));
-            }
-            Vec16<R> pk;
-#pragma unroll
-            for (int q = 0; q < PER; ++q) { pk.v[2 * q] = out[q].re; pk.v[2 * q + 1] = out[q].im; }
-            stv(reinterpret_cast<R*>(X + ((size_t)c * K1 + k) * ny + j0 + r0), pk);
-        }
+        row_store_spectrum<R, L, V>(buf, X, ny, j0);
         __syncthreads();
     }
 }
@@ -486,48 +557,10 @@ __global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS) __maxnreg__((MODE ==
         const int j0 = w.blk * T;
         if (do_fft) {
             const cx<R>* __restrict__ X = reinterpret_cast<const cx<R>*>(F.X);
-            constexpr int K1 = L + 1, L2 = 2 * L;
-            // stage this block's rows of the spectrum, [c][k][r], with contiguous
-            // T-row chunks per (c, k) (the signal buffers are free here)
-            cx<R>* stg = buf;
-            constexpr int PER = 16 / (int)sizeof(cx<R>);
-            for (int p = tid; p < 3 * K1 * T / PER; p += C::THREADS) {
-                const int e = p * PER, r = e % T, ck = e / T;
-                cx<R>* dst = stg + stage_slot<R, T>(p) * PER;
-                if (j0 + r < ny) {
-                    cp_async16(dst, X + (size_t)ck * ny + j0 + r);
-                } else {
-#pragma unroll
-                    for (int q = 0; q < PER; ++q) dst[q] = mkc((R)0, (R)0);
-                }
-            }
-            cp_async_wait_all();
+            row_stage_spectrum<R, L, V>(X, buf, ny, j0);
             __syncthreads();
-            static_assert((2 * G * T / PER) % (T == 2 ? 32 : 64) == 0, "swizzle strides");
-            const int kb = 2 * t + par;
-            auto xval = [&](int c, int rr, int k, int r) -> cx<R> {
-                // k = kb + 2*G*rr: the swizzle of a slot depends only on the bits below
-                // 2*G*T/PER pieces, so the slots of a thread are its slot at rr = 0 plus
-                // a constant per rr (immediate offsets, no per-value swizzle)
-                const int off = 2 * G * rr * T;
-                if (k <= L) return stg[stage_index<R, T>((c * K1 + kb) * T + r) + off];
-                return conjc(stg[stage_index<R, T>((c * K1 + (L2 - kb)) * T + r) - off]);
-            };
             cx<R> v[E];
-#pragma unroll
-            for (int r = 0; r < E; ++r) {
-                const int k = 2 * (t + G * r) + par;
-                cx<R> z;
-                if (g < T) {
-                    const cx<R> bx = xval(0, r, k, g), by = xval(1, r, k, g);
-                    z = mkc(bx.re - by.im, bx.im + by.re);
-                } else {
-                    const int ra = 2 * (g - T);
-                    const cx<R> za = xval(2, r, k, ra), zb = xval(2, r, k, ra + 1);
-                    z = mkc(za.re - zb.im, za.im + zb.re);
-                }
-                v[r] = z;
-            }
+            row_load_inverse<R, L, V>(buf, v, t, g, par);
             __syncthreads();
             FI::run(v, t, buf + s * BUF, twp);
             __syncthreads();

@@ -71,48 +71,12 @@ __global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS) __maxnreg__((RowCfg<
         const int j0 = w.blk * T;
         const int cur = st->cur;
         cx<R>* __restrict__ X = reinterpret_cast<cx<R>*>(F.X);
-        constexpr int K1 = L + 1, L2 = 2 * L;
         if (do_fft) {
             // ---- 1. inverse transform of stage s (k_row_inverse_fast) ----
-            cx<R>* stg = buf;
-            constexpr int PER = 16 / (int)sizeof(cx<R>);
-            for (int p = tid; p < 3 * K1 * T / PER; p += C::THREADS) {
-                const int e = p * PER, r = e % T, ck = e / T;
-                cx<R>* dst = stg + stage_slot<R, T>(p) * PER;
-                if (j0 + r < ny) {
-                    cp_async16(dst, X + (size_t)ck * ny + j0 + r);
-                } else {
-#pragma unroll
-                    for (int q = 0; q < PER; ++q) dst[q] = mkc((R)0, (R)0);
-                }
-            }
-            cp_async_wait_all();
+            row_stage_spectrum<R, L, V>(X, buf, ny, j0);
             __syncthreads();
-            static_assert((2 * G * T / PER) % (T == 2 ? 32 : 64) == 0, "swizzle strides");
-            const int kb = 2 * t + par;
-            auto xval = [&](int c, int rr, int k, int r) -> cx<R> {
-                // k = kb + 2*G*rr: the swizzle of a slot depends only on the bits below
-                // 2*G*T/PER pieces, so the slots of a thread are its slot at rr = 0 plus
-                // a constant per rr (immediate offsets, no per-value swizzle)
-                const int off = 2 * G * rr * T;
-                if (k <= L) return stg[stage_index<R, T>((c * K1 + kb) * T + r) + off];
-                return conjc(stg[stage_index<R, T>((c * K1 + (L2 - kb)) * T + r) - off]);
-            };
             cx<R> v[E];
-#pragma unroll
-            for (int r = 0; r < E; ++r) {
-                const int k = 2 * (t + G * r) + par;
-                cx<R> z;
-                if (g < T) {
-                    const cx<R> bx = xval(0, r, k, g), by = xval(1, r, k, g);
-                    z = mkc(bx.re - by.im, bx.im + by.re);
-                } else {
-                    const int ra = 2 * (g - T);
-                    const cx<R> za = xval(2, r, k, ra), zb = xval(2, r, k, ra + 1);
-                    z = mkc(za.re - zb.im, za.im + zb.re);
-                }
-                v[r] = z;
-            }
+            row_load_inverse<R, L, V>(buf, v, t, g, par);
             __syncthreads();
             FI::run(v, t, buf + s * BUF, twp);
             __syncthreads();
@@ -269,30 +233,7 @@ __global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS) __maxnreg__((RowCfg<
 #pragma unroll
         for (int i = 0; i < E; ++i) buf[s * BUF + padi<E>(FF::out_index(t, i))] = v[i];
         __syncthreads();
-        constexpr int PER = 16 / (int)sizeof(cx<R>), TP = T / PER;
-        for (int e = tid; e < 3 * K1 * TP; e += C::THREADS) {
-            const int rp = e % TP, rest = e / TP;
-            const int k = rest % K1, c = rest / K1;
-            const int r0 = rp * PER;
-            if (j0 + r0 >= ny) continue;
-            const int km = (L2 - k) % L2;
-            cx<R> out[PER];
-#pragma unroll
-            for (int q = 0; q < PER; ++q) {
-                const int r = r0 + q;
-                int gg, half;
-                if (c < 2) { gg = r; half = c; }
-                else { gg = T + r / 2; half = r & 1; }
-                const cx<R> zk = buf[(2 * gg + (k & 1)) * BUF + padi<E>(k >> 1)];
-                const cx<R> zm = buf[(2 * gg + (km & 1)) * BUF + padi<E>(km >> 1)];
-                if (half == 0) out[q] = mkc((R)0.5 * (zk.re + zm.re), (R)0.5 * (zk.im - zm.im));
-                else out[q] = mkc((R)0.5 * (zk.im + zm.im), (R)0.5 * (zm.re - zk.re));
-            }
-            Vec16<R> pk;
-#pragma unroll
-            for (int q = 0; q < PER; ++q) { pk.v[2 * q] = out[q].re; pk.v[2 * q + 1] = out[q].im; }
-            stv(reinterpret_cast<R*>(X + ((size_t)c * K1 + k) * ny + j0 + r0), pk);
-        }
+        row_store_spectrum<R, L, V>(buf, X, ny, j0);
         __syncthreads();
     }
 }
