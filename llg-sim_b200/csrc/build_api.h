@@ -60,6 +60,7 @@ struct LaunchGeom {
     int grid_rfull;   // register-FFT row-inverse pass, full epilogue
     int grid_col;
     int grid_fused;   // fused row pass (k_row_fused)
+    int nsm;          // SMs of the device
     bool any_demag;
     bool fuse_rows;   // end a stage and start the next in one row pass where possible
     int row_var;      // register-FFT radix plan of the row kernels (FPlan V)

@@ -134,7 +134,8 @@ cudaError_t prepare_eval_kernels(size_t smem_row, size_t smem_col) {
             both((const void*)k_row_inverse_fast<R, L, 0, V>, sm);
             both((const void*)k_row_inverse_fast<R, L, 1, V>, sm);
             both((const void*)k_row_inverse_fast<R, L, 2, V>, sm);
-            both((const void*)k_row_fused<R, L, V>, sm);
+            both((const void*)k_row_fused<R, L, V, 1>, sm);
+            if constexpr (fused_xt_ok<R, L, V>()) both((const void*)k_row_fused<R, L, V, 2>, sm);
         }
         if constexpr (ColCfg<R, L, V>::SMEM + kStaticSmemCol <= kSmemMax) {
             both((const void*)k_column_fast<R, L, V, false>, (int)ColCfg<R, L, V, false>::SMEM);
@@ -174,7 +175,7 @@ cudaError_t launch_one(int which, const EvalSpec& spec, const LaunchGeom& g, cud
                         torque<<<grid, 256, 0, s>>>(g.films, g.row_items, g.n_row_items, CPI, spec);
                         ++count;
                     } else if (spec.rhs == RHS_MINIMIZE) {
-                        row(k_row_inverse_fast<R, L, 2, V>, g.grid_rfull, C::THREADS, C::SMEM);
+                        row(k_row_inverse_fast<R, L, 2, V>, g.grid_rfull, C::THREADS * inverse_xt<R, L, 2, V>(), C::SMEM);
                     } else {
                         row(k_row_inverse_fast<R, L, 0, V>, g.grid_rfull, C::THREADS, C::SMEM);
                     }
@@ -219,8 +220,15 @@ cudaError_t launch_fused(const EvalSpec& si, const EvalSpec& sf, const LaunchGeo
         constexpr int L = decltype(LC)::value, V = decltype(VC)::value;
         if constexpr (RowCfg<R, L, V>::SMEM <= kSmemMax) {
             using C = RowCfg<R, L, V>;
-            k_row_fused<R, L, V><<<g.grid_fused, C::THREADS, C::SMEM, s>>>(g.films, g.row_items, g.n_row_items, si,
-                                                                           sf);
+            if constexpr (fused_xt_ok<R, L, V>()) {
+                if (g.n_row_items <= g.nsm) {   // one block per SM at most
+                    k_row_fused<R, L, V, 2><<<g.n_row_items, 2 * C::THREADS, C::SMEM, s>>>(g.films, g.row_items,
+                                                                                          g.n_row_items, si, sf);
+                    return;
+                }
+            }
+            k_row_fused<R, L, V, 1><<<g.grid_fused, C::THREADS, C::SMEM, s>>>(g.films, g.row_items, g.n_row_items, si,
+                                                                              sf);
         }
     });
     if (nk) *nk += 1;
@@ -250,7 +258,7 @@ void fast_occupancy(int nx, int ny, int row_var, int col_var, int* fwd_blocks_pe
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_row_forward_fast<R, L, V>, C::THREADS, C::SMEM);
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_row_inverse_fast<R, L, 1, V>, C::THREADS, C::SMEM);
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k_row_inverse_fast<R, L, 0, V>, C::THREADS, C::SMEM);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d, k_row_fused<R, L, V>, C::THREADS, C::SMEM);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d, k_row_fused<R, L, V, 1>, C::THREADS, C::SMEM);
             *fwd_blocks_per_sm = std::max(1, a);
             *inv_blocks_per_sm = std::max(1, b);
             *full_blocks_per_sm = std::max(1, c);

@@ -106,13 +106,21 @@ __device__ __forceinline__ void load_tables(cx<R>* twp, const cx<R>* __restrict_
     for (int i = threadIdx.x; i < L; i += blockDim.x) pre[i] = gpre[i];
 }
 
+// Barrier over the threads of the block's transforms: all of them, or the first
+// THREADS of a block that has as many again (XT = 2; barrier 15).
+template <int THREADS, int XT>
+__device__ __forceinline__ void fft_sync() {
+    if constexpr (XT == 1) __syncthreads();
+    else asm volatile("bar.sync 15, %0;" ::"n"(THREADS) : "memory");
+}
+
 // Stages the spectrum of a block's rows, [c][k][r] in swizzled 16-byte pieces with
 // contiguous T-row chunks per (c, k), into the signal buffers (free here).
-template <typename R, int L, int V>
+template <typename R, int L, int V, int NT = RowCfg<R, L, V>::THREADS>   // NT: threads of the block
 __device__ __forceinline__ void row_stage_spectrum(const cx<R>* __restrict__ X, cx<R>* stg, int ny, int j0) {
     using C = RowCfg<R, L, V>;
     constexpr int T = C::T, PER = 16 / (int)sizeof(cx<R>), TP = T / PER;
-    for (int p = threadIdx.x; p < 3 * (L + 1) * TP; p += C::THREADS) {
+    for (int p = threadIdx.x; p < 3 * (L + 1) * TP; p += NT) {
         const int ck = p / TP, r = p % TP * PER;
         cx<R>* dst = stg + stage_slot<R, T>(p) * PER;
         if (j0 + r < ny) {
@@ -168,13 +176,13 @@ __device__ __forceinline__ void row_load_inverse(const cx<R>* stg, cx<R> (&v)[Ro
 // buffers.  The two real fields of a signal come from the same two values, so each
 // value is read once; PER consecutive rows of one (component, kx) make one 16-byte
 // store into the column-major spectrum.
-template <typename R, int L, int V>
+template <typename R, int L, int V, int NT = RowCfg<R, L, V>::THREADS>
 __device__ __forceinline__ void row_store_spectrum(const cx<R>* buf, cx<R>* __restrict__ X, int ny, int j0) {
     using C = RowCfg<R, L, V>;
     constexpr int T = C::T, E = C::E, BUF = C::BUF, K1 = L + 1;
     constexpr int PER = 16 / (int)sizeof(cx<R>), TP = T / PER;
     const size_t plane = (size_t)K1 * ny;
-    for (int e = threadIdx.x; e < K1 * TP; e += C::THREADS) {
+    for (int e = threadIdx.x; e < K1 * TP; e += NT) {
         const int k = e / TP, r0 = e % TP * PER;
         if (j0 + r0 >= ny) continue;
         // bins k and 2L - k (mod 2L) have the parity of k
@@ -527,11 +535,20 @@ __global__ void __launch_bounds__(ColCfg<R, L, V, LEAN>::THREADS) __maxnreg__((C
 // ---------------------------------------------------------------------------
 // MODE 0: full epilogue; 1: no epilogue, the demag field is written to the film's
 // bdem planes for k_stage_torque; 2: the minimiser epilogue (RHS_MINIMIZE).
+// The minimiser's FP64 cell update is a long dependent chain, and the films up to 256
+// cells wide have fewer row blocks than the SMs can hold: there the block has as many
+// threads again (XT = 2), which take no part in the transforms but halve the cells per
+// thread of the epilogue.
 template <typename R, int L, int MODE, int V>
-__global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS) __maxnreg__((MODE == 1 ? RowCfg<R, L, V>::MAXREG : RowCfg<R, L, V>::REG2)) k_row_inverse_fast(const FilmDev* __restrict__ films,
+__host__ __device__ constexpr int inverse_xt() {
+    return MODE == 2 && sizeof(R) == 4 && V == 0 && L <= 256 && RowCfg<R, L, V>::THREADS <= 192 ? 2 : 1;
+}
+template <typename R, int L, int MODE, int V>
+__global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS * inverse_xt<R, L, MODE, V>()) __maxnreg__((MODE == 1 ? RowCfg<R, L, V>::MAXREG : RowCfg<R, L, V>::REG2)) k_row_inverse_fast(const FilmDev* __restrict__ films,
                                                                             const WorkItem* __restrict__ items,
                                                                             int nitems, EvalSpec spec) {
     using C = RowCfg<R, L, V>;
+    constexpr int NT = C::THREADS * inverse_xt<R, L, MODE, V>();
     using FI = GroupFFT<R, L, true, V>;
     constexpr int G = C::G, E = C::E, T = C::T, BUF = C::BUF;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -557,25 +574,28 @@ __global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS) __maxnreg__((MODE ==
         const int j0 = w.blk * T;
         if (do_fft) {
             const cx<R>* __restrict__ X = reinterpret_cast<const cx<R>*>(F.X);
-            row_stage_spectrum<R, L, V>(X, buf, ny, j0);
+            row_stage_spectrum<R, L, V, NT>(X, buf, ny, j0);
             __syncthreads();
-            cx<R> v[E];
-            row_load_inverse<R, L, V>(buf, v, t, g, par);
-            __syncthreads();
-            FI::run(v, t, buf + s * BUF, twp);
-            __syncthreads();
-            if (par) {
+            constexpr int XT = NT / C::THREADS;
+            if (XT == 1 || tid < C::THREADS) {   // threads of the transforms
+                cx<R> v[E];
+                row_load_inverse<R, L, V>(buf, v, t, g, par);
+                fft_sync<C::THREADS, XT>();
+                FI::run(v, t, buf + s * BUF, twp);
+                fft_sync<C::THREADS, XT>();
+                if (par) {
 #pragma unroll
-                for (int i = 0; i < E; ++i) buf[s * BUF + padi<E>(FI::out_index(t, i))] = v[i];
-            }
-            __syncthreads();
-            if (!par) {
-                const cx<R>* ob = buf + (s + 1) * BUF;
-                cx<R>* db = buf + s * BUF;
+                    for (int i = 0; i < E; ++i) buf[s * BUF + padi<E>(FI::out_index(t, i))] = v[i];
+                }
+                fft_sync<C::THREADS, XT>();
+                if (!par) {
+                    const cx<R>* ob = buf + (s + 1) * BUF;
+                    cx<R>* db = buf + s * BUF;
 #pragma unroll
-                for (int i = 0; i < E; ++i) {
-                    const int nn = FI::out_index(t, i);
-                    db[padi<E>(nn)] = v[i] + cmulc(ob[padi<E>(nn)], pre[nn]);
+                    for (int i = 0; i < E; ++i) {
+                        const int nn = FI::out_index(t, i);
+                        db[padi<E>(nn)] = v[i] + cmulc(ob[padi<E>(nn)], pre[nn]);
+                    }
                 }
             }
             __syncthreads();

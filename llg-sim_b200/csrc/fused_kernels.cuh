@@ -26,13 +26,20 @@ namespace llg {
 // si: stage s (inverse half: m_in, k_out, rhs, field terms); sf: stage s+1
 // (forward half: m_in receives m_{s+1}, the combination kidx / a with
 // sf.kidx[sf.nterm - 1] == si.k_out).  Both carry the same request gate.
+// XT = 2: the block has as many threads again, which take no part in the transforms
+// but halve the cells per thread of step 2 — for launches with at most one block per
+// SM, where latency is all that counts and the threads would be free anyway.
 template <typename R, int L, int V>
-__global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS) __maxnreg__((RowCfg<R, L, V>::REG2)) k_row_fused(
+__host__ __device__ constexpr bool fused_xt_ok() {   // one block of twice the threads at 168 registers, groups within a warp
+    return V == 0 && RowCfg<R, L, V>::THREADS <= 192 && RowCfg<R, L, V>::G <= 32;
+}
+template <typename R, int L, int V, int XT>
+__global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS * XT) __maxnreg__((XT == 1 ? RowCfg<R, L, V>::REG2 : regs_for_blocks(2 * RowCfg<R, L, V>::THREADS, 1))) k_row_fused(
     const FilmDev* __restrict__ films, const WorkItem* __restrict__ items, int nitems, EvalSpec si, EvalSpec sf) {
     using C = RowCfg<R, L, V>;
     using FF = GroupFFT<R, L, false, V>;
     using FI = GroupFFT<R, L, true, V>;
-    constexpr int G = C::G, E = C::E, T = C::T, BUF = C::BUF;
+    constexpr int G = C::G, E = C::E, T = C::T, BUF = C::BUF, NT = C::THREADS * XT;
     // phase 2 takes W cells per step of its loop, two in FP32 and one in FP64 (the same
     // registers): with EARLY the stencil, m0 and the previous torques of a step are all
     // loaded before any arithmetic, one memory round trip per step instead of one per
@@ -54,6 +61,7 @@ __global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS) __maxnreg__((RowCfg<
         cx<R>* z = c < 2 ? &buf[(2 * r) * BUF + padi<E>(i)] : &buf[(2 * (T + r / 2)) * BUF + padi<E>(i)];
         return (c == 0 || (c == 2 && (r & 1) == 0)) ? &z->re : &z->im;
     };
+    const bool fft = XT == 1 || tid < C::THREADS;   // threads of the transforms
     bool tables = false;
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const WorkItem w = items[it];
@@ -73,25 +81,27 @@ __global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS) __maxnreg__((RowCfg<
         cx<R>* __restrict__ X = reinterpret_cast<cx<R>*>(F.X);
         if (do_fft) {
             // ---- 1. inverse transform of stage s (k_row_inverse_fast) ----
-            row_stage_spectrum<R, L, V>(X, buf, ny, j0);
+            row_stage_spectrum<R, L, V, NT>(X, buf, ny, j0);
             __syncthreads();
-            cx<R> v[E];
-            row_load_inverse<R, L, V>(buf, v, t, g, par);
-            __syncthreads();
-            FI::run(v, t, buf + s * BUF, twp);
-            __syncthreads();
-            if (par) {
+            if (fft) {
+                cx<R> v[E];
+                row_load_inverse<R, L, V>(buf, v, t, g, par);
+                fft_sync<C::THREADS, XT>();
+                FI::run(v, t, buf + s * BUF, twp);
+                fft_sync<C::THREADS, XT>();
+                if (par) {
 #pragma unroll
-                for (int i = 0; i < E; ++i) buf[s * BUF + padi<E>(FI::out_index(t, i))] = v[i];
-            }
-            __syncthreads();
-            if (!par) {
-                const cx<R>* ob = buf + (s + 1) * BUF;
-                cx<R>* db = buf + s * BUF;
+                    for (int i = 0; i < E; ++i) buf[s * BUF + padi<E>(FI::out_index(t, i))] = v[i];
+                }
+                fft_sync<C::THREADS, XT>();
+                if (!par) {
+                    const cx<R>* ob = buf + (s + 1) * BUF;
+                    cx<R>* db = buf + s * BUF;
 #pragma unroll
-                for (int i = 0; i < E; ++i) {
-                    const int nn = FI::out_index(t, i);
-                    db[padi<E>(nn)] = v[i] + cmulc(ob[padi<E>(nn)], pre[nn]);
+                    for (int i = 0; i < E; ++i) {
+                        const int nn = FI::out_index(t, i);
+                        db[padi<E>(nn)] = v[i] + cmulc(ob[padi<E>(nn)], pre[nn]);
+                    }
                 }
             }
             __syncthreads();
@@ -118,7 +128,7 @@ __global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS) __maxnreg__((RowCfg<
             const R cs = (R)(dt * sf.a[nq]);   // k_s coefficient
             const R Ms = (R)F.ms;
             const LocalCoef<R> cf = local_coef<R>(F, si.dmi != 0);
-            for (int e = tid; e < NV; e += C::THREADS) {
+            for (int e = tid; e < NV; e += NT) {
                 const int c0 = e * W, r = c0 / L, i0 = c0 - r * L, j = j0 + r;
                 if (j >= ny) {   // rows past the film are zero in the forward transform
                     if (do_fft)
@@ -217,8 +227,8 @@ __global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS) __maxnreg__((RowCfg<
         if (!do_fft) continue;
         __syncthreads();
         // ---- 3. forward transform of stage s+1 (k_row_forward_fast) ----
-        cx<R> v[E];
-        {
+        if (fft) {
+            cx<R> v[E];
             const cx<R>* zb = buf + (2 * g) * BUF;
 #pragma unroll
             for (int r = 0; r < E; ++r) {
@@ -226,14 +236,14 @@ __global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS) __maxnreg__((RowCfg<
                 const cx<R> x = zb[padi<E>(nn)];
                 v[r] = par ? cmul(x, pre[nn]) : x;
             }
+            fft_sync<C::THREADS, XT>();
+            FF::run(v, t, buf + s * BUF, twp);
+            fft_sync<C::THREADS, XT>();
+#pragma unroll
+            for (int i = 0; i < E; ++i) buf[s * BUF + padi<E>(FF::out_index(t, i))] = v[i];
         }
         __syncthreads();
-        FF::run(v, t, buf + s * BUF, twp);
-        __syncthreads();
-#pragma unroll
-        for (int i = 0; i < E; ++i) buf[s * BUF + padi<E>(FF::out_index(t, i))] = v[i];
-        __syncthreads();
-        row_store_spectrum<R, L, V>(buf, X, ny, j0);
+        row_store_spectrum<R, L, V, NT>(buf, X, ny, j0);
         __syncthreads();
     }
 }

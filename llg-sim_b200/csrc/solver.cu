@@ -711,6 +711,7 @@ struct Engine final : EngineBase {
         geom.any_demag = any_demag;
         geom.fast_row = 0;
         geom.fast_col = 0;
+        geom.nsm = nsm_count();
         geom.fuse_rows = !env_flag("LLG_B200_NO_FUSE");
         geom.row_var = 0;
         geom.col_var = 0;
