@@ -115,8 +115,13 @@ cudaError_t prepare_eval_kernels(size_t smem_row, size_t smem_col) {
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k_row_inverse<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_row_fused_generic<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row);
+    e = cudaFuncSetAttribute(k_row_fused_generic<R, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row);
     if (e != cudaSuccess) return e;
+    if (sizeof(R) == 4) {
+        e = cudaFuncSetAttribute(k_row_fused_generic<R, sizeof(R) == 4 ? 512 : 256>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row);
+        if (e != cudaSuccess) return e;
+    }
     e = cudaFuncSetAttribute(k_column<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_col);
     if (e != cudaSuccess) return e;
     // fast kernels: every instantiation whose shared memory fits; the whole unified
@@ -214,8 +219,14 @@ bool can_fuse(const EvalSpec& si, const EvalSpec& sf, const LaunchGeom& g) {
 
 template <typename R>
 cudaError_t launch_fused(const EvalSpec& si, const EvalSpec& sf, const LaunchGeom& g, cudaStream_t s, int* nk) {
-    if (!g.fast_row)
-        k_row_fused_generic<R><<<g.grid_row, 256, g.smem_row, s>>>(g.films, g.row_items, g.n_row_items, si, sf);
+    if (!g.fast_row) {
+        if (sizeof(R) == 4 && g.n_row_items <= g.nsm)
+            k_row_fused_generic<R, sizeof(R) == 4 ? 512 : 256><<<g.n_row_items, sizeof(R) == 4 ? 512 : 256, g.smem_row, s>>>(
+                g.films, g.row_items, g.n_row_items, si, sf);
+        else
+            k_row_fused_generic<R, 256><<<g.grid_row, 256, g.smem_row, s>>>(g.films, g.row_items, g.n_row_items, si,
+                                                                            sf);
+    }
     dispatch_LV<R>(g.fast_row, g.row_var, [&](auto LC, auto VC) {
         constexpr int L = decltype(LC)::value, V = decltype(VC)::value;
         if constexpr (RowCfg<R, L, V>::SMEM <= kSmemMax) {

@@ -253,8 +253,11 @@ __global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS * XT) __maxnreg__((XT
 // replaces two launches by one; its loads of a step are all in flight together, and
 // the field and torque arithmetic needs neither the reductions nor the FP64 of the
 // full epilogue.  Same operations in the same order as the unfused kernels.
-template <typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) k_row_fused_generic(const FilmDev* __restrict__ films,
+// NT threads: 512 in FP32 for launches with at most one block per SM (two rows of up to
+// 256 cells are then one step), else 256 and two blocks per SM (one in FP64, whose
+// butterflies need the registers).
+template <typename R, int NT>
+__global__ void __launch_bounds__(NT, sizeof(R) == 4 && NT == 256 ? 2 : 1) k_row_fused_generic(const FilmDev* __restrict__ films,
                                                               const WorkItem* __restrict__ items, int nitems,
                                                               EvalSpec si, EvalSpec sf) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
