@@ -55,6 +55,7 @@ constexpr size_t kStaticSmemCol = 64;   // mbarriers and the timeout flag of k_c
 bool lean_epilogue(const EvalSpec& e) {
     return e.err == ERR_NONE && !e.reduce && e.local && (e.rhs == RHS_LLG || e.rhs == RHS_RELAX);
 }
+constexpr int log2_of(int v) { return v <= 1 ? 0 : 1 + log2_of(v / 2); }
 int stage_grid(long long work) {
     return (int)std::max(1LL, std::min((work + 255) / 256, 148LL * 8));
 }
@@ -173,11 +174,11 @@ cudaError_t launch_one(int which, const EvalSpec& spec, const LaunchGeom& g, cud
                         row(k_row_forward_fast<R, L, V>, g.grid_row, C::THREADS, C::SMEM);
                     } else if (lean_epilogue(spec) || lean_err45_epilogue(spec)) {
                         // transform only, then the torque epilogue as a streaming kernel
-                        constexpr int CPI = C::T * L;
+                        constexpr int LOG_L = log2_of(L), LOG_T = log2_of(C::T);
                         row(k_row_inverse_fast<R, L, 1, V>, g.grid_rinv, C::THREADS, C::SMEM);
-                        const int grid = stage_grid((long long)g.n_row_items * CPI);
+                        const int grid = stage_grid((long long)g.n_row_items * C::T * L);
                         auto torque = lean_err45_epilogue(spec) ? k_stage_torque<R, true> : k_stage_torque<R, false>;
-                        torque<<<grid, 256, 0, s>>>(g.films, g.row_items, g.n_row_items, CPI, spec);
+                        torque<<<grid, 256, 0, s>>>(g.films, g.row_items, g.n_row_items, LOG_L, LOG_T, spec);
                         ++count;
                     } else if (spec.rhs == RHS_MINIMIZE) {
                         row(k_row_inverse_fast<R, L, 2, V>, g.grid_rfull, C::THREADS * inverse_xt<R, L, 2, V>(), C::SMEM);

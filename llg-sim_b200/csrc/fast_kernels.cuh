@@ -250,76 +250,64 @@ __global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS) __maxnreg__((RowCfg<
             cq[q] = q < spec.nterm ? (R)(dt * spec.a[q]) : (R)0;
         }
         const R Ms = (R)F.ms;
-        // m_s = normalize(m0 + sum_q dt*a_q*k_q) in two sweeps over 16-byte vectors of
-        // W cells: (1) per component, the combination (all its loads in flight
-        // together) into the packed signal slots; (2) per cell, normalisation (or
-        // vacuum), the m_s store and the scaling by Ms.  Signal slots: x, y of row r
-        // in buffer 2r (re, im); z of rows 2p, 2p+1 in buffer 2(T+p) (re, im).
-        constexpr int W = Vec16<R>::W, NV = T * L / W;
-        auto slot = [&](int c, int r, int i) -> R* {
-            cx<R>* z = c < 2 ? &buf[(2 * r) * BUF + padi<E>(i)] : &buf[(2 * (T + r / 2)) * BUF + padi<E>(i)];
-            return (c == 0 || (c == 2 && (r & 1) == 0)) ? &z->re : &z->im;
-        };
-        // two vectors per thread and round: both vectors' loads are in flight before
-        // either is stored (the stores go to shared memory after the loads)
-        constexpr int U = 2;
-        for (int e0 = tid; e0 < 3 * NV; e0 += U * C::THREADS) {
-            Vec16<R> a[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int e = e0 + u * C::THREADS;
-                const int c = e / NV, ev = e - c * NV;
-                const int r = (ev * W) / L, j = j0 + r;
-#pragma unroll
-                for (int l = 0; l < W; ++l) a[u].v[l] = (R)0;
-                if (e < 3 * NV && j < ny) {
-                    const int idx = c * n + j * L + (ev * W - r * L);
-                    if (spec.nterm > 0) {
-                        a[u] = ldv(m0 + idx);
-                        Vec16<R> ka[6];
-#pragma unroll
-                        for (int q = 0; q < 6; ++q)
-                            if (q < spec.nterm) ka[q] = ldv(kp[q] + idx);
-#pragma unroll
-                        for (int q = 0; q < 6; ++q)
-                            if (q < spec.nterm) {
-#pragma unroll
-                                for (int l = 0; l < W; ++l) a[u].v[l] = a[u].v[l] + cq[q] * ka[q].v[l];
-                            }
-                    } else {
-                        a[u] = ldv(ms + idx);
-                    }
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int e = e0 + u * C::THREADS;
-                if (e >= 3 * NV) continue;
-                const int c = e / NV, ev = e - c * NV;
-                const int c0 = ev * W, r = c0 / L, i0 = c0 - r * L;
-#pragma unroll
-                for (int l = 0; l < W; ++l) *slot(c, r, i0 + l) = a[u].v[l];
-            }
-        }
-        __syncthreads();
+        // m_s = normalize(m0 + sum_q dt*a_q*k_q), W cells per step, the three
+        // components together; the state goes to m_s and,
+        // scaled by Ms, to the signal slots: x, y of row r in buffer 2r (re, im); z of
+        // rows 2p, 2p+1 in buffer 2(T+p) (re, im).
+        constexpr int W = 2, NV = T * L / W;
+        using VW = VecW<R, W>;
         for (int e = tid; e < NV; e += C::THREADS) {
             const int c0 = e * W, r = c0 / L, i0 = c0 - r * L, j = j0 + r;
-            Vec16<R> v0, v1, v2;
-#pragma unroll
-            for (int l = 0; l < W; ++l) {
-                R a[3] = {*slot(0, r, i0 + l), *slot(1, r, i0 + l), *slot(2, r, i0 + l)};
-                if (spec.nterm > 0 && j < ny) {
-                    if (cell_inside(F, j * L + i0 + l)) normalize3(a);
-                    else { a[0] = (R)0; a[1] = (R)0; a[2] = (R)0; }
-                }
-                v0.v[l] = a[0]; v1.v[l] = a[1]; v2.v[l] = a[2];
-                *slot(0, r, i0 + l) = Ms * a[0];
-                *slot(1, r, i0 + l) = Ms * a[1];
-                *slot(2, r, i0 + l) = Ms * a[2];
-            }
-            if (spec.nterm > 0 && j < ny) {
+            VW a[3];
+            if (j < ny) {
                 const int idx = j * L + i0;
-                stv(ms + idx, v0); stv(ms + n + idx, v1); stv(ms + 2 * n + idx, v2);
+                if (spec.nterm > 0) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) a[c] = ldw<R, W>(m0 + c * n + idx);
+#pragma unroll
+                    for (int h = 0; h < 6; h += 2) {   // two torques in flight at a time
+                        VW ka[2][3];
+#pragma unroll
+                        for (int q = h; q < h + 2; ++q)
+                            if (q < spec.nterm)
+#pragma unroll
+                                for (int c = 0; c < 3; ++c) ka[q - h][c] = ldw<R, W>(kp[q] + c * n + idx);
+#pragma unroll
+                        for (int q = h; q < h + 2; ++q)
+                            if (q < spec.nterm)
+#pragma unroll
+                                for (int c = 0; c < 3; ++c)
+#pragma unroll
+                                    for (int l = 0; l < W; ++l)
+                                        a[c].v[l] = fma_rn(cq[q], ka[q - h][c].v[l], a[c].v[l]);
+                    }
+#pragma unroll
+                    for (int l = 0; l < W; ++l) {
+                        R v3[3] = {a[0].v[l], a[1].v[l], a[2].v[l]};
+                        if (cell_inside(F, idx + l)) normalize3(v3);
+                        else { v3[0] = (R)0; v3[1] = (R)0; v3[2] = (R)0; }   // vacuum pinned at m = 0
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) a[c].v[l] = v3[c];
+                    }
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) stw<R, W>(ms + c * n + idx, a[c]);
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) a[c] = ldw<R, W>(ms + c * n + idx);
+                }
+            } else {   // rows past the film are zero in the transform
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+#pragma unroll
+                    for (int l = 0; l < W; ++l) a[c].v[l] = (R)0;
+            }
+            if (do_fft) {
+#pragma unroll
+                for (int l = 0; l < W; ++l) {
+                    buf[(2 * r) * BUF + padi<E>(i0 + l)] = mkc(Ms * a[0].v[l], Ms * a[1].v[l]);
+                    cx<R>* z = &buf[(2 * (T + r / 2)) * BUF + padi<E>(i0 + l)];
+                    *((r & 1) ? &z->im : &z->re) = Ms * a[2].v[l];
+                }
             }
         }
         if (!do_fft) continue;

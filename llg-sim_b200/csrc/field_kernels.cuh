@@ -536,9 +536,9 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 0 : 2) k_row_forward(con
                     for (int q = 0; q < 6; ++q) {
                         if (q < spec.nterm) {
                             const R* k = kp[q];
-                            v[0] = v[0] + cq[q] * k[idx];
-                            v[1] = v[1] + cq[q] * k[n + idx];
-                            v[2] = v[2] + cq[q] * k[2 * n + idx];
+                            v[0] = fma_rn(cq[q], k[idx], v[0]);
+                            v[1] = fma_rn(cq[q], k[n + idx], v[1]);
+                            v[2] = fma_rn(cq[q], k[2 * n + idx], v[2]);
                         }
                     }
                     if (cell_inside(F, idx)) normalize3(v);

@@ -201,14 +201,14 @@ __global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS * XT) __maxnreg__((XT
                         for (int c = 0; c < 3; ++c) {
                             const VW kv = EARLY ? kq[EARLY ? q : 0][c] : ldw<R, W>(kp[q] + c * n + base);
 #pragma unroll
-                            for (int l = 0; l < W; ++l) a[c].v[l] = a[c].v[l] + cq[q] * kv.v[l];
+                            for (int l = 0; l < W; ++l) a[c].v[l] = fma_rn(cq[q], kv.v[l], a[c].v[l]);
                         }
                     }
                 }
 #pragma unroll
                 for (int c = 0; c < 3; ++c)
 #pragma unroll
-                    for (int l = 0; l < W; ++l) a[c].v[l] = a[c].v[l] + cs * ko[c].v[l];
+                    for (int l = 0; l < W; ++l) a[c].v[l] = fma_rn(cs, ko[c].v[l], a[c].v[l]);
 #pragma unroll
                 for (int l = 0; l < W; ++l) {
                     R v3[3] = {a[0].v[l], a[1].v[l], a[2].v[l]};
@@ -329,9 +329,9 @@ __global__ void __launch_bounds__(NT, sizeof(R) == 4 && NT == 256 ? 2 : 1) k_row
                 for (int q = 0; q < 5; ++q)
                     if (q < nq)
 #pragma unroll
-                        for (int c = 0; c < 3; ++c) v[c] = v[c] + cq[q] * kq[q][c];
+                        for (int c = 0; c < 3; ++c) v[c] = fma_rn(cq[q], kq[q][c], v[c]);
 #pragma unroll
-                for (int c = 0; c < 3; ++c) v[c] = v[c] + cs * k[c];
+                for (int c = 0; c < 3; ++c) v[c] = fma_rn(cs, k[c], v[c]);
                 if (coef_inside(cf, idx)) normalize3(v);
                 else { v[0] = (R)0; v[1] = (R)0; v[2] = (R)0; }   // vacuum pinned at m = 0
 #pragma unroll

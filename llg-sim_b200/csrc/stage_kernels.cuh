@@ -3,8 +3,10 @@
 // occupancy: k_stage_torque takes the local terms and the demag field that the
 // row-inverse transform left in the film's bdem planes, forms the torque, stores
 // k_s and, for the last RK45 stage, the error norm.  It walks the row work items
-// of one launch segment, CPI cells per item (a multiple of 512, so a warp never
-// spans two items and therefore never two films).
+// of one launch segment, T * L cells per item (a multiple of 512, so a warp never
+// spans two items and therefore never two films).  It is bound by issue (56 % active
+// at 1024 x 1024 cells), so positions are shifts and masks: L and T are powers of two
+// (a 64-bit division per cell was a fifth of its instructions).
 #pragma once
 #include "field_kernels.cuh"
 
@@ -14,14 +16,15 @@ namespace llg {
 // (coalesced loads, ~60 registers, high occupancy).
 template <typename R, bool ERR45>
 __global__ void __launch_bounds__(256, 4) k_stage_torque(const FilmDev* __restrict__ films,
-                                                          const WorkItem* __restrict__ items, int nitems, int cpi,
-                                                          EvalSpec spec) {
-    const long long total = (long long)nitems * cpi;
+                                                          const WorkItem* __restrict__ items, int nitems, int log_l,
+                                                          int log_t, EvalSpec spec) {
+    const int log_cpi = log_l + log_t;
+    const long long total = (long long)nitems << log_cpi;
     int coef_film = -1;
     LocalCoef<R> cf;
     for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < total;
          v += (long long)gridDim.x * blockDim.x) {
-        const WorkItem w = items[v / cpi];
+        const WorkItem w = items[v >> log_cpi];
         const FilmDev& F = films[w.film];
         if (w.film != coef_film) {   // coefficients of the local terms, once per film
             cf = local_coef<R>(F, spec.dmi != 0);
@@ -30,7 +33,7 @@ __global__ void __launch_bounds__(256, 4) k_stage_torque(const FilmDev* __restri
         StepState* st = F.st;
         if (skip_item(spec, st)) continue;   // uniform over the warp (one item per warp)
         const int nx = F.nx, ny = F.ny, n = nx * ny;
-        const int c0 = (int)(v % cpi), r = c0 / nx, i = c0 - r * nx, j = w.blk * F.rows_per_block + r;
+        const int i = (int)v & (nx - 1), j = (w.blk << log_t) + (((int)v >> log_l) & ((1 << log_t) - 1));
         double errmax = 0.0;
         bool errnan = false;
         if (j < ny) {

@@ -10,7 +10,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("prec", [0, 1])
 @pytest.mark.parametrize("nx,ny,demag,holes", [(96, 20, True, False), (50, 33, True, True), (7, 5, True, False),
-                                               (60, 1, True, False), (300, 16, True, True), (30, 9, False, False)])
+                                               (60, 1, True, False), (300, 16, True, True), (30, 9, False, False),
+                                               (30, 320, True, False)])   # more row blocks than SMs
 def test_fused_generic_rows_equal_unfused(orc, gpu, monkeypatch, nx, ny, demag, holes, prec):
     mask = holes_mask(nx, ny, [(0.1 * nx, 0.0, 0.2 * ny)]) if holes else None
     c = case(nx, ny, dmi=1e-3, k_u=5e4, demag=demag, mask=mask)
