@@ -15,6 +15,12 @@ FftPlan make_plan(int L);
 std::vector<FftPlan> plan_candidates(int L);
 // The plan with padded signals where `buffers` of them fit smem_max bytes, else unpadded.
 FftPlan padded_plan(FftPlan p, bool fp64, int buffers, size_t smem_max);
+// Threads of a block that transforms nsig signals of the plan and sweeps over
+// `sweeps` * L values besides: a pass of radix p has nsig L / p butterflies, so the
+// multiple of 32 in [128, most] with the fewest rounds over the plan, a round weighted
+// by its radix, and over the sweeps (1536 = 16 * 12 * 8 with 3 signals: 288, 384 and 576
+// butterflies take 4 rounds of 512 threads where 256 threads take 7); the smallest of equals.
+int fft_block_threads(const FftPlan& plan, int nsig, int sweeps, int most);
 // Pass tables of a plan (fft_smem.cuh) into out[2L].
 cudaError_t launch_pass_tables(const FftPlan& plan, void* out, bool fp64, cudaStream_t s);
 cudaError_t launch_twiddles(void* tw, int L2, bool fp64, cudaStream_t s);

@@ -375,6 +375,23 @@ FftPlan padded_plan(FftPlan p, bool fp64, int buffers, size_t smem_max) {
     return p;
 }
 
+int fft_block_threads(const FftPlan& plan, int nsig, int sweeps, int most) {
+    int best = 128;
+    long long best_cost = 0;
+    for (int nt = 128; nt <= most; nt += 32) {
+        long long cost = ((long long)sweeps * plan.L + nt - 1) / nt;
+        for (int q = 0; q < plan.npass; ++q) {
+            const long long n = (long long)nsig * (plan.L / plan.radix[q]);
+            cost += (n + nt - 1) / nt * plan.radix[q];
+        }
+        if (best_cost == 0 || cost < best_cost) {
+            best_cost = cost;
+            best = nt;
+        }
+    }
+    return best;
+}
+
 cudaError_t launch_pass_tables(const FftPlan& plan, void* out, bool fp64, cudaStream_t s) {
     const int blocks = (2 * plan.L + 255) / 256;
     if (fp64) k_pass_tables_smem<double><<<blocks, 256, 0, s>>>(plan, reinterpret_cast<cx<double>*>(out));

@@ -43,6 +43,7 @@ struct llg_demag_op {
     // (nullptr: general path), and the plans / pass tables of lengths nx and ny
     llg::r4<double>* Kf = nullptr;   // [nx+1][ny+1] (xx, xy, yy, zz) / (px py)
     llg::FftPlan plan_nx{}, plan_ny{};
+    int column_threads = 256;
     llg::cx<double>* tab_nx = nullptr;   // [2 nx] pass tables, then [2 nx] exp(-2 pi i k / (2 nx))
     llg::cx<double>* tab_ny = nullptr;
 };
@@ -161,10 +162,12 @@ __global__ void __launch_bounds__(kOpenThreads) k_open_rows_forward(int nx, int 
     }
 }
 
+constexpr int kOpenColumnMax = 512;   // most threads of a column block (fft_block_threads)
+
 // One kx column: the odd and then the even ky bins of the three components (six
 // padded buffers at a time, so that ny = 2048 fits), product with the folded kernel
 // and inverse.  The odd half waits in O, the even half adds it and replaces X.
-__global__ void __launch_bounds__(kOpenThreads) k_open_column(int nx, int ny, const llg::r4<double>* __restrict__ Kf,
+__global__ void __launch_bounds__(kOpenColumnMax) k_open_column(int nx, int ny, const llg::r4<double>* __restrict__ Kf,
                                                               cx<double>* __restrict__ X, cx<double>* __restrict__ O,
                                                               llg::FftPlan plan, const cx<double>* __restrict__ tab,
                                                               const cx<double>* __restrict__ tw) {
@@ -176,13 +179,13 @@ __global__ void __launch_bounds__(kOpenThreads) k_open_column(int nx, int ny, co
     const llg::r4<double>* kc = Kf + (long long)kx * (ny + 1);
     for (int par = 1; par >= 0; --par) {
         for (int c = 0; c < 3; ++c)
-            for (int y = threadIdx.x; y < L; y += kOpenThreads) {
+            for (int y = threadIdx.x; y < L; y += blockDim.x) {
                 const cx<double> x = X[c * plane + col + y];
                 A[c * LP + plan.at(y)] = par ? llg::cmul(x, tw[y]) : x;
             }
         __syncthreads();
         cx<double>* res = llg::fft_smem<double, false>(A, B, 3, plan, tab, tw);
-        for (int kk = threadIdx.x; kk < L; kk += kOpenThreads) {
+        for (int kk = threadIdx.x; kk < L; kk += blockDim.x) {
             const int ky = 2 * kk + par;
             const llg::r4<double> K = kc[ky <= ny ? ky : 2 * ny - ky];
             const double kxy = ky <= ny ? K.y : -K.y;
@@ -195,7 +198,7 @@ __global__ void __launch_bounds__(kOpenThreads) k_open_column(int nx, int ny, co
         __syncthreads();
         const cx<double>* r2 = llg::fft_smem<double, true>(res, res == A ? B : A, 3, plan, tab, tw);
         for (int c = 0; c < 3; ++c)
-            for (int y = threadIdx.x; y < L; y += kOpenThreads) {
+            for (int y = threadIdx.x; y < L; y += blockDim.x) {
                 const cx<double> v = r2[c * LP + plan.at(y)];
                 const long long o = c * plane + col + y;   // every y by the same thread in both rounds
                 if (par) O[o] = llg::cmulc(v, tw[y]);
@@ -311,6 +314,7 @@ void open_path_create(llg_demag_op* op) {
     constexpr size_t kMax = 227 * 1024;
     op->plan_nx = llg::padded_plan(llg::make_plan(op->nx), true, 4, kMax);
     op->plan_ny = llg::padded_plan(llg::make_plan(op->ny), true, 6, kMax);
+    op->column_threads = llg::fft_block_threads(op->plan_ny, 3, 12, kOpenColumnMax);
     auto attr = [&](const void* f) {
         return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax) == cudaSuccess;
     };
@@ -346,7 +350,7 @@ int demag_op_apply_device(llg_demag_op* op, double ms, const double* d_m_aos, do
         const int rows = 3 * ((op->ny + 1) / 2);
         k_open_rows_forward<<<rows, kOpenThreads, row, s>>>(op->nx, op->ny, ms, d_m_aos, X, op->plan_nx, op->tab_nx,
                                                             twx);
-        k_open_column<<<op->nx + 1, kOpenThreads, col, s>>>(op->nx, op->ny, op->Kf, X, O, op->plan_ny, op->tab_ny, twy);
+        k_open_column<<<op->nx + 1, op->column_threads, col, s>>>(op->nx, op->ny, op->Kf, X, O, op->plan_ny, op->tab_ny, twy);
         k_open_rows_inverse<<<rows, kOpenThreads, row, s>>>(op->nx, op->ny, X, op->plan_nx, op->tab_nx, twx, d_b_aos);
         PBC_TRY(cudaGetLastError());
         return LLG_OK;

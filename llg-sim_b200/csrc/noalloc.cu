@@ -26,7 +26,7 @@ constexpr size_t kScratchBytes = size_t(32) << 20;  // 32 MiB
 constexpr int kMaxDevices = 64;
 constexpr int kMaxLen = 2048;  // largest nx, ny
 constexpr int kT = 2;          // rows per block
-constexpr int kThreads = 256;
+constexpr int kThreads = 512;  // most threads per block (fft_block_threads)
 
 // The shared scratch.  In host code this name is only a stand-in for the
 // device array; kernels receive its device address from cudaGetSymbolAddress.
@@ -288,13 +288,15 @@ extern "C" int llg_demag_field_noalloc(int64_t nx, int64_t ny, double ms, const 
     const size_t smem_row = 4 * (size_t)G * prow.stride() * sizeof(cx<float>);
     const size_t smem_col = 12 * (size_t)nc * pcol.stride() * sizeof(cx<float>);
     const int row_blocks = (iny + kT - 1) / kT;
+    const int row_threads = fft_block_threads(prow, 2 * G, 6 * kT, kThreads);
+    const int col_threads = fft_block_threads(pcol, 6 * nc, 8 * nc, kThreads);
     k_na_twiddles<<<(2 * inx + 2 * iny + 255) / 256, 256, 0, s>>>(tw_row, inx, tw_col, iny, prow, pcol, pass_row,
                                                                  pass_col);
-    k_na_rows_forward<<<row_blocks, kThreads, smem_row, s>>>(inx, iny, (float)ms, m, X, pass_row, tw_row, prow);
-    k_na_column<<<(inx + nc) / nc, kThreads, smem_col, s>>>(inx, iny, nc, kernel_planes,
+    k_na_rows_forward<<<row_blocks, row_threads, smem_row, s>>>(inx, iny, (float)ms, m, X, pass_row, tw_row, prow);
+    k_na_column<<<(inx + nc) / nc, col_threads, smem_col, s>>>(inx, iny, nc, kernel_planes,
                                                             1.0 / (4.0 * (double)nx * (double)ny), X, pass_col, tw_col,
                                                             pcol);
-    k_na_rows_inverse<<<row_blocks, kThreads, smem_row, s>>>(inx, iny, X, pass_row, tw_row, prow, b_out);
+    k_na_rows_inverse<<<row_blocks, row_threads, smem_row, s>>>(inx, iny, X, pass_row, tw_row, prow, b_out);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         std::snprintf(msg, sizeof(msg), "llg_demag_field_noalloc: launch failed: %s", cudaGetErrorString(e));
