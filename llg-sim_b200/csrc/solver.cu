@@ -1383,6 +1383,12 @@ struct Engine final : EngineBase {
         return LLG_OK;
     }
 
+    // Attempts (iterations) per graph: 8, or 2 where a pass has several segments — their
+    // graphs have a node per segment and the forks and joins between them, and an attempt
+    // of a mixed batch runs for long enough to hide its launch (64 mixed films: the first
+    // pass of a new batch pays 13 ms for a graph of 8).
+    int graph_reps() const { return rseg.size() > 1 || cseg.size() > 1 ? 2 : 8; }
+
     static long long graph_key(int kind, int fmask, int reps) {
         return ((long long)kind << 40) | ((long long)fmask << 32) | (long long)reps;
     }
@@ -1503,11 +1509,11 @@ struct Engine final : EngineBase {
         if ((rc = set_control(c, p, inv.get(), false))) return rc;
         // Poll the device every 32 attempts.  With a step-count target no film can
         // finish in fewer attempts than its remaining steps, so a round launches at
-        // most the smallest remaining count (graphs of 8 attempts, the rest one by one)
+        // most the smallest remaining count (graphs of several attempts, the rest one by one)
         // and no attempt is launched after every film is done.  With an end time a round
         // is no longer than the steps of the current size that are left of it (an idle
         // attempt costs its launches, 25 to 45 us).
-        const int reps = 8;
+        const int reps = graph_reps();
         cudaGraphExec_t ge = nullptr;
         if ((rc = attempt_graph(kind, fmask, reps, &ge))) return rc;
         if ((rc = eval(stage1_spec(kind, fmask, 0)))) return rc;
@@ -1614,7 +1620,7 @@ struct Engine final : EngineBase {
         k_relax_control<<<(nf + 127) / 128, 128, 0, stream>>>(d_films, d_relax, nf, S);
         CUDA_TRY(cudaGetLastError());
         launches += 1;
-        const int reps = 8;
+        const int reps = graph_reps(), unit = 8 / reps;   // graphs per 8 iterations
         const long long key = graph_key(KIND_RELAX, fmask, reps);
         // the graph bakes the settings into the controller launches: rebuild when they differ
         if (graphs.count(key) && std::memcmp(&relax_graph_settings, &S, sizeof(S)) != 0) {
@@ -1633,9 +1639,9 @@ struct Engine final : EngineBase {
         long long iters = 0;
         int per_poll = 4;
         for (;;) {
-            for (int q = 0; q < per_poll; ++q)
+            for (int q = 0; q < per_poll * unit; ++q)
                 if ((rc = graph_launch(key, ge))) return rc;
-            iters += per_poll * reps;
+            iters += per_poll * 8;
             if (iters > max_iters)
                 return set_error(LLG_ERR_TIMEOUT, "relax did not finish within %lld iterations", max_iters);
             CUDA_TRY(cudaMemcpyAsync(h_relax, d_relax, sizeof(RelaxStateDev) * nf, cudaMemcpyDeviceToHost, stream));
@@ -1649,7 +1655,7 @@ struct Engine final : EngineBase {
                 if (!done) left = std::max(left, st->max_accepted_steps - h_relax[f].accepted + 1);
             }
             if (all) break;
-            per_poll = (int)std::min<long long>(4, (left + reps - 1) / reps);
+            per_poll = (int)std::min<long long>(4, (left + 7) / 8);
         }
         for (int f = 0; f < nf; ++f) {
             const RelaxStateDev& Q = h_relax[f];
@@ -1709,7 +1715,7 @@ struct Engine final : EngineBase {
         k_minimize_begin<<<(nf + 127) / 128, 128, 0, stream>>>(d_films, d_min, nf);
         CUDA_TRY(cudaGetLastError());
         launches += 1;
-        const int reps = 8;
+        const int reps = graph_reps(), unit = 8 / reps;   // graphs per 8 iterations
         const long long key = graph_key(KIND_MINIMIZE, fmask, reps);
         // the graph bakes the settings into the controller launches: rebuild when they differ
         if (graphs.count(key) && std::memcmp(&minimize_graph_settings, &S, sizeof(S)) != 0) {
@@ -1722,18 +1728,18 @@ struct Engine final : EngineBase {
         cudaGraphExec_t ge = nullptr;
         if ((rc = get_graph(key, reps, [&]() { return launch_minimize_iteration(fmask, S); }, &ge))) return rc;
         // every film finishes within max_iters iterations; the bound is a safety net
-        const long long bound = std::max<long long>(st->max_iters, 0) + 4 * reps;
+        const long long bound = std::max<long long>(st->max_iters, 0) + 32;
         long long iters = 0;
         int per_poll = 1;
         bool all = true;
         for (int f = 0; f < nf; ++f) all &= h_min[f].done != 0;
         while (!all) {
-            for (int q = 0; q < per_poll; ++q)
+            for (int q = 0; q < per_poll * unit; ++q)
                 if ((rc = graph_launch(key, ge))) return rc;
-            iters += (long long)per_poll * reps;
+            iters += (long long)per_poll * 8;
             // no more than max_iters leaves to do: a finished film's iteration still costs its launches
             per_poll = (int)std::max<long long>(
-                1, std::min<long long>(std::min(per_poll * 2, 8), (st->max_iters - iters + reps - 1) / reps));
+                1, std::min<long long>(std::min(per_poll * 2, 8), (st->max_iters - iters + 7) / 8));
             CUDA_TRY(cudaMemcpyAsync(h_min, d_min, sizeof(MinimizeStateDev) * nf, cudaMemcpyDeviceToHost, stream));
             CUDA_TRY(cudaStreamSynchronize(stream));
             all = true;
