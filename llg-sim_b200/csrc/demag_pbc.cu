@@ -128,7 +128,7 @@ constexpr int kOpenThreads = 256;
 // Signal w of a row pair p (rows j0 = 2p, j0+1): w = 0, 1: x + i y of row j0 + w;
 // w = 2: z of row j0 + i z of row j0 + 1.  One signal per block: two transforms
 // in 4 padded buffers, so that two blocks fit an SM at nx = 1536.
-__global__ void __launch_bounds__(kOpenThreads) k_open_rows_forward(int nx, int ny, double ms,
+__global__ void __launch_bounds__(kOpenThreads, 2) k_open_rows_forward(int nx, int ny, double ms,
                                                                     const double* __restrict__ m,
                                                                     cx<double>* __restrict__ X, llg::FftPlan plan,
                                                                     const cx<double>* __restrict__ tab,
@@ -141,6 +141,7 @@ __global__ void __launch_bounds__(kOpenThreads) k_open_rows_forward(int nx, int 
     const int ja = w < 2 ? 2 * p + w : 2 * p, jb = 2 * p + 1;
     if (ja >= ny) return;
     const bool second = w < 2 || jb < ny;
+#pragma unroll 2
     for (int i = threadIdx.x; i < L; i += kOpenThreads) {
         const double* a = m + ((long long)ja * nx + i) * 3;
         cx<double> v;
@@ -164,52 +165,85 @@ __global__ void __launch_bounds__(kOpenThreads) k_open_rows_forward(int nx, int 
 
 constexpr int kOpenColumnMax = 512;   // most threads of a column block (fft_block_threads)
 
-// One kx column: the odd and then the even ky bins of the three components (six
-// padded buffers at a time, so that ny = 2048 fits), product with the folded kernel
-// and inverse.  The odd half waits in O, the even half adds it and replaces X.
+// Two signals of a pair q of columns (kx = 2q, 2q + 1): w = 0, 1: x and y of column
+// 2q + w, which the kernel couples; w = 2: z of both.  The odd and then the even ky
+// bins (four padded buffers at a time), product with the folded kernel and inverse;
+// the odd half waits in O, the even half adds it and replaces X.
+//
+// What bounds it: shared-memory passes, FP64 butterflies and the waits between them.
+// Two signals per block let two blocks of 256 threads share an SM at ny = 1536, so
+// that the passes of one fill the waits of the other; with all three components of a
+// column per block (one block of 512 threads) the kernel took 412 us there, now 343 us.
 __global__ void __launch_bounds__(kOpenColumnMax) k_open_column(int nx, int ny, const llg::r4<double>* __restrict__ Kf,
                                                               cx<double>* __restrict__ X, cx<double>* __restrict__ O,
                                                               llg::FftPlan plan, const cx<double>* __restrict__ tab,
                                                               const cx<double>* __restrict__ tw) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int L = ny, LP = plan.stride(), kx = blockIdx.x;
-    const long long plane = (long long)(nx + 1) * ny, col = (long long)kx * ny;
+    const int L = ny, LP = plan.stride();
+    const int q = blockIdx.x / 3, w = blockIdx.x - 3 * q;
+    const int ka = w < 2 ? 2 * q + w : 2 * q;
+    if (ka > nx) return;
+    const bool second = w < 2 || ka + 1 <= nx;
+    const long long plane = (long long)(nx + 1) * ny, other = w < 2 ? plane : ny;   // first to second signal
     cx<double>* A = reinterpret_cast<cx<double>*>(smem_raw);
-    cx<double>* B = A + 3 * LP;
-    const llg::r4<double>* kc = Kf + (long long)kx * (ny + 1);
+    cx<double>* B = A + 2 * LP;
+    cx<double>* xc = X + (w < 2 ? 0 : 2 * plane) + (long long)ka * ny;
+    cx<double>* oc = O + (w < 2 ? 0 : 2 * plane) + (long long)ka * ny;
+    const llg::r4<double>* kc = Kf + (long long)ka * (ny + 1);
+    const llg::r4<double>* kd = w == 2 && second ? kc + (ny + 1) : kc;
     for (int par = 1; par >= 0; --par) {
-        for (int c = 0; c < 3; ++c)
-            for (int y = threadIdx.x; y < L; y += blockDim.x) {
-                const cx<double> x = X[c * plane + col + y];
-                A[c * LP + plan.at(y)] = par ? llg::cmul(x, tw[y]) : x;
-            }
-        __syncthreads();
-        cx<double>* res = llg::fft_smem<double, false>(A, B, 3, plan, tab, tw);
-        for (int kk = threadIdx.x; kk < L; kk += blockDim.x) {
-            const int ky = 2 * kk + par;
-            const llg::r4<double> K = kc[ky <= ny ? ky : 2 * ny - ky];
-            const double kxy = ky <= ny ? K.y : -K.y;
-            cx<double>* s = res + plan.at(kk);
-            const cx<double> Mx = s[0], My = s[LP], Mz = s[2 * LP];
-            s[0] = mkc(K.x * Mx.re + kxy * My.re, K.x * Mx.im + kxy * My.im);
-            s[LP] = mkc(kxy * Mx.re + K.z * My.re, kxy * Mx.im + K.z * My.im);
-            s[2 * LP] = mkc(K.w * Mz.re, K.w * Mz.im);
+#pragma unroll 2
+        for (int y = threadIdx.x; y < L; y += blockDim.x) {
+            const cx<double> x0 = xc[y], x1 = second ? xc[other + y] : mkc(0.0, 0.0), t = tw[y];
+            const cx<double> t0 = llg::cmul(x0, t), t1 = llg::cmul(x1, t);
+            const int at = plan.at(y);
+            A[at] = mkc(par ? t0.re : x0.re, par ? t0.im : x0.im);
+            A[LP + at] = mkc(par ? t1.re : x1.re, par ? t1.im : x1.im);
         }
         __syncthreads();
-        const cx<double>* r2 = llg::fft_smem<double, true>(res, res == A ? B : A, 3, plan, tab, tw);
-        for (int c = 0; c < 3; ++c)
-            for (int y = threadIdx.x; y < L; y += blockDim.x) {
-                const cx<double> v = r2[c * LP + plan.at(y)];
-                const long long o = c * plane + col + y;   // every y by the same thread in both rounds
-                if (par) O[o] = llg::cmulc(v, tw[y]);
-                else X[o] = v + O[o];
+        cx<double>* res = llg::fft_smem<double, false>(A, B, 2, plan, tab, tw);
+#pragma unroll 2
+        for (int kk = threadIdx.x; kk < L; kk += blockDim.x) {
+            const int ky = 2 * kk + par, kf = ky <= ny ? ky : 2 * ny - ky;
+            cx<double>* s = res + plan.at(kk);
+            const cx<double> Ma = s[0], Mb = s[LP];
+            const llg::r4<double> K = kc[kf];
+            if (w < 2) {
+                const double kxy = ky <= ny ? K.y : -K.y;
+                s[0] = mkc(K.x * Ma.re + kxy * Mb.re, K.x * Ma.im + kxy * Mb.im);
+                s[LP] = mkc(kxy * Ma.re + K.z * Mb.re, kxy * Ma.im + K.z * Mb.im);
+            } else {
+                const double kb = kd[kf].w;
+                s[0] = mkc(K.w * Ma.re, K.w * Ma.im);
+                s[LP] = mkc(kb * Mb.re, kb * Mb.im);
             }
+        }
+        __syncthreads();
+        const cx<double>* r2 = llg::fft_smem<double, true>(res, res == A ? B : A, 2, plan, tab, tw);
+        // every y by the same thread in both rounds
+        if (par) {
+#pragma unroll 2
+            for (int y = threadIdx.x; y < L; y += blockDim.x) {
+                const cx<double> t = tw[y];
+                const int at = plan.at(y);
+                oc[y] = llg::cmulc(r2[at], t);
+                if (second) oc[other + y] = llg::cmulc(r2[LP + at], t);
+            }
+        } else {
+#pragma unroll 2
+            for (int y = threadIdx.x; y < L; y += blockDim.x) {
+                const cx<double> o0 = oc[y], o1 = second ? oc[other + y] : mkc(0.0, 0.0);
+                const int at = plan.at(y);
+                xc[y] = r2[at] + o0;
+                if (second) xc[other + y] = r2[LP + at] + o1;
+            }
+        }
         __syncthreads();
     }
 }
 
 // Signals as in the forward pass; the field goes to the AoS output.
-__global__ void __launch_bounds__(kOpenThreads) k_open_rows_inverse(int nx, int ny, const cx<double>* __restrict__ X,
+__global__ void __launch_bounds__(kOpenThreads, 2) k_open_rows_inverse(int nx, int ny, const cx<double>* __restrict__ X,
                                                                     llg::FftPlan plan,
                                                                     const cx<double>* __restrict__ tab,
                                                                     const cx<double>* __restrict__ tw,
@@ -225,6 +259,7 @@ __global__ void __launch_bounds__(kOpenThreads) k_open_rows_inverse(int nx, int 
     const int c0 = w < 2 ? 0 : 2;
     const cx<double>* xa = X + (long long)c0 * K1 * ny + ja;
     const cx<double>* xb = w < 2 ? X + (long long)K1 * ny + ja : X + (long long)2 * K1 * ny + jb;
+#pragma unroll 4
     for (int k = threadIdx.x; k < K1; k += kOpenThreads) {
         const cx<double> u = xa[(long long)k * ny];
         const cx<double> v = second ? xb[(long long)k * ny] : mkc(0.0, 0.0);
@@ -313,8 +348,11 @@ void open_path_create(llg_demag_op* op) {
     }
     constexpr size_t kMax = 227 * 1024;
     op->plan_nx = llg::padded_plan(llg::make_plan(op->nx), true, 4, kMax);
-    op->plan_ny = llg::padded_plan(llg::make_plan(op->ny), true, 6, kMax);
-    op->column_threads = llg::fft_block_threads(op->plan_ny, 3, 12, kOpenColumnMax);
+    op->plan_ny = llg::padded_plan(llg::make_plan(op->ny), true, 4, kMax);
+    // 128 registers a thread: two blocks of 256 where their buffers fit an SM (1 KiB of
+    // each is reserved), one of 512 where they do not
+    const bool two = 2 * (4 * (size_t)op->plan_ny.stride() * sizeof(cx<double>) + 1024) <= kMax + 1024;
+    op->column_threads = llg::fft_block_threads(op->plan_ny, 2, 8, two ? 256 : kOpenColumnMax);
     auto attr = [&](const void* f) {
         return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax) == cudaSuccess;
     };
@@ -346,11 +384,12 @@ int demag_op_apply_device(llg_demag_op* op, double ms, const double* d_m_aos, do
         const cx<double>* twx = op->tab_nx + 2 * op->nx;
         const cx<double>* twy = op->tab_ny + 2 * op->ny;
         const size_t row = 4 * (size_t)op->plan_nx.stride() * sizeof(cx<double>);
-        const size_t col = 6 * (size_t)op->plan_ny.stride() * sizeof(cx<double>);
+        const size_t col = 4 * (size_t)op->plan_ny.stride() * sizeof(cx<double>);
         const int rows = 3 * ((op->ny + 1) / 2);
         k_open_rows_forward<<<rows, kOpenThreads, row, s>>>(op->nx, op->ny, ms, d_m_aos, X, op->plan_nx, op->tab_nx,
                                                             twx);
-        k_open_column<<<op->nx + 1, op->column_threads, col, s>>>(op->nx, op->ny, op->Kf, X, O, op->plan_ny, op->tab_ny, twy);
+        k_open_column<<<3 * (op->nx / 2 + 1), op->column_threads, col, s>>>(op->nx, op->ny, op->Kf, X, O, op->plan_ny,
+                                                                          op->tab_ny, twy);
         k_open_rows_inverse<<<rows, kOpenThreads, row, s>>>(op->nx, op->ny, X, op->plan_nx, op->tab_nx, twx, d_b_aos);
         PBC_TRY(cudaGetLastError());
         return LLG_OK;

@@ -57,3 +57,13 @@ def test_asymmetric_real_planes_keep_the_general_path(gpu, orc, tmp_path):
     want = _convolve(k, MS, m, nx, ny)
     assert np.abs(op.field(MS, m) - want).max() <= 1e-10 * np.abs(want).max()
     op.close()
+
+
+@pytest.mark.parametrize("nx,ny", [(3, 300), (2, 1536), (5, 2048), (600, 7), (2048, 2)])
+def test_open_path_long_columns_and_rows(gpu, orc, nx, ny):
+    """Column blocks of 128 to 512 threads, rows of several rounds of the grouped loads."""
+    m = orc.init_random(nx * ny, 5 + nx)
+    op = gpu.DemagOp(gpu.Grid2D(nx, ny, DX, DY, DZ), 0, 0)
+    want = _convolve(op.kspace().reshape(4, 2 * ny, 2 * nx), MS, m, nx, ny)
+    assert np.abs(op.field(MS, m) - want).max() <= 1e-10 * np.abs(want).max()
+    op.close()
