@@ -36,11 +36,13 @@ constexpr int kRedThreads = 256;
 // Both operands MN-major, no swizzle: element (mn, k) of a tile sits at byte
 // (k / 8) * LBO + (mn / 8) * SBO + (k % 8) * 16 + (mn % 8) * 2 with SBO = 128
 // (the 8-channel groups of one cell group are adjacent) and LBO = (MN / 8) * 128.
-// Measured at 16 films of 128 x 128 cells, 32 channels: 127 us per layer with one
-// 64-bit division per 16-byte chunk of the gather (a thread's time went into index
-// arithmetic).
+// What bounds it: the gather (nine reads of every activation through L1 and as many
+// shared-memory writes).  Measured at 16 films of 128 x 128 cells, 32 channels: 127 us
+// per layer with one 64-bit division per 16-byte chunk of the gather, 44 us with the
+// image position formed once per chunk, 33 us with loads of 512 consecutive bytes per
+// warp that are in flight while the tensor cores work on the chunk before.
 template <int CIN, int NN>
-__global__ void __launch_bounds__(128) k_wgrad_tc(const __nv_bfloat16* __restrict__ x,
+__global__ void __launch_bounds__(128, 4) k_wgrad_tc(const __nv_bfloat16* __restrict__ x,
                                                   const __nv_bfloat16* __restrict__ g, int nimg, int H, int W,
                                                   long long cells_per_cta, float* __restrict__ part, int* err,
                                                   long long spin) {
@@ -71,40 +73,59 @@ __global__ void __launch_bounds__(128) k_wgrad_tc(const __nv_bfloat16* __restric
     const uint32_t idesc = instr_desc_bf16(kTile, NN, true, true);
     uint32_t phase = 0;
     bool ok = true, first = true;
-    for (long long c0 = c_begin; c0 < c_end; c0 += kWgKC) {
-        // A: (cell k, tap, 8-channel group) -> one 16-byte chunk.  Thread t takes cell
-        // t % 64 and half of the groups: the image position is formed once per chunk, a
-        // thread's groups of a tap are one 32-byte sector (16 bytes for 16 channels), and
-        // eight neighbouring lanes store the 128 consecutive bytes of a core matrix.
-        {
-            const int k = t & (kWgKC - 1), half = t >> 6;
-            const long long p = c0 + k;
+    // A: (cell k, tap, 8-channel group) -> one 16-byte chunk.  A warp takes 16 cells;
+    // one of its loads is 32 / GROUPS neighbouring cells with all their groups, 512
+    // consecutive bytes.  The eight lanes of a 16-byte access phase are eight cells,
+    // each with the group that puts them on all banks, in the load (cells CIN * 2 bytes
+    // apart) as in the store (the 128 consecutive bytes of core matrices).
+    // B: (cell k, 8-channel group of the output gradient).
+    // All reads of a chunk are in flight together, and while the tensor cores work on
+    // the chunk before.
+    constexpr int VA = GROUPS / 2, VB = kWgKC * (NN / 8) / 128;
+    static_assert(kWgKC * (NN / 8) % 128 == 0, "whole rounds of 128 threads");
+    static_assert(kWgKC == 64 && (GROUPS == 2 || GROUPS == 4) && kTile % CIN == 0, "gather layout");
+    uint4 va[9 * VA], vb[VB];
+    const int lane = t & 31, cg = (((lane & 7) >> (GROUPS == 4 ? 1 : 2)) + (lane >> 3)) & (GROUPS - 1);
+    const int ka = warp * 16 + (lane / (8 * GROUPS)) * 8 + (lane & 7);   // + b * 8 for batch b
+    auto load = [&](long long c0) {
+#pragma unroll
+        for (int b = 0; b < VA; ++b) {
+            const long long p = c0 + ka + b * 8;
             const bool valid = p < c_end;
             const unsigned pu = valid ? (unsigned)p : 0u;   // fewer than 2^28 cells
             const unsigned rem = pu % (unsigned)hw;
             const int yy = (int)(rem / (unsigned)W), xx = (int)(rem % (unsigned)W);
             const __nv_bfloat16* xc = x + (long long)pu * CIN;
-            unsigned char* ak = As + (k >> 3) * A_LBO + (k & 7) * 16;
 #pragma unroll
             for (int tap = 0; tap < 9; ++tap) {
                 const int dy = tap / 3 - 1, dx = tap % 3 - 1;
                 const bool in = valid && yy + dy >= 0 && yy + dy < H && xx + dx >= 0 && xx + dx < W;
                 const uint4* src = reinterpret_cast<const uint4*>(xc + ((long long)dy * W + dx) * CIN);
-#pragma unroll
-                for (int q = 0; q < GROUPS / 2; ++q) {
-                    const int cg = half * (GROUPS / 2) + q;
-                    const uint4 v = in ? src[cg] : make_uint4(0u, 0u, 0u, 0u);
-                    const int m = tap * CIN + cg * 8;
-                    *reinterpret_cast<uint4*>(ak + (m / kTile) * A_TILE + ((m % kTile) >> 3) * 128) = v;
-                }
+                va[tap * VA + b] = in ? src[cg] : make_uint4(0u, 0u, 0u, 0u);
             }
         }
-        // B: (cell k, 8-channel group of the output gradient)
-        for (int e = t; e < kWgKC * (NN / 8); e += 128) {
-            const int k = e / (NN / 8), ng = e - k * (NN / 8);
-            const long long p = c0 + k;
-            const uint4 v = p < c_end ? reinterpret_cast<const uint4*>(g + p * NN)[ng] : make_uint4(0u, 0u, 0u, 0u);
-            *reinterpret_cast<uint4*>(Bs + (k >> 3) * B_LBO + ng * 128 + (k & 7) * 16) = v;
+#pragma unroll
+        for (int r = 0; r < VB; ++r) {
+            const int e = t + r * 128, kb = e / (NN / 8), ng = e - kb * (NN / 8);
+            const long long pb = c0 + kb;
+            vb[r] = pb < c_end ? reinterpret_cast<const uint4*>(g + pb * NN)[ng] : make_uint4(0u, 0u, 0u, 0u);
+        }
+    };
+    if (c_begin < c_end) load(c_begin);
+    for (long long c0 = c_begin; c0 < c_end; c0 += kWgKC) {
+#pragma unroll
+        for (int b = 0; b < VA; ++b) {
+            unsigned char* ak = As + ((ka >> 3) + b) * A_LBO + (ka & 7) * 16 + cg * 128;
+#pragma unroll
+            for (int tap = 0; tap < 9; ++tap) {
+                const int m = tap * CIN;
+                *reinterpret_cast<uint4*>(ak + (m / kTile) * A_TILE + ((m % kTile) >> 3) * 128) = va[tap * VA + b];
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < VB; ++r) {
+            const int e = t + r * 128, kb = e / (NN / 8), ng = e - kb * (NN / 8);
+            *reinterpret_cast<uint4*>(Bs + (kb >> 3) * B_LBO + ng * 128 + (kb & 7) * 16) = vb[r];
         }
         fence_async_smem();
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -121,6 +142,7 @@ __global__ void __launch_bounds__(128) k_wgrad_tc(const __nv_bfloat16* __restric
             mma_commit(&bar);
         }
         first = false;
+        if (c0 + kWgKC < c_end) load(c0 + kWgKC);
         // the chunk buffers are rewritten only after these MMAs have read them
         ok = mbar_wait_n(&bar, phase, spin);
         phase ^= 1u;
