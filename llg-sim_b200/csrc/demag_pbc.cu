@@ -125,9 +125,11 @@ __global__ void k_pbc_extract(const cx<double>* __restrict__ M, int nx, int ny, 
 // kernel (75 MB), the field out.
 constexpr int kOpenThreads = 256;
 
-// Signal w of a row pair p (rows j0 = 2p, j0+1): w = 0, 1: x + i y of row j0 + w;
-// w = 2: z of row j0 + i z of row j0 + 1.  One signal per block: two transforms
-// in 4 padded buffers, so that two blocks fit an SM at nx = 1536.
+// Component w of a row pair p (rows j0 = 2p, j0+1): row j0 + i row j0+1.  One signal
+// per block: two transforms in 4 padded buffers, so that two blocks fit an SM at
+// nx = 1536.  The two rows of a bin are neighbours in X: a lane pair takes them, so
+// that every store is a whole 32-byte sector (at nx = ny = 1536 the forward rows went
+// from 151 to 110 us, the inverse from 152 to 136).
 __global__ void __launch_bounds__(kOpenThreads, 2) k_open_rows_forward(int nx, int ny, double ms,
                                                                     const double* __restrict__ m,
                                                                     cx<double>* __restrict__ X, llg::FftPlan plan,
@@ -137,29 +139,27 @@ __global__ void __launch_bounds__(kOpenThreads, 2) k_open_rows_forward(int nx, i
     const int L = nx, LP = plan.stride(), K1 = nx + 1;
     cx<double>* A = reinterpret_cast<cx<double>*>(smem_raw);
     cx<double>* B = A + 2 * LP;
-    const int p = blockIdx.x / 3, w = blockIdx.x - 3 * p;
-    const int ja = w < 2 ? 2 * p + w : 2 * p, jb = 2 * p + 1;
-    if (ja >= ny) return;
-    const bool second = w < 2 || jb < ny;
-#pragma unroll 2
+    const int p = blockIdx.x / 3, w = blockIdx.x - 3 * p, ja = 2 * p;
+    const bool second = ja + 1 < ny;
+    const double* ma = m + (long long)ja * nx * 3 + w;
+    const double* mb = ma + (second ? (long long)nx * 3 : 0);
+#pragma unroll 4
     for (int i = threadIdx.x; i < L; i += kOpenThreads) {
-        const double* a = m + ((long long)ja * nx + i) * 3;
-        cx<double> v;
-        if (w < 2) v = mkc(ms * a[0], ms * a[1]);
-        else v = mkc(ms * a[2], second ? ms * m[((long long)jb * nx + i) * 3 + 2] : 0.0);
+        const double a = ma[3 * (long long)i], b = mb[3 * (long long)i];
+        const cx<double> v = mkc(ms * a, second ? ms * b : 0.0);
         A[plan.at(i)] = v;
         A[LP + plan.at(i)] = llg::cmul(v, tw[i]);
     }
     __syncthreads();
     const cx<double>* res = llg::fft_smem<double, false>(A, B, 2, plan, tab, tw);
-    const int c0 = w < 2 ? 0 : 2;
-    cx<double>* xa = X + (long long)c0 * K1 * ny + ja;
-    cx<double>* xb = w < 2 ? X + (long long)K1 * ny + ja : X + (long long)2 * K1 * ny + jb;
-    for (int k = threadIdx.x; k < K1; k += kOpenThreads) {
+    const int r = threadIdx.x & 1;
+    if (r && !second) return;
+    cx<double>* x = X + (long long)w * K1 * ny + ja + r;
+    for (int k = threadIdx.x >> 1; k < K1; k += kOpenThreads / 2) {
         const int km = k ? 2 * L - k : 0;
         const cx<double> zk = res[(k & 1) * LP + plan.at(k >> 1)], zm = res[(km & 1) * LP + plan.at(km >> 1)];
-        xa[(long long)k * ny] = mkc(0.5 * (zk.re + zm.re), 0.5 * (zk.im - zm.im));
-        if (second) xb[(long long)k * ny] = mkc(0.5 * (zk.im + zm.im), 0.5 * (zm.re - zk.re));
+        x[(long long)k * ny] = r ? mkc(0.5 * (zk.im + zm.im), 0.5 * (zm.re - zk.re))
+                                 : mkc(0.5 * (zk.re + zm.re), 0.5 * (zk.im - zm.im));
     }
 }
 
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(kOpenColumnMax) k_open_column(int nx, int ny, 
     }
 }
 
-// Signals as in the forward pass; the field goes to the AoS output.
+// Signals and lane pairs as in the forward pass; the field goes to the AoS output.
 __global__ void __launch_bounds__(kOpenThreads, 2) k_open_rows_inverse(int nx, int ny, const cx<double>* __restrict__ X,
                                                                     llg::FftPlan plan,
                                                                     const cx<double>* __restrict__ tab,
@@ -252,33 +252,25 @@ __global__ void __launch_bounds__(kOpenThreads, 2) k_open_rows_inverse(int nx, i
     const int L = nx, LP = plan.stride(), K1 = nx + 1;
     cx<double>* A = reinterpret_cast<cx<double>*>(smem_raw);
     cx<double>* B = A + 2 * LP;
-    const int p = blockIdx.x / 3, w = blockIdx.x - 3 * p;
-    const int ja = w < 2 ? 2 * p + w : 2 * p, jb = 2 * p + 1;
-    if (ja >= ny) return;
-    const bool second = w < 2 || jb < ny;
-    const int c0 = w < 2 ? 0 : 2;
-    const cx<double>* xa = X + (long long)c0 * K1 * ny + ja;
-    const cx<double>* xb = w < 2 ? X + (long long)K1 * ny + ja : X + (long long)2 * K1 * ny + jb;
+    const int p = blockIdx.x / 3, w = blockIdx.x - 3 * p, ja = 2 * p, r = threadIdx.x & 1;
+    const bool second = ja + 1 < ny, reads = !r || second;
+    const cx<double>* x = X + (long long)w * K1 * ny + ja + r;
 #pragma unroll 4
-    for (int k = threadIdx.x; k < K1; k += kOpenThreads) {
-        const cx<double> u = xa[(long long)k * ny];
-        const cx<double> v = second ? xb[(long long)k * ny] : mkc(0.0, 0.0);
-        A[(k & 1) * LP + plan.at(k >> 1)] = mkc(u.re - v.im, u.im + v.re);
-        const int km = 2 * L - k;   // conjugate bins: conj(u) + i conj(v)
-        if (k > 0 && k < L) A[(km & 1) * LP + plan.at(km >> 1)] = mkc(u.re + v.im, v.re - u.im);
+    for (int k0 = 0; k0 < K1; k0 += kOpenThreads / 2) {
+        const int k = k0 + (threadIdx.x >> 1), km = 2 * L - k;
+        const cx<double> a = reads && k < K1 ? x[(long long)k * ny] : mkc(0.0, 0.0);
+        // u of row ja and v of row ja + 1: bin k is u + i v, bin km conj(u) + i conj(v)
+        const cx<double> o = mkc(__shfl_xor_sync(0xffffffffu, a.re, 1), __shfl_xor_sync(0xffffffffu, a.im, 1));
+        if (!r && k < K1) A[(k & 1) * LP + plan.at(k >> 1)] = mkc(a.re - o.im, a.im + o.re);
+        if (r && k > 0 && k < L) A[(km & 1) * LP + plan.at(km >> 1)] = mkc(o.re + a.im, a.re - o.im);
     }
     __syncthreads();
     const cx<double>* res = llg::fft_smem<double, true>(A, B, 2, plan, tab, tw);
+    double* ba = b + (long long)ja * nx * 3 + w;
     for (int i = threadIdx.x; i < L; i += kOpenThreads) {
         const cx<double> z = res[plan.at(i)] + llg::cmulc(res[LP + plan.at(i)], tw[i]);
-        double* o = b + ((long long)ja * nx + i) * 3;
-        if (w < 2) {
-            o[0] = z.re;
-            o[1] = z.im;
-        } else {
-            o[2] = z.re;
-            if (second) b[((long long)jb * nx + i) * 3 + 2] = z.im;
-        }
+        ba[3 * (long long)i] = z.re;
+        if (second) ba[3 * ((long long)nx + i)] = z.im;
     }
 }
 
