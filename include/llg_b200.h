@@ -284,8 +284,8 @@ int llg_solver_launch_count(llg_solver* s, int64_t* out);
  *   kernel_planes device, FP64 [4][ny+1][nx+1]: the planes llg_demag_kernel_kspace returns
  *   b_out         device, FP32 SoA [3][ny][nx], overwritten with B_demag (T)
  *   stream        cudaStream_t or NULL; the call is asynchronous on it
- * Scratch: one static 32 MiB device array per GPU that loads the library,
- * held until exit; requires 1 <= nx, ny <= 2048 and
+ * Scratch: one static 32 MiB device array (and 64 KiB of twiddle tables) per
+ * GPU that loads the library, held until exit; requires 1 <= nx, ny <= 2048 and
  * 24*(nx+1)*ny + 16*(nx+ny) <= 32 MiB (e.g. 1024 x 1024), else LLG_ERR_INVALID.
  * The first call on a device looks up the array's device address and opts the
  * kernels into large shared memory; make that first call before any stream

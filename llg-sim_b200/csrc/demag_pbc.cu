@@ -118,11 +118,13 @@ __global__ void k_pbc_extract(const cx<double>* __restrict__ M, int nx, int ny, 
 // in ky), so a quarter of it serves all bins; forward transform, kernel product and
 // inverse of a column are one kernel.
 //
-// What bounds it: HBM.  At 1536 x 1536 cells the general path moves about 5.8 GB
-// (its padded planes are 453 MB and cross HBM twice in every pass), this one about
-// 0.8 GB: m in (56 MB), the spectrum [3][nx+1][ny] out and in twice (113 MB each
-// way), the odd-bin half of the columns through scratch (mostly L2), the folded
-// kernel (75 MB), the field out.
+// What bounds it: at 1536 x 1536 cells the general path moves about 5.8 GB through HBM
+// (its padded planes are 453 MB and cross it twice in every pass) and takes 4.7 ms;
+// this one about 0.8 GB (m in 56 MB, the spectrum [3][nx+1][ny] out and in twice, 113
+// MB each way, the odd-bin half of the columns through scratch, mostly L2, the folded
+// kernel 75 MB, the field out) in 0.59 ms.  What is left is latency: the FP64 buffers
+// leave an SM 16 warps and little L1 for the pass tables (L1 at 50 to 58 % of its
+// throughput, HBM at 11 to 13 %).
 constexpr int kOpenThreads = 256;
 
 // Component w of a row pair p (rows j0 = 2p, j0+1): row j0 + i row j0+1.  One signal
