@@ -86,10 +86,19 @@ struct FilmCtl {
 // ---------------------------------------------------------------------------
 // small kernels (one thread per film unless noted)
 // ---------------------------------------------------------------------------
+// Whether the film's k1 holds its present gamma and alpha (a torque contains both).
+// The reference keeps the torque of an accepted step whatever the caller changes them to
+// (llg.rs:854-867), but evaluates it again after a rejected attempt; a k1 kept over a
+// rejection is therefore only right while they are the ones it was evaluated with.
+__device__ __forceinline__ bool k1_current(const FilmDev& F, const StepState* st) {
+    return st->k1_gamma == F.gamma && st->k1_alpha == F.alpha;
+}
+
 __global__ void k_set_control(FilmDev* films, int nfilms, Control c, const FilmCtl* __restrict__ fc) {
     int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= nfilms) return;
-    StepState* st = films[f].st;
+    const FilmDev& F = films[f];
+    StepState* st = F.st;
     if (!fc[f].keep_dt) st->dt = fc[f].dt;
     st->t_end = c.t_end;
     st->max_err = c.max_err;
@@ -102,7 +111,7 @@ __global__ void k_set_control(FilmDev* films, int nfilms, Control c, const FilmC
     st->err_code = 0;
     st->err_bits = 0ull;
     st->req = REQ_NONE;
-    if (fc[f].invalidate_fsal) st->fsal_valid = 0;
+    if (fc[f].invalidate_fsal || (!st->accepted && !k1_current(F, st))) st->fsal_valid = 0;
     if (c.reset_time) st->t = 0.0;
     if (isfinite(c.t_end)) {
         double rem = c.t_end - st->t;
@@ -113,7 +122,8 @@ __global__ void k_set_control(FilmDev* films, int nfilms, Control c, const FilmC
 
 // Step-size controller of one film (llg.rs:997-1025 for order 5, llg.rs:401-435 for
 // order 3).
-__device__ void controller_core(StepState* st, int order) {
+__device__ void controller_core(const FilmDev& F, int order) {
+    StepState* st = F.st;
     const unsigned long long bits = st->err_bits;
     st->err_bits = 0ull;
     const double err = __longlong_as_double((long long)bits);
@@ -140,8 +150,13 @@ __device__ void controller_core(StepState* st, int order) {
     }
     // an accepted step flips k7 into k1; a rejected attempt leaves the state and k1's
     // buffer untouched: k1 = f(m0) holds either way, and is evaluated once, before the
-    // first attempt of a call
-    st->fsal_valid = 1;
+    // first attempt of a call (before the next one too where a rejected attempt used a
+    // k1 of other gamma or alpha)
+    if (acc || !st->fsal_valid) {   // evaluated in this call: k7, or stage 1
+        st->k1_gamma = F.gamma;
+        st->k1_alpha = F.alpha;
+    }
+    st->fsal_valid = acc || k1_current(F, st) ? 1 : 0;
     st->accepted = acc ? 1 : 0;
     st->dt = dt_next;
     if (st->attempts_left > 0) st->attempts_left -= 1;
@@ -157,8 +172,7 @@ __device__ void controller_core(StepState* st, int order) {
 __global__ void k_controller(FilmDev* films, int nfilms, int order) {
     int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= nfilms) return;
-    StepState* st = films[f].st;
-    if (st->active) controller_core(st, order);
+    if (films[f].st->active) controller_core(films[f], order);
 }
 
 // Sums the per-block partial reductions of one film (deterministic) into every
@@ -209,7 +223,7 @@ __global__ void k_finalize(FilmDev* films, int nfilms, int req, STATE* ctl, SETT
     finalize_film(F, acc);
     if (lane != 0) return;
     if constexpr (MODE == END_STEP) {
-        controller_core(st, 3);
+        controller_core(F, 3);
         if (!st->active) return;   // non-finite: the host finds err_code
     }
 #pragma unroll
@@ -1279,7 +1293,7 @@ struct Engine final : EngineBase {
     // Stages 2 to s of one integrator attempt and, for a run or a single step, the
     // controller (relax runs it at the end of its iteration).  Stage 1 is not among
     // them: the caller evaluates it once before its first attempt, since after any
-    // attempt k1 of the film's state is valid.  req gates every kernel on
+    // attempt k1 of the film's state is valid (run() treats the exception).  req gates every kernel on
     // StepState::req (relax).
     int launch_attempt(int kind, int fmask, int req, bool control = true) {
         int rc;
@@ -1504,6 +1518,15 @@ struct Engine final : EngineBase {
         c.target_acc = n_acc;
         c.attempts = max_attempts > 0 ? max_attempts : -1;
         c.reset_time = 1;
+        // A film whose k1 was evaluated with another gamma or alpha than this call's keeps it
+        // after an accepted step and needs a new one after a rejected one (k1_current): as
+        // long as there is such a film, attempts go out one by one, each after its stage 1.
+        auto other_k1 = [&](int f) {
+            const StepState& s = h_states[f];
+            return !s.fsal_valid || s.k1_gamma != p[f].gamma || s.k1_alpha != p[f].alpha;
+        };
+        bool by_one = false;
+        for (int f = 0; f < nf; ++f) by_one |= h_states[f].fsal_valid && other_k1(f);
         std::unique_ptr<bool[]> inv(new bool[nf]);
         fsal_flags(kind, p, fmask, inv.get());
         if ((rc = set_control(c, p, inv.get(), false))) return rc;
@@ -1537,6 +1560,8 @@ struct Engine final : EngineBase {
                     }
                 if (need < 32.0) round = (long long)need;
             }
+            if (!first && by_one && (rc = eval(stage1_spec(kind, fmask, 0)))) return rc;
+            if (by_one) round = 1;
             first = false;
             round = std::min(round, limit - launched);
             long long q = 0;
@@ -1549,6 +1574,10 @@ struct Engine final : EngineBase {
             bool any = false;
             for (int f = 0; f < nf; ++f) any |= h_states[f].active != 0;
             if (!any || launched >= limit) break;
+            if (by_one) {
+                by_one = false;
+                for (int f = 0; f < nf; ++f) by_one |= h_states[f].active && other_k1(f);
+            }
         }
         for (int f = 0; f < nf; ++f) {
             const StepState& s = h_states[f];

@@ -72,6 +72,7 @@ struct StepState {
     int err_code;
     int order;                    // 5 for RK45, 3 for RK23 (controller exponent 1/order)
     int req;                      // request of the device relax controller (ReqKind)
+    double k1_gamma, k1_alpha;    // gamma and alpha that the FSAL torque k1 was evaluated with
     double lam;                   // minimiser pseudo-step lambda of the next update
     double red[RED_NSLOT];        // finalised reductions of the last reduction pass
 };
