@@ -10,6 +10,8 @@ void llg_set_error_message(const char* msg);
 
 namespace llg {
 
+constexpr size_t kSmemMax = 227 * 1024;   // most shared memory of a block
+
 FftPlan make_plan(int L);
 // Radix plans of length L for the autotuner (the first is make_plan(L)), unpadded.
 std::vector<FftPlan> plan_candidates(int L);

@@ -509,6 +509,8 @@ cudaError_t conv_launch(const __nv_bfloat16* x, int nimg, int H, int W, const La
     const long long cells = (long long)nimg * H * W;
     if (cells <= 0) return cudaSuccess;
     const long long ntiles = (cells + kTile - 1) / kTile;
+    // the kernels' shared-memory limits are state of the process: always the ones of the
+    // widest layer, so that no thread lowers them between another one's setting and launch
     if (W <= kHaloW && (L.cin == 16 || L.cin == 32) && !conv_oneshot_forced()) {
         int dev = 0, nsm = 148;
         cudaGetDevice(&dev);
@@ -517,14 +519,16 @@ cudaError_t conv_launch(const __nv_bfloat16* x, int nimg, int H, int W, const La
         if (L.cin == 32) {
             const size_t smem = conv_pipe_smem_bytes<32>(L.npad);
             cudaError_t e = cudaFuncSetAttribute(k_conv3x3_pipe<NCOL, EPI, R, 32>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)conv_pipe_smem_bytes<32>(kCh));
             if (e != cudaSuccess) return e;
             k_conv3x3_pipe<NCOL, EPI, R, 32><<<grid, kPipeThreads, smem, s>>>(x, nimg, H, W, L, y, m_out, out32, mask, act,
                                                                         err, spin);
         } else {
             const size_t smem = conv_pipe_smem_bytes<16>(L.npad);
             cudaError_t e = cudaFuncSetAttribute(k_conv3x3_pipe<NCOL, EPI, R, 16>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)conv_pipe_smem_bytes<16>(kCh));
             if (e != cudaSuccess) return e;
             k_conv3x3_pipe<NCOL, EPI, R, 16><<<grid, kPipeThreads, smem, s>>>(x, nimg, H, W, L, y, m_out, out32, mask, act,
                                                                         err, spin);
@@ -533,7 +537,7 @@ cudaError_t conv_launch(const __nv_bfloat16* x, int nimg, int H, int W, const La
     }
     const size_t smem = conv_smem_bytes(L.cin, L.npad);
     cudaError_t e = cudaFuncSetAttribute(k_conv3x3_tc<NCOL, EPI, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+                                         (int)conv_smem_bytes(kCh, kCh));
     if (e != cudaSuccess) return e;
     k_conv3x3_tc<NCOL, EPI, R><<<(unsigned)ntiles, kTile, smem, s>>>(x, nimg, H, W, L, y, m_out, out32, mask, act, err,
                                                                      spin);

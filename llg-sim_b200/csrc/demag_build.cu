@@ -410,17 +410,18 @@ template <typename R>
 cudaError_t launch_fft_strided(void* data, const FftPlan& base, const void* tw, const void* tw2, long long elem_stride, int nsig_a,
                                long long stride_a, int nsig_b, long long stride_b, bool inverse, cudaStream_t s) {
     constexpr bool fp64 = sizeof(R) == 8;
-    constexpr size_t kMax = 227 * 1024;
     const int L = base.L;
+    // (the kernels' shared-memory limits are state of the process: always the largest, so
+    // that a thread with shorter signals does not lower them for another one)
     if (elem_stride > 1 && stride_a == 1) {
         // adjacent columns: tile NS of them per block where shared memory allows
         int ns = 1;
         while (ns < 8 && nsig_a % (2 * ns) == 0 && 2 * (size_t)(2 * ns) * L * sizeof(cx<R>) <= 200 * 1024) ns *= 2;
         if (ns > 1) {
-            const FftPlan plan = padded_plan(base, fp64, 2 * ns, kMax);
+            const FftPlan plan = padded_plan(base, fp64, 2 * ns, kSmemMax);
             const size_t smem = 2 * (size_t)ns * plan.stride() * sizeof(cx<R>);
             cudaError_t e = cudaFuncSetAttribute(k_fft_strided_tiled<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)smem);
+                                                 (int)kSmemMax);
             if (e != cudaSuccess) return e;
             k_fft_strided_tiled<R><<<(nsig_a / ns) * nsig_b, 256, smem, s>>>(
                 reinterpret_cast<cx<R>*>(data), plan, reinterpret_cast<const cx<R>*>(tw),
@@ -428,9 +429,10 @@ cudaError_t launch_fft_strided(void* data, const FftPlan& base, const void* tw, 
             return cudaGetLastError();
         }
     }
-    const FftPlan plan = padded_plan(base, fp64, 2, kMax);
+    const FftPlan plan = padded_plan(base, fp64, 2, kSmemMax);
     size_t smem = 2 * (size_t)plan.stride() * sizeof(cx<R>);
-    cudaError_t e = cudaFuncSetAttribute(k_fft_strided<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e =
+        cudaFuncSetAttribute(k_fft_strided<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
     if (e != cudaSuccess) return e;
     k_fft_strided<R><<<nsig_a * nsig_b, 256, smem, s>>>(
         reinterpret_cast<cx<R>*>(data), plan, reinterpret_cast<const cx<R>*>(tw),

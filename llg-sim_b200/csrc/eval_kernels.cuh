@@ -47,7 +47,6 @@ bool dispatch_LV(int L, int V, F&& f) {
     return done;
 }
 
-constexpr size_t kSmemMax = 227 * 1024;
 constexpr size_t kStaticSmemCol = 64;   // mbarriers and the timeout flag of k_column_fast
 
 // Intermediate RK stages need only the torque: no reductions, error norm or
@@ -107,24 +106,26 @@ cudaError_t build_pass_tables(void* out, int L_, int v, cudaStream_t s) {
     return err;
 }
 
+// Opts a kernel into the largest dynamic shared memory it can have beside its static
+// part; an error where `need` exceeds that.  The limit is state of the process: set to
+// one engine's size it refused the launches of a live engine with longer films.
+static cudaError_t allow_max_smem(const void* kernel, size_t need) {
+    cudaFuncAttributes fa;
+    cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
+    if (e != cudaSuccess) return e;
+    const size_t most = kSmemMax - fa.sharedSizeBytes;
+    if (need > most) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 template <typename R>
 cudaError_t prepare_eval_kernels(size_t smem_row, size_t smem_col) {
-    cudaError_t e;
-    e = cudaFuncSetAttribute(k_row_forward<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_row_inverse<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_row_inverse<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_row_fused_generic<R, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row);
-    if (e != cudaSuccess) return e;
-    if (sizeof(R) == 4) {
-        e = cudaFuncSetAttribute(k_row_fused_generic<R, sizeof(R) == 4 ? 512 : 256>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row);
-        if (e != cudaSuccess) return e;
-    }
-    e = cudaFuncSetAttribute(k_column<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_col);
-    if (e != cudaSuccess) return e;
+    constexpr int NT = sizeof(R) == 4 ? 512 : 256;
+    for (const void* f : {(const void*)k_row_forward<R>, (const void*)k_row_inverse<R, false>,
+                          (const void*)k_row_inverse<R, true>, (const void*)k_row_fused_generic<R, 256>,
+                          (const void*)k_row_fused_generic<R, NT>})
+        if (cudaError_t e = allow_max_smem(f, smem_row)) return e;
+    if (cudaError_t e = allow_max_smem((const void*)k_column<R>, smem_col)) return e;
     // fast kernels: every instantiation whose shared memory fits; the whole unified
     // L1/shared array as shared memory, so that occupancy is bounded by registers
     // and the blocks' own shared memory only
