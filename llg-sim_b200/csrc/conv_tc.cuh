@@ -201,11 +201,11 @@ __global__ void __launch_bounds__(kTile) k_conv3x3_tc(const __nv_bfloat16* __res
                      kk > 0 ? 1u : 0u);
         mma_commit(&bar);
     }
-    const bool done = mbar_wait_n(&bar, 0, spin);
+    const bool done = __all_sync(0xffffffffu, mbar_wait_n(&bar, 0, spin));   // uniform over the warp (tmem_ld)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (!done) {
-        if (t == 0) atomicExch(err, 1);
-        mbar_wait(&bar, 0);   // one more bounded wait for the MMAs before the TMEM is freed
+        atomicExch(err, 1);    // any warp that gave up reports: its cells are not written
+        mbar_wait(&bar, 0);    // one more bounded wait for the MMAs before the TMEM is freed
     } else {
         float acc[NCOL];
         tmem_ld<NCOL>(tmem + ((uint32_t)(warp * 32) << 16), acc);
@@ -381,9 +381,14 @@ __global__ void __launch_bounds__(kPipeThreads) k_conv3x3_pipe(const __nv_bfloat
         mbar_arrive_expect_tx(&bar_halo[buf], bytes);
         bulk_copy_g2s(Hs + (size_t)buf * kHaloCells * CIN * 2, x + lo * CIN, bytes, &bar_halo[buf]);
     };
-    // Outstanding asynchronous work, tracked identically by every thread (the tile
-    // sequence is fixed): the phase parity of the last copy issued into each halo
-    // buffer that has not been waited for (-1: none), and of the last MMA commit.
+    // Outstanding asynchronous work as a thread knows it: the phase parity of the last
+    // MMA commit (-1: seen complete) and of the last copy into each halo buffer; the
+    // issuing threads (t = 0 the MMAs, t = kTile the copies) drain what is left at the end.
+    // The waits are bounded per thread, and the warps reach them at different times
+    // (builders are not held up by an epilogue), so one thread may give up on what
+    // another one sees complete.  A thread that gives up (ok = false) reports it, and from
+    // then on only takes part in the barriers: it waits, builds, issues and stores nothing,
+    // but never leaves the loop early, so that every barrier is reached by all threads.
     int halo_pending[2] = {-1, -1};
     int mma_pending = -1;
     long long tile = blockIdx.x;
@@ -400,18 +405,18 @@ __global__ void __launch_bounds__(kPipeThreads) k_conv3x3_pipe(const __nv_bfloat
     long long prev = -1;
     for (; tile < ntiles; tile += gridDim.x, ++k) {
         const int hb = k & 1;
-        ok = mbar_wait_n(&bar_halo[hb], (uint32_t)((k >> 1) & 1), spin);
-        if (!ok) break;
-        halo_pending[hb] = -1;
-        if (mma_pending >= 0) {   // the MMAs of the previous tile have read the im2col buffer
+        if (ok) {
+            ok = mbar_wait_n(&bar_halo[hb], (uint32_t)((k >> 1) & 1), spin);
+            if (ok) halo_pending[hb] = -1;
+        }
+        if (ok && mma_pending >= 0) {   // the MMAs of the previous tile have read the im2col buffer
             ok = mbar_wait_n(&bar_mma, (uint32_t)mma_pending, spin);
-            if (!ok) break;
-            mma_pending = -1;
+            if (ok) mma_pending = -1;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
         // the other halo buffer was read by the previous tile's im2col build (before
         // the previous barrier): refill it with the next tile's range
-        if (tile + gridDim.x < ntiles) {
+        if (ok && tile + gridDim.x < ntiles) {
             if (t == kTile) {
                 fence_async_smem();
                 issue_halo(tile + gridDim.x, hb ^ 1);
@@ -421,7 +426,7 @@ __global__ void __launch_bounds__(kPipeThreads) k_conv3x3_pipe(const __nv_bfloat
         // im2col row of cell p from the halo (zero outside the image): threads 128 + i and
         // 256 + i share cell i, 4 taps and 5 taps.  Lanes start at different 8-channel groups, so the eight lanes of a 16-byte
         // access phase, whose cells are CIN * 2 bytes apart, cover all banks.
-        if (t >= kTile) {
+        if (ok && t >= kTile) {
             long long lo, cnt;
             halo_range(tile, &lo, &cnt);
             const unsigned char* hsrc = Hs + (size_t)hb * kHaloCells * CIN * 2;
@@ -453,16 +458,17 @@ __global__ void __launch_bounds__(kPipeThreads) k_conv3x3_pipe(const __nv_bfloat
         __syncthreads();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc_col = (uint32_t)hb * kAcc;
-        if (t == 0) {
+        if (ok && t == 0) {
             const uint32_t a0 = smem_addr(As), b0 = smem_addr(Bs);
             for (int kk = 0; kk < K / 16; ++kk)
                 mma_bf16(tmem + acc_col, smem_desc(a0 + kk * 256, 128, sbo), smem_desc(b0 + kk * 256, 128, sbo), idesc,
                          kk > 0 ? 1u : 0u);
             mma_commit(&bar_mma);
         }
-        mma_pending = k & 1;
-        // epilogue of the previous tile while the tensor cores work on this one
-        if (prev >= 0 && t < kTile) {
+        if (ok) mma_pending = k & 1;
+        // epilogue of the previous tile while the tensor cores work on this one (tmem_ld:
+        // whole warps only)
+        if (prev >= 0 && t < kTile && __all_sync(0xffffffffu, ok)) {
             float acc[NCOL];
             tmem_ld<NCOL>(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(hb ^ 1) * kAcc, acc);
             const long long p = prev * kTile + t;
@@ -474,20 +480,21 @@ __global__ void __launch_bounds__(kPipeThreads) k_conv3x3_pipe(const __nv_bfloat
         ok = mbar_wait_n(&bar_mma, (uint32_t)mma_pending, spin);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (ok) mma_pending = -1;
-        if (ok && t < kTile) {
-            float acc[NCOL];
-            tmem_ld<NCOL>(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((k - 1) & 1) * kAcc, acc);
-            const long long p = prev * kTile + t;
-            if (p < total) conv_epilogue<NCOL, EPI, R>(acc, p, hw, L, y, m_out, out32, mask, act);
-        }
+    }
+    if (prev >= 0 && t < kTile && __all_sync(0xffffffffu, ok)) {
+        float acc[NCOL];
+        tmem_ld<NCOL>(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((k - 1) & 1) * kAcc, acc);
+        const long long p = prev * kTile + t;
+        if (p < total) conv_epilogue<NCOL, EPI, R>(acc, p, hw, L, y, m_out, out32, mask, act);
     }
     if (!ok) {
-        if (t == 0) atomicExch(err, 1);
-        // one more bounded wait for the copies and MMAs still in flight, so that none
-        // writes shared memory or TMEM after the CTA has released them
-        if (mma_pending >= 0) mbar_wait(&bar_mma, (uint32_t)mma_pending);
+        atomicExch(err, 1);
+        // one more bounded wait for the copies and MMAs still in flight, by the threads
+        // that issued them, so that none writes shared memory or TMEM after the CTA has
+        // released them
+        if (t == 0 && mma_pending >= 0) mbar_wait(&bar_mma, (uint32_t)mma_pending);
         for (int b = 0; b < 2; ++b)
-            if (halo_pending[b] >= 0) mbar_wait(&bar_halo[b], (uint32_t)halo_pending[b]);
+            if (t == kTile && halo_pending[b] >= 0) mbar_wait(&bar_halo[b], (uint32_t)halo_pending[b]);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

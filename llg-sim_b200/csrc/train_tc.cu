@@ -112,26 +112,32 @@ __global__ void __launch_bounds__(128, 4) k_wgrad_tc(const __nv_bfloat16* __rest
         }
     };
     if (c_begin < c_end) load(c_begin);
+    // The waits are bounded per thread: one that gives up (ok = false) reports it, and from
+    // then on only takes part in the barriers (no writes, no MMAs), so that every barrier
+    // is reached by all threads and no MMA result is stored without all of its operands.
     for (long long c0 = c_begin; c0 < c_end; c0 += kWgKC) {
+        if (ok) {
 #pragma unroll
-        for (int b = 0; b < VA; ++b) {
-            unsigned char* ak = As + ((ka >> 3) + b) * A_LBO + (ka & 7) * 16 + cg * 128;
+            for (int b = 0; b < VA; ++b) {
+                unsigned char* ak = As + ((ka >> 3) + b) * A_LBO + (ka & 7) * 16 + cg * 128;
 #pragma unroll
-            for (int tap = 0; tap < 9; ++tap) {
-                const int m = tap * CIN;
-                *reinterpret_cast<uint4*>(ak + (m / kTile) * A_TILE + ((m % kTile) >> 3) * 128) = va[tap * VA + b];
+                for (int tap = 0; tap < 9; ++tap) {
+                    const int m = tap * CIN;
+                    *reinterpret_cast<uint4*>(ak + (m / kTile) * A_TILE + ((m % kTile) >> 3) * 128) =
+                        va[tap * VA + b];
+                }
             }
-        }
 #pragma unroll
-        for (int r = 0; r < VB; ++r) {
-            const int e = t + r * 128, kb = e / (NN / 8), ng = e - kb * (NN / 8);
-            *reinterpret_cast<uint4*>(Bs + (kb >> 3) * B_LBO + ng * 128 + (kb & 7) * 16) = vb[r];
+            for (int r = 0; r < VB; ++r) {
+                const int e = t + r * 128, kb = e / (NN / 8), ng = e - kb * (NN / 8);
+                *reinterpret_cast<uint4*>(Bs + (kb >> 3) * B_LBO + ng * 128 + (kb & 7) * 16) = vb[r];
+            }
         }
         fence_async_smem();
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncthreads();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (t == 0) {
+        if (ok && t == 0) {
             const uint32_t a0 = smem_addr(As), b0 = smem_addr(Bs);
             for (int tile = 0; tile < NT; ++tile)
                 for (int kk = 0; kk < kWgKC / 16; ++kk) {
@@ -144,14 +150,19 @@ __global__ void __launch_bounds__(128, 4) k_wgrad_tc(const __nv_bfloat16* __rest
         first = false;
         if (c0 + kWgKC < c_end) load(c0 + kWgKC);
         // the chunk buffers are rewritten only after these MMAs have read them
-        ok = mbar_wait_n(&bar, phase, spin);
-        phase ^= 1u;
+        if (ok) {
+            ok = mbar_wait_n(&bar, phase, spin);
+            phase ^= 1u;
+        }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (!ok) break;
     }
     if (!ok) {
-        if (t == 0) atomicExch(err, 1);
-        mbar_wait(&bar, phase ^ 1u);   // one more bounded wait for the MMAs before the TMEM is freed
+        atomicExch(err, 1);
+        // one more bounded wait for the MMAs before the TMEM is freed
+        if (t == 0) mbar_wait(&bar, phase ^ 1u);
+    }
+    if (!__all_sync(0xffffffffu, ok)) {
+        // nothing to store: the call reports the timeout
     } else if (!first) {
         for (int tile = 0; tile < NT; ++tile) {
             float acc[NN];
