@@ -141,6 +141,7 @@ cudaError_t prepare_eval_kernels(size_t smem_row, size_t smem_col) {
             both((const void*)k_row_inverse_fast<R, L, 0, V>, sm);
             both((const void*)k_row_inverse_fast<R, L, 1, V>, sm);
             both((const void*)k_row_inverse_fast<R, L, 2, V>, sm);
+            if constexpr (inverse_xt_ok<R, L, V>()) both((const void*)k_row_inverse_fast<R, L, 2, V, 2>, sm);
             both((const void*)k_row_fused<R, L, V, 1>, sm);
             if constexpr (fused_xt_ok<R, L, V>()) both((const void*)k_row_fused<R, L, V, 2>, sm);
         }
@@ -182,7 +183,13 @@ cudaError_t launch_one(int which, const EvalSpec& spec, const LaunchGeom& g, cud
                         torque<<<grid, 256, 0, s>>>(g.films, g.row_items, g.n_row_items, LOG_L, LOG_T, spec);
                         ++count;
                     } else if (spec.rhs == RHS_MINIMIZE) {
-                        row(k_row_inverse_fast<R, L, 2, V>, g.grid_rfull, C::THREADS * inverse_xt<R, L, 2, V>(), C::SMEM);
+                        if constexpr (inverse_xt_ok<R, L, V>()) {
+                            if (g.n_row_items <= g.nsm) {   // one block per SM at most
+                                row(k_row_inverse_fast<R, L, 2, V, 2>, g.n_row_items, 2 * C::THREADS, C::SMEM);
+                                return;
+                            }
+                        }
+                        row(k_row_inverse_fast<R, L, 2, V>, g.grid_rfull, C::THREADS, C::SMEM);
                     } else {
                         row(k_row_inverse_fast<R, L, 0, V>, g.grid_rfull, C::THREADS, C::SMEM);
                     }

@@ -523,20 +523,23 @@ __global__ void __launch_bounds__(ColCfg<R, L, V, LEAN>::THREADS) __maxnreg__((C
 // ---------------------------------------------------------------------------
 // MODE 0: full epilogue; 1: no epilogue, the demag field is written to the film's
 // bdem planes for k_stage_torque; 2: the minimiser epilogue (RHS_MINIMIZE).
-// The minimiser's FP64 cell update is a long dependent chain, and the films up to 256
-// cells wide have fewer row blocks than the SMs can hold: there the block has as many
-// threads again (XT = 2), which take no part in the transforms but halve the cells per
-// thread of the epilogue.
-template <typename R, int L, int MODE, int V>
-__host__ __device__ constexpr int inverse_xt() {
-    return MODE == 2 && sizeof(R) == 4 && V == 0 && L <= 256 && RowCfg<R, L, V>::THREADS <= 192 ? 2 : 1;
+// The minimiser's FP64 cell update is a long dependent chain: in launches with at most
+// one block per SM (inverse_xt_ok, chosen by the launch as for k_row_fused) the block has
+// as many threads again (XT = 2), which take no part in the transforms but halve the cells
+// per thread of the epilogue (an iteration of one 256 x 256 film, 64 blocks: 36 us, with
+// the one-fold form 44 before this form).  With more blocks than SMs two blocks of the
+// one-fold form share an SM, which keeps its threads busy in the transforms too: 16 such
+// films 144 us per iteration, with the two-fold form 225; 64 films of 64 x 64 55 and 77.
+template <typename R, int L, int V>
+__host__ __device__ constexpr bool inverse_xt_ok() {
+    return sizeof(R) == 4 && V == 0 && L <= 256 && RowCfg<R, L, V>::THREADS <= 192;
 }
-template <typename R, int L, int MODE, int V>
-__global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS * inverse_xt<R, L, MODE, V>()) __maxnreg__((MODE == 1 ? RowCfg<R, L, V>::MAXREG : RowCfg<R, L, V>::REG2)) k_row_inverse_fast(const FilmDev* __restrict__ films,
+template <typename R, int L, int MODE, int V, int XT = 1>
+__global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS * XT) __maxnreg__((MODE == 1 ? RowCfg<R, L, V>::MAXREG : RowCfg<R, L, V>::REG2)) k_row_inverse_fast(const FilmDev* __restrict__ films,
                                                                             const WorkItem* __restrict__ items,
                                                                             int nitems, EvalSpec spec) {
     using C = RowCfg<R, L, V>;
-    constexpr int NT = C::THREADS * inverse_xt<R, L, MODE, V>();
+    constexpr int NT = C::THREADS * XT;
     using FI = GroupFFT<R, L, true, V>;
     constexpr int G = C::G, E = C::E, T = C::T, BUF = C::BUF;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -564,7 +567,6 @@ __global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS * inverse_xt<R, L, MO
             const cx<R>* __restrict__ X = reinterpret_cast<const cx<R>*>(F.X);
             row_stage_spectrum<R, L, V, NT>(X, buf, ny, j0);
             __syncthreads();
-            constexpr int XT = NT / C::THREADS;
             if (XT == 1 || tid < C::THREADS) {   // threads of the transforms
                 cx<R> v[E];
                 row_load_inverse<R, L, V>(buf, v, t, g, par);
