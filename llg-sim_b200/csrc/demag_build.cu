@@ -259,9 +259,13 @@ template __global__ void k_twiddles<double>(cx<double>*, int);
 
 template <typename R>
 __global__ void k_pass_tables_smem(FftPlan plan, cx<R>* out) {
-    double s, c;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; pass_table_entry(plan, e, &c, &s); e += gridDim.x * blockDim.x)
-        out[e] = mkc((R)c, (R)s);
+    int num, den;
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; pass_table_entry(plan, e, &num, &den);
+         e += gridDim.x * blockDim.x) {
+        double s, c;
+        sincospi(2.0 * (double)num / (double)den, &s, &c);
+        out[e] = mkc((R)c, (R)-s);
+    }
 }
 
 static constexpr int kRadices[] = {16, 12, 10, 8, 6, 5, 4, 3, 2};   // radices with a register butterfly

@@ -357,16 +357,17 @@ __device__ cx<R>* fft_smem(cx<R>* a, cx<R>* b, int nsig, const FftPlan& plan, co
 
 // Pass tables of a plan: for every pass s >= 1 (radix p, stride ns = product of the
 // earlier radices) W_{ns p}^{k r} at [r * ns + k], r < p, k < ns, pass after pass.
-// Fewer than 2L entries.  Entry e; false past the end.
-__device__ __forceinline__ bool pass_table_entry(const FftPlan& plan, int e, double* c, double* s) {
+// Fewer than 2L entries.  Entry e is exp(-2 pi i num / den); false past the end.
+__device__ __forceinline__ bool pass_table_entry(const FftPlan& plan, int e, int* num, int* den) {
     if (plan.npass == 0) return false;
     int ns = plan.radix[0];
+#pragma unroll 1
     for (int q = 1; q < plan.npass; ++q) {
         const int p = plan.radix[q], n = p * ns;
         if (e < n) {
-            const long long r = e / ns, k = e % ns;
-            sincospi(2.0 * (double)((k * r) % n) / (double)n, s, c);
-            *s = -*s;
+            const int r = e / ns;
+            *num = (e - r * ns) * r;   // k r < n
+            *den = n;
             return true;
         }
         e -= n;

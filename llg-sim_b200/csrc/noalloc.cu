@@ -37,23 +37,31 @@ static __device__ __align__(256) cx<float> g_pass_tables[4 * kMaxLen];
 std::mutex g_setup_mutex;
 void* g_scratch_addr[kMaxDevices] = {nullptr};
 void* g_tables_addr[kMaxDevices] = {nullptr};
+int g_sm_count[kMaxDevices] = {0};
 
 inline size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
-// exp(-2 pi i k / (2L)) of both lengths and the pass tables of both plans.
-__global__ void k_na_twiddles(cx<float>* tw_row, int nx, cx<float>* tw_col, int ny, FftPlan prow, FftPlan pcol,
-                              cx<float>* pass_row, cx<float>* pass_col) {
+// exp(-2 pi i k / (2L)) of both lengths and the pass tables of both plans.  One sincospi,
+// one plan index and a rolled loop over the passes keep the code short: its fetch is most
+// of the kernel's 2 to 3 us.
+struct Plans {
+    FftPlan p[2];   // rows, columns
+};
+__global__ void k_na_twiddles(cx<float>* tw_row, int nx, cx<float>* tw_col, int ny,
+                              const __grid_constant__ Plans plans, cx<float>* pass_row, cx<float>* pass_col) {
     const int total = 2 * nx + 2 * ny;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
+    // entries [0, total): twiddles, [total, 2 total): pass tables (one sincospi per thread)
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < 2 * total; q += gridDim.x * blockDim.x) {
+        const bool tables = q >= total;
+        const int e = tables ? q - total : q;
         const bool row = e < 2 * nx;
-        double pc, ps;
-        if (pass_table_entry(row ? prow : pcol, row ? e : e - 2 * nx, &pc, &ps))
-            (row ? pass_row : pass_col)[row ? e : e - 2 * nx] = mkc((float)pc, (float)ps);
         const int k = row ? e : e - 2 * nx;
-        const int L2 = row ? 2 * nx : 2 * ny;
+        int num = k, den = row ? 2 * nx : 2 * ny;
+        if (tables && !pass_table_entry(plans.p[row ? 0 : 1], k, &num, &den)) continue;
         double s, c;
-        sincospi(2.0 * (double)k / (double)L2, &s, &c);
-        (row ? tw_row : tw_col)[k] = mkc((float)c, (float)(-s));
+        sincospi(2.0 * (double)num / (double)den, &s, &c);
+        cx<float>* out = tables ? (row ? pass_row : pass_col) : (row ? tw_row : tw_col);
+        out[k] = mkc((float)c, (float)-s);
     }
 }
 
@@ -101,36 +109,34 @@ __global__ void __launch_bounds__(kThreads) k_na_rows_forward(int nx, int ny, fl
     }
 }
 
-// NC adjacent kx columns: pruned y transform, kernel multiply, pruned inverse.
-// kp: FP64 kernel planes [4][ny+1][nx+1] (xx, xy, yy, zz), unscaled.  The planes run
-// along kx, so a block of one column reads 8 of every 32-byte sector; with NC = 4
-// columns a block reads whole sectors (columns_per_block: as many as leave two
-// blocks per SM).
-__global__ void __launch_bounds__(kThreads) k_na_column(int nx, int ny, int nc, const double* __restrict__ kp,
-                                                        double scale, cx<float>* __restrict__ X,
-                                                        const cx<float>* __restrict__ twp,
+// One kx column: pruned y transform, kernel multiply, pruned inverse.
+// kp: FP64 kernel planes [4][ny+1][nx+1] (xx, xy, yy, zz), unscaled.  A block reads 8 of
+// every 32-byte sector of the planes (the L2 holds them for its neighbours): blocks of up
+// to four columns, which read whole sectors, left SMs without a block on films up to 256
+// cells wide and registers for one block per SM on wide ones (column pass at 64 x 256
+// 20.5 us against 13, whole call at 1000 x 500 126 against 117).
+__global__ void __launch_bounds__(kThreads) k_na_column(int nx, int ny, const double* __restrict__ kp, double scale,
+                                                        cx<float>* __restrict__ X, const cx<float>* __restrict__ twp,
                                                         const cx<float>* __restrict__ tw, FftPlan plan) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int L = ny, K1 = nx + 1, kx0 = blockIdx.x * nc, LP = plan.stride();
-    const int nv = min(nc, K1 - kx0);   // columns of this block
+    const int L = ny, K1 = nx + 1, kx = blockIdx.x, LP = plan.stride();
     const size_t plane = (size_t)(ny + 1) * (nx + 1);
     cx<float>* A = reinterpret_cast<cx<float>*>(smem_raw);
-    cx<float>* B = A + 6 * nc * LP;
-    // signals: column q, component c, parity p at 6 q + 2 c + p
-    for (int e = threadIdx.x; e < 3 * nv * L; e += blockDim.x) {
-        const int cq = e / L, y = e - cq * L, c = cq / nv, q = cq - c * nv;
-        const cx<float> x = X[((size_t)c * K1 + kx0 + q) * ny + y];
-        cx<float>* s = A + (6 * q + 2 * c) * LP + plan.at(y);
+    cx<float>* B = A + 6 * LP;
+    // signals: component c, parity p at 2 c + p
+    for (int e = threadIdx.x; e < 3 * L; e += blockDim.x) {
+        const int c = e / L, y = e - c * L;
+        const cx<float> x = X[((size_t)c * K1 + kx) * ny + y];
+        cx<float>* s = A + 2 * c * LP + plan.at(y);
         s[0] = x;
         s[LP] = cmul(x, tw[y]);
     }
     __syncthreads();
-    cx<float>* res = fft_smem<float, false>(A, B, 6 * nv, plan, twp, tw);
-    // one kernel entry serves both ky and 2 ny - ky (Kxy odd); consecutive threads
-    // take the columns of one ky
-    for (int e = threadIdx.x; e < nv * (ny + 1); e += blockDim.x) {
-        const int kyf = e / nv, q = e - kyf * nv, par = kyf & 1;
-        const size_t o = (size_t)kyf * (nx + 1) + kx0 + q;
+    cx<float>* res = fft_smem<float, false>(A, B, 6, plan, twp, tw);
+    // one kernel entry serves both ky and 2 ny - ky (Kxy odd)
+    for (int kyf = threadIdx.x; kyf <= ny; kyf += blockDim.x) {
+        const int par = kyf & 1;
+        const size_t o = (size_t)kyf * (nx + 1) + kx;
         const float kxx = (float)(kp[o] * scale), kyy = (float)(kp[2 * plane + o] * scale);
         const float kzz = (float)(kp[3 * plane + o] * scale);
         const float kxyf = (float)(kp[plane + o] * scale);
@@ -138,7 +144,7 @@ __global__ void __launch_bounds__(kThreads) k_na_column(int nx, int ny, int nc, 
             const int ky = h ? 2 * ny - kyf : kyf;
             if (h && (kyf == 0 || kyf == ny)) break;
             const float kxy = kxyf * (h ? -1.f : 1.f);
-            cx<float>* s = res + (6 * q + par) * LP + plan.at(ky >> 1);
+            cx<float>* s = res + par * LP + plan.at(ky >> 1);
             const cx<float> Mx = s[0], My = s[2 * LP], Mz = s[4 * LP];
             s[0] = mkc(kxx * Mx.re + kxy * My.re, kxx * Mx.im + kxy * My.im);
             s[2 * LP] = mkc(kxy * Mx.re + kyy * My.re, kxy * Mx.im + kyy * My.im);
@@ -147,18 +153,22 @@ __global__ void __launch_bounds__(kThreads) k_na_column(int nx, int ny, int nc, 
     }
     __syncthreads();
     cx<float>* other = res == A ? B : A;
-    cx<float>* res2 = fft_smem<float, true>(res, other, 6 * nv, plan, twp, tw);
-    for (int e = threadIdx.x; e < 3 * nv * L; e += blockDim.x) {
-        const int cq = e / L, y = e - cq * L, c = cq / nv, q = cq - c * nv;
-        const cx<float>* s = res2 + (6 * q + 2 * c) * LP + plan.at(y);
-        X[((size_t)c * K1 + kx0 + q) * ny + y] = s[0] + cmulc(s[LP], tw[y]);
+    cx<float>* res2 = fft_smem<float, true>(res, other, 6, plan, twp, tw);
+    for (int e = threadIdx.x; e < 3 * L; e += blockDim.x) {
+        const int c = e / L, y = e - c * L;
+        const cx<float>* s = res2 + 2 * c * LP + plan.at(y);
+        X[((size_t)c * K1 + kx) * ny + y] = s[0] + cmulc(s[LP], tw[y]);
     }
 }
 
-int columns_per_block(const FftPlan& plan) {
-    int nc = 1;
-    while (nc < 4 && 12 * (size_t)(2 * nc) * plan.stride() * sizeof(cx<float>) <= 110 * 1024) nc *= 2;
-    return nc;
+// Most threads of a launch's blocks, transforms of length L.  Up to 64 cells 128 threads
+// cover a pass in one round (1024 x 64: 52 us, 55 with 256).  Beyond, with at most one block
+// per SM latency is all that counts: 512.  With more, registers (64 to 80 a thread) decide how many of the blocks that
+// fit the shared memory are resident: 384 threads where a block's buffers exceed `wide`
+// bytes, 256 otherwise (whole calls with rows of 512, 384 and 256 threads: 1000 x 400
+// 110, 105, 107, 500 x 500 68, 65, 72; with columns: 1000 x 1000 247, 244, 254, 800 x 640 127, 125, 118 us).
+int most_threads(int L, int blocks, int nsm, size_t smem, size_t wide) {
+    return L <= 64 ? 128 : blocks <= nsm ? kThreads : smem > wide ? 384 : 256;
 }
 
 // Rows: C2R along x keeping nx cells, B_demag to b (SoA FP32).
@@ -240,6 +250,9 @@ int setup(int dev, void** out, void** tables) {
         cudaFuncSetAttribute(k_na_rows_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, smax) != cudaSuccess ||
         cudaFuncSetAttribute(k_na_column, cudaFuncAttributeMaxDynamicSharedMemorySize, smax) != cudaSuccess)
         return LLG_ERR_CUDA;
+    int nsm = 148;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    g_sm_count[dev] = nsm;
     g_scratch_addr[dev] = ptr;
     g_tables_addr[dev] = tab;
     *out = ptr;
@@ -284,18 +297,17 @@ extern "C" int llg_demag_field_noalloc(int64_t nx, int64_t ny, double ms, const 
     const FftPlan pcol = padded_plan(make_plan(iny), false, 12, 227 * 1024);
     cx<float>* pass_row = static_cast<cx<float>*>(tables);
     cx<float>* pass_col = pass_row + 2 * kMaxLen;
-    const int nc = columns_per_block(pcol);
     const size_t smem_row = 4 * (size_t)G * prow.stride() * sizeof(cx<float>);
-    const size_t smem_col = 12 * (size_t)nc * pcol.stride() * sizeof(cx<float>);
+    const size_t smem_col = 12 * (size_t)pcol.stride() * sizeof(cx<float>);
     const int row_blocks = (iny + kT - 1) / kT;
-    const int row_threads = fft_block_threads(prow, 2 * G, 6 * kT, kThreads);
-    const int col_threads = fft_block_threads(pcol, 6 * nc, 8 * nc, kThreads);
-    k_na_twiddles<<<(2 * inx + 2 * iny + 255) / 256, 256, 0, s>>>(tw_row, inx, tw_col, iny, prow, pcol, pass_row,
-                                                                 pass_col);
+    const int nsm = g_sm_count[dev];
+    const int row_threads = fft_block_threads(prow, 2 * G, 6 * kT, most_threads(inx, row_blocks, nsm, smem_row, 45 * 1024));
+    const int col_threads = fft_block_threads(pcol, 6, 8, most_threads(iny, inx + 1, nsm, smem_col, 75 * 1024));
+    k_na_twiddles<<<(4 * inx + 4 * iny + 255) / 256, 256, 0, s>>>(tw_row, inx, tw_col, iny, Plans{{prow, pcol}},
+                                                                 pass_row, pass_col);
     k_na_rows_forward<<<row_blocks, row_threads, smem_row, s>>>(inx, iny, (float)ms, m, X, pass_row, tw_row, prow);
-    k_na_column<<<(inx + nc) / nc, col_threads, smem_col, s>>>(inx, iny, nc, kernel_planes,
-                                                            1.0 / (4.0 * (double)nx * (double)ny), X, pass_col, tw_col,
-                                                            pcol);
+    k_na_column<<<inx + 1, col_threads, smem_col, s>>>(inx, iny, kernel_planes, 1.0 / (4.0 * (double)nx * (double)ny),
+                                                       X, pass_col, tw_col, pcol);
     k_na_rows_inverse<<<row_blocks, row_threads, smem_row, s>>>(inx, iny, X, pass_row, tw_row, prow, b_out);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
