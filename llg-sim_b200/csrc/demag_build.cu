@@ -213,44 +213,30 @@ __global__ void k_twiddles(cx<R>* tw, int L2) {
     }
 }
 
+// In-place transforms of ns signals per block (fewer in the last block of a row of tiles).
+// rows: a signal is contiguous and threads run along it; else the signals are adjacent
+// columns and threads run along them, so that each row of a tile is ns contiguous elements
+// (whole 32-byte sectors in FP64 instead of half ones).
 template <typename R>
 __global__ void __launch_bounds__(256) k_fft_strided(cx<R>* data, FftPlan plan, const cx<R>* tw, const cx<R>* tw2,
                                                      long long elem_stride, int nsig_a, long long stride_a,
-                                                     long long stride_b, int inverse) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    cx<R>* A = reinterpret_cast<cx<R>*>(smem_raw);
-    cx<R>* B = A + plan.stride();
-    const int sig = blockIdx.x;
-    const long long base = (long long)(sig % nsig_a) * stride_a + (long long)(sig / nsig_a) * stride_b;
-    for (int t = threadIdx.x; t < plan.L; t += blockDim.x) A[plan.at(t)] = data[base + t * elem_stride];
-    __syncthreads();
-    cx<R>* res = inverse ? fft_smem<R, true>(A, B, 1, plan, tw, tw2) : fft_smem<R, false>(A, B, 1, plan, tw, tw2);
-    for (int t = threadIdx.x; t < plan.L; t += blockDim.x) data[base + t * elem_stride] = res[plan.at(t)];
-}
-
-// Column transforms of adjacent signals (stride between signals 1 element): a block
-// takes NS neighbouring columns, so that one row of the tile is NS consecutive
-// elements in memory (whole 32-byte sectors in FP64 instead of half ones); each
-// signal's arithmetic is the one of k_fft_strided.
-template <typename R>
-__global__ void __launch_bounds__(256) k_fft_strided_tiled(cx<R>* data, FftPlan plan, const cx<R>* tw,
-                                                           const cx<R>* tw2, long long elem_stride, int nsig_a,
-                                                           long long stride_b, int ns, int inverse) {
+                                                     long long stride_b, int ns, int rows, int inverse) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int L = plan.L, LP = plan.stride();
     cx<R>* A = reinterpret_cast<cx<R>*>(smem_raw);
     cx<R>* B = A + (size_t)ns * LP;
-    const int tiles_a = nsig_a / ns;
-    const long long base = (long long)(blockIdx.x % tiles_a) * ns + (long long)(blockIdx.x / tiles_a) * stride_b;
-    for (int e = threadIdx.x; e < ns * L; e += blockDim.x) {
-        const int c = e % ns, t = e / ns;
-        A[(size_t)c * LP + plan.at(t)] = data[base + c + t * elem_stride];
+    const int tiles_a = (nsig_a + ns - 1) / ns;
+    const int a0 = (int)(blockIdx.x % tiles_a) * ns, nv = min(ns, nsig_a - a0);
+    cx<R>* d = data + a0 * stride_a + (long long)(blockIdx.x / tiles_a) * stride_b;
+    for (int e = threadIdx.x; e < nv * L; e += blockDim.x) {
+        const int t = rows ? e % L : e / nv, c = rows ? e / L : e % nv;
+        A[(size_t)c * LP + plan.at(t)] = d[c * stride_a + t * elem_stride];
     }
     __syncthreads();
-    cx<R>* res = inverse ? fft_smem<R, true>(A, B, ns, plan, tw, tw2) : fft_smem<R, false>(A, B, ns, plan, tw, tw2);
-    for (int e = threadIdx.x; e < ns * L; e += blockDim.x) {
-        const int c = e % ns, t = e / ns;
-        data[base + c + t * elem_stride] = res[(size_t)c * LP + plan.at(t)];
+    cx<R>* res = inverse ? fft_smem<R, true>(A, B, nv, plan, tw, tw2) : fft_smem<R, false>(A, B, nv, plan, tw, tw2);
+    for (int e = threadIdx.x; e < nv * L; e += blockDim.x) {
+        const int t = rows ? e % L : e / nv, c = rows ? e / L : e % nv;
+        d[c * stride_a + t * elem_stride] = res[(size_t)c * LP + plan.at(t)];
     }
 }
 
@@ -414,33 +400,31 @@ template <typename R>
 cudaError_t launch_fft_strided(void* data, const FftPlan& base, const void* tw, const void* tw2, long long elem_stride, int nsig_a,
                                long long stride_a, int nsig_b, long long stride_b, bool inverse, cudaStream_t s) {
     constexpr bool fp64 = sizeof(R) == 8;
-    const int L = base.L;
-    // (the kernels' shared-memory limits are state of the process: always the largest, so
-    // that a thread with shorter signals does not lower them for another one)
-    if (elem_stride > 1 && stride_a == 1) {
-        // adjacent columns: tile NS of them per block where shared memory allows
-        int ns = 1;
-        while (ns < 8 && nsig_a % (2 * ns) == 0 && 2 * (size_t)(2 * ns) * L * sizeof(cx<R>) <= 200 * 1024) ns *= 2;
-        if (ns > 1) {
-            const FftPlan plan = padded_plan(base, fp64, 2 * ns, kSmemMax);
-            const size_t smem = 2 * (size_t)ns * plan.stride() * sizeof(cx<R>);
-            cudaError_t e = cudaFuncSetAttribute(k_fft_strided_tiled<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)kSmemMax);
-            if (e != cudaSuccess) return e;
-            k_fft_strided_tiled<R><<<(nsig_a / ns) * nsig_b, 256, smem, s>>>(
-                reinterpret_cast<cx<R>*>(data), plan, reinterpret_cast<const cx<R>*>(tw),
-                reinterpret_cast<const cx<R>*>(tw2), elem_stride, nsig_a, stride_b, ns, inverse ? 1 : 0);
-            return cudaGetLastError();
-        }
-    }
-    const FftPlan plan = padded_plan(base, fp64, 2, kSmemMax);
-    size_t smem = 2 * (size_t)plan.stride() * sizeof(cx<R>);
+    const bool rows = elem_stride == 1;
+    int ns = 1;
+    // Signals per block: as many as leave 2.5 blocks per SM and three of them room in the
+    // shared memory of one (128 threads at 122 registers: four fit the registers).  FP64
+    // pass, us, with one signal of 256 threads per block and now: 300 x 300 rows 18.6 and
+    // 8.4, 512 x 512 27.0 and 14.6, columns 20.6 and 8.9, 32.4 and 16.1; a launch of fewer
+    // blocks than SMs keeps 256 threads (rows of 2000 x 40: 11.5, with 128 15.4).
+    int dev = 0, nsm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    auto smem_of = [&](int n) { return 2 * (size_t)n * padded_plan(base, fp64, 2 * n, kSmemMax).stride() * sizeof(cx<R>); };
+    auto blocks_of = [&](int n) { return (nsig_a + n - 1) / n * nsig_b; };
+    while (ns < 8 && smem_of(2 * ns) <= 74 * 1024 && 2 * blocks_of(2 * ns) >= 5 * nsm) ns *= 2;
+
+    const FftPlan plan = padded_plan(base, fp64, 2 * ns, kSmemMax);
+    const int blocks = blocks_of(ns);
+    // the kernel's shared-memory limit is state of the process: always the largest, so that
+    // a thread with shorter signals does not lower it for another one
     cudaError_t e =
         cudaFuncSetAttribute(k_fft_strided<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
     if (e != cudaSuccess) return e;
-    k_fft_strided<R><<<nsig_a * nsig_b, 256, smem, s>>>(
+    k_fft_strided<R><<<blocks, blocks > nsm ? 128 : 256, smem_of(ns), s>>>(
         reinterpret_cast<cx<R>*>(data), plan, reinterpret_cast<const cx<R>*>(tw),
-        reinterpret_cast<const cx<R>*>(tw2), elem_stride, nsig_a, stride_a, stride_b, inverse ? 1 : 0);
+        reinterpret_cast<const cx<R>*>(tw2), elem_stride, nsig_a, stride_a, stride_b, ns, rows ? 1 : 0,
+        inverse ? 1 : 0);
     return cudaGetLastError();
 }
 template cudaError_t launch_fft_strided<float>(void*, const FftPlan&, const void*, const void*, long long, int, long long, int,
