@@ -233,7 +233,7 @@ cudaError_t launch_fused(const EvalSpec& si, const EvalSpec& sf, const LaunchGeo
             k_row_fused_generic<R, sizeof(R) == 4 ? 512 : 256><<<g.n_row_items, sizeof(R) == 4 ? 512 : 256, g.smem_row, s>>>(
                 g.films, g.row_items, g.n_row_items, si, sf);
         else
-            k_row_fused_generic<R, 256><<<g.grid_row, 256, g.smem_row, s>>>(g.films, g.row_items, g.n_row_items, si,
+            k_row_fused_generic<R, 256><<<g.grid_fused, 256, g.smem_row, s>>>(g.films, g.row_items, g.n_row_items, si,
                                                                             sf);
     }
     dispatch_LV<R>(g.fast_row, g.row_var, [&](auto LC, auto VC) {

@@ -643,14 +643,21 @@ struct Engine final : EngineBase {
                 CUDA_TRY(launch_twiddles(tw_col, 2 * ny, sizeof(R) == 8, stream));
                 F.tw_row = tw_row;
                 F.tw_col = tw_col;
-                if (!frow[f]) {
-                    if ((rc = dalloc(&F.twg_row, sizeof(cx<R>) * 2 * (size_t)nx))) return rc;
-                    CUDA_TRY(launch_pass_tables(F.plan_row, F.twg_row, sizeof(R) == 8, stream));
-                }
-                if (!fcol[f]) {
-                    if ((rc = dalloc(&F.twg_col, sizeof(cx<R>) * 2 * (size_t)ny))) return rc;
-                    CUDA_TRY(launch_pass_tables(F.plan_col, F.twg_col, sizeof(R) == 8, stream));
-                }
+                // pass tables of the generic transforms: one for all films of a length, which
+                // run the same plan
+                auto generic_tables = [&](const std::vector<char>& fast, int FilmDev::*len, FftPlan FilmDev::*plan,
+                                          void* FilmDev::*tab) -> int {
+                    for (int e = 0; e < f && !(F.*tab); ++e)
+                        if (!fast[e] && fh[e].*len == F.*len) F.*tab = fh[e].*tab;
+                    if (F.*tab) return LLG_OK;
+                    if (int r = dalloc(&(F.*tab), sizeof(cx<R>) * 2 * (size_t)(F.*len))) return r;
+                    CUDA_TRY(launch_pass_tables(F.*plan, F.*tab, sizeof(R) == 8, stream));
+                    return LLG_OK;
+                };
+                if (!frow[f] && (rc = generic_tables(frow, &FilmDev::nx, &FilmDev::plan_row, &FilmDev::twg_row)))
+                    return rc;
+                if (!fcol[f] && (rc = generic_tables(fcol, &FilmDev::ny, &FilmDev::plan_col, &FilmDev::twg_col)))
+                    return rc;
                 // register-FFT pass tables of every radix plan the film's lengths have
                 const FastCfg& fc = fcs[f];
                 for (int v = 0; v < 2; ++v) {
@@ -756,7 +763,7 @@ struct Engine final : EngineBase {
                     s.n_row_items = (int)sp.second.second;
                     s.fast_row = L;
                     s.row_var = v;
-                    int fb = gen_r, ib = gen_r, ub = gen_r, zb = 1, cb = 1;
+                    int fb = gen_r, ib = gen_r, ub = gen_r, zb = gen_r, cb = 1;
                     if (L) fast_occupancy<R>(L, 0, v, 0, &fb, &ib, &ub, &zb, &cb);
                     s.grid_row = balanced(s.n_row_items, fb);
                     s.grid_rinv = balanced(s.n_row_items, ib);
@@ -921,9 +928,11 @@ struct Engine final : EngineBase {
             float t0 = 0.f, t1 = 0.f, t2 = 0.f, t3 = 0.f;
             int rc2;
             if ((rc2 = tune(0, stage, sg, &sg.grid_row, nr, oc[0], &t0))) return rc2;
-            if ((rc2 = tune(2, stage, sg, &sg.grid_rinv, nr, oc[1], &t1))) return rc2;
-            if ((rc2 = tune(2, full, sg, &sg.grid_rfull, nr, oc[2], &t2))) return rc2;
-            if (sg.fast_row && sg.fuse_rows && (rc2 = tune(3, stage, sg, &sg.grid_fused, nr, oc[3], &t3))) return rc2;
+            if (sg.fast_row) {   // (the generic inverse pass takes the forward pass's grid)
+                if ((rc2 = tune(2, stage, sg, &sg.grid_rinv, nr, oc[1], &t1))) return rc2;
+                if ((rc2 = tune(2, full, sg, &sg.grid_rfull, nr, oc[2], &t2))) return rc2;
+            }
+            if (sg.fuse_rows && (rc2 = tune(3, stage, sg, &sg.grid_fused, nr, oc[3], &t3))) return rc2;
             *total = t0 + t1 + t2 + t3;
             return LLG_OK;
         };
@@ -982,16 +991,19 @@ struct Engine final : EngineBase {
             if (tuning && (rc = time_col(v, &t))) return rc;
             cseg[i] = cseg_alt[i][v];
         }
-        // generic shared-memory kernels: the radix order / grouping of each length,
-        // timed on the segment's passes at its current grid
+        // generic shared-memory kernels: the radix order / grouping of each length, timed
+        // on the segment's passes at its current grid: columns, or the fused row pass (five
+        // of an attempt's seven), or its two halves where rows are not fused
         auto time_pass = [&](int kind, LaunchGeom& g, float* t) -> int {
-            const int whiches[2][2] = {{0, 2}, {1, 1}};
-            const int nw = kind == 0 ? 2 : 1;
-            for (int w = 0; w < 2; ++w)
-                for (int q = 0; q < nw; ++q) CUDA_TRY(launch_one<R>(whiches[kind][q], stage, g, stream));
+            auto pass = [&]() -> cudaError_t {
+                if (kind == 1) return launch_one<R>(1, stage, g, stream);
+                if (g.fuse_rows) return launch_fused<R>(stage, next, g, stream);
+                cudaError_t e = launch_one<R>(0, stage, g, stream);
+                return e == cudaSuccess ? launch_one<R>(2, stage, g, stream) : e;
+            };
+            for (int w = 0; w < 2; ++w) CUDA_TRY(pass());
             CUDA_TRY(cudaEventRecord(e0, stream));
-            for (int r = 0; r < 4; ++r)
-                for (int q = 0; q < nw; ++q) CUDA_TRY(launch_one<R>(whiches[kind][q], stage, g, stream));
+            for (int r = 0; r < 4; ++r) CUDA_TRY(pass());
             CUDA_TRY(cudaEventRecord(e1, stream));
             CUDA_TRY(cudaEventSynchronize(e1));
             CUDA_TRY(cudaEventElapsedTime(t, e0, e1));
@@ -1025,12 +1037,14 @@ struct Engine final : EngineBase {
                 for (int L : lengths) {
                     const std::vector<FftPlan> cand = plan_candidates(L);
                     auto apply = [&](const FftPlan& pl) -> int {
+                        const void* made = nullptr;   // the films of a length share the tables
                         for (int f : films[i]) {
                             if ((kind == 0 ? fh[f].nx : fh[f].ny) != L) continue;
                             FftPlan& dst = kind == 0 ? fh[f].plan_row : fh[f].plan_col;
                             void* tab = kind == 0 ? fh[f].twg_row : fh[f].twg_col;
                             dst = generic_plan(pl);
-                            if (tab) CUDA_TRY(launch_pass_tables(dst, tab, sizeof(R) == 8, stream));
+                            if (tab && tab != made) CUDA_TRY(launch_pass_tables(dst, tab, sizeof(R) == 8, stream));
+                            made = tab ? tab : made;
                         }
                         return upload_films();
                     };
