@@ -1693,7 +1693,8 @@ struct Engine final : EngineBase {
         // Each iteration executes one request per film; accepted steps are capped by
         // max_accepted_steps and every step size reaches dt_min within a bounded number
         // of rejections, so this bound is only a safety net against a stuck film.
-        const long long max_iters = 16 * std::max<long long>(st->max_accepted_steps, 1) + 1000000;
+        const long long cap = std::min<long long>(std::max<long long>(st->max_accepted_steps, 1), 1LL << 56);
+        const long long max_iters = 16 * cap + 1000000;
         long long iters = 0;
         int per_poll = 4;
         for (;;) {
@@ -1710,7 +1711,8 @@ struct Engine final : EngineBase {
             for (int f = 0; f < nf; ++f) {
                 const bool done = (h_relax[f].done != 0) || h_states[f].err_code != 0;
                 all &= done;
-                if (!done) left = std::max(left, st->max_accepted_steps - h_relax[f].accepted + 1);
+                if (!done)   // at most a round counts: max_accepted_steps may be the largest integer
+                    left = std::max(left, std::min<long long>(32, st->max_accepted_steps - h_relax[f].accepted) + 1);
             }
             if (all) break;
             per_poll = (int)std::min<long long>(4, (left + 7) / 8);
