@@ -106,8 +106,6 @@ template <typename R>
 cudaError_t launch_fused(const EvalSpec& si, const EvalSpec& sf, const LaunchGeom& g, cudaStream_t s,
                          int* nk = nullptr);
 template <typename R>
-cudaError_t launch_eval(const EvalSpec& spec, const LaunchGeom& g, cudaStream_t s);
-template <typename R>
 cudaError_t prepare_eval_kernels(size_t smem_row, size_t smem_col);
 // Launches one pass of an evaluation: 0 = row forward, 1 = column, 2 = row inverse
 // (on the register-FFT path with the streaming stage kernels around them); adds the

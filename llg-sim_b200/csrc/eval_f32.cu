@@ -10,6 +10,5 @@ template bool can_fuse<float>(const EvalSpec&, const EvalSpec&, const LaunchGeom
 template cudaError_t launch_one<float>(int, const EvalSpec&, const LaunchGeom&, cudaStream_t, int*);
 template cudaError_t launch_fused<float>(const EvalSpec&, const EvalSpec&, const LaunchGeom&, cudaStream_t, int*);
 template cudaError_t prepare_eval_kernels<float>(size_t, size_t);
-template cudaError_t launch_eval<float>(const EvalSpec&, const LaunchGeom&, cudaStream_t);
 
 }  // namespace llg

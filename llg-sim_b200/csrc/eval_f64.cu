@@ -10,6 +10,5 @@ template bool can_fuse<double>(const EvalSpec&, const EvalSpec&, const LaunchGeo
 template cudaError_t launch_one<double>(int, const EvalSpec&, const LaunchGeom&, cudaStream_t, int*);
 template cudaError_t launch_fused<double>(const EvalSpec&, const EvalSpec&, const LaunchGeom&, cudaStream_t, int*);
 template cudaError_t prepare_eval_kernels<double>(size_t, size_t);
-template cudaError_t launch_eval<double>(const EvalSpec&, const LaunchGeom&, cudaStream_t);
 
 }  // namespace llg

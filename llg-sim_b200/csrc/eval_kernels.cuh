@@ -256,17 +256,6 @@ cudaError_t launch_fused(const EvalSpec& si, const EvalSpec& sf, const LaunchGeo
 }
 
 template <typename R>
-cudaError_t launch_eval(const EvalSpec& spec, const LaunchGeom& g, cudaStream_t s) {
-    cudaError_t e = launch_one<R>(0, spec, g, s, nullptr);
-    if (e != cudaSuccess) return e;
-    if (spec.demag && g.any_demag) {
-        e = launch_one<R>(1, spec, g, s, nullptr);
-        if (e != cudaSuccess) return e;
-    }
-    return launch_one<R>(2, spec, g, s, nullptr);
-}
-
-template <typename R>
 void fast_occupancy(int nx, int ny, int row_var, int col_var, int* fwd_blocks_per_sm, int* inv_blocks_per_sm,
                     int* full_blocks_per_sm, int* fused_blocks_per_sm, int* col_blocks_per_sm) {
     *fwd_blocks_per_sm = *inv_blocks_per_sm = *full_blocks_per_sm = *fused_blocks_per_sm = *col_blocks_per_sm = 1;
