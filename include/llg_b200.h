@@ -285,15 +285,16 @@ int llg_solver_launch_count(llg_solver* s, int64_t* out);
  *   kernel_planes device, FP64 [4][ny+1][nx+1]: the planes llg_demag_kernel_kspace returns
  *   b_out         device, FP32 SoA [3][ny][nx], overwritten with B_demag (T)
  *   stream        cudaStream_t or NULL; the call is asynchronous on it
- * Scratch: one static 32 MiB device array (and 64 KiB of twiddle tables) per
- * GPU that loads the library, held until exit; requires 1 <= nx, ny <= 2048 and
+ * Scratch: two static device arrays per GPU that loads the library, 32 MiB of
+ * spectrum and twiddles and 64 KiB of pass tables, held until exit; requires
+ * 1 <= nx, ny <= 2048 and
  * 24*(nx+1)*ny + 16*(nx+ny) <= 32 MiB (e.g. 1024 x 1024), else LLG_ERR_INVALID.
- * The first call on a device looks up the array's device address and opts the
+ * The first call on a device looks up the arrays' device addresses and opts the
  * kernels into large shared memory; make that first call before any stream
  * capture.  After cudaDeviceReset the next call on that device repeats this
- * set-up (the reset drops the context the address belonged to), so it too
- * belongs before any capture.  Every call shares the array (no state carries over: each call
- * rewrites all of it before reading), so calls that overlap on the GPU — on
+ * set-up (the reset drops the context the addresses belonged to), so it too
+ * belongs before any capture.  Every call shares both arrays (no state carries over: each call
+ * rewrites what it reads of them, the pass tables too), so calls that overlap on the GPU — on
  * different streams or from different threads — race; serialise them. */
 int llg_demag_field_noalloc(int64_t nx, int64_t ny, double ms, const float* m, const double* kernel_planes,
                             float* b_out, void* stream);

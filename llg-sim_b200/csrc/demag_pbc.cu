@@ -318,10 +318,12 @@ __global__ void k_open_fold(const cx<double>* __restrict__ K, int nx, int ny, do
 }
 
 // Sets the pruned path of an open operator up.  The planes qualify when they are
-// real and even to kOpenTol of their largest value: a built kernel is to a few
-// 1e-16, and dropping what is below 1e-13 changes the field by less than the
-// transforms' own rounding.  A cache file may hold any planes: others keep the
-// general path, and so does an operator for which the extra buffers do not fit.
+// real and even to kOpenTol of their largest value: built kernels of cells about as thick
+// as wide are to 1e-15 or so, and dropping what is below 1e-13 changes the field by no
+// more than the rounding of the kernel sums themselves.  Sums over many points can
+// exceed it (cells of 4 x 4 x 1 nm: 1.4e-13), and a cache file may hold any planes: such
+// operators keep the general path, and so does one for which the extra buffers do not
+// fit.
 constexpr double kOpenTol = 1e-13;
 void open_path_create(llg_demag_op* op) {
     const size_t nk = (size_t)(op->nx + 1) * (op->ny + 1);

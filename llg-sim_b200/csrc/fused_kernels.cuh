@@ -43,9 +43,11 @@ __global__ void __launch_bounds__(RowCfg<R, L, V>::THREADS * XT) __maxnreg__((XT
     // phase 2 takes W cells per step of its loop, two in FP32 and one in FP64 (the same
     // registers): with EARLY the stencil, m0 and the previous torques of a step are all
     // loaded before any arithmetic, one memory round trip per step instead of one per
-    // term.  Plan 1 and the 384-thread FP64 blocks have too few registers for that: they
-    // load the torques where they are used and take the general path for interior
-    // cells too.
+    // term.  Plan 1 and the FP64 blocks of 384 threads before doubling (L = 1024) have too
+    // few registers for that: they load the torques where they are used and take the
+    // general path for interior cells too.  The cap of the one-fold block decides: FP64
+    // blocks doubled to 384 threads keep the early loads at 168 registers and spill for
+    // it (80 to 104 bytes of stores).
     constexpr int W = sizeof(R) == 4 ? 2 : 1, NV = T * L / W;
     using VW = VecW<R, W>;
     constexpr bool EARLY = V == 0 && (sizeof(R) == 4 || C::REG2 > 200);

@@ -5,9 +5,10 @@
 // real-time loop that must not pay allocation latency, or code running where
 // cudaMalloc is not permitted.  llg_demag_field_noalloc serves them: the
 // caller passes device pointers for the magnetisation, the kernel planes and
-// the output; the spectrum scratch and the twiddle tables live in one
-// file-scope static device array of kScratchBytes (every GPU that loads this
-// library holds that array until the process exits).
+// the output; the spectrum scratch and the twiddles live in one file-scope static
+// device array of kScratchBytes (32 MiB), the pass tables of the two transforms in
+// another of 64 KiB (every GPU that loads this library holds both until the process
+// exits).  Every call rewrites both, so overlapping calls race on them.
 //
 // Same algorithm as the three evaluation passes of field_kernels.cuh (zero-
 // padded FFT convolution, demag_fft_uniform.rs:636-769): pruned R2C rows ->
