@@ -77,6 +77,7 @@ struct Control {
     double t_end, max_err, headroom, dt_min, dt_max;
     long long target_acc, attempts;
     int reset_time;
+    int steps;        // 1: the call steps the films (what follows uses k1)
 };
 struct FilmCtl {
     double dt;
@@ -112,7 +113,7 @@ __global__ void k_set_control(FilmDev* films, int nfilms, Control c, const FilmC
     st->err_code = 0;
     st->err_bits = 0ull;
     st->req = REQ_NONE;
-    if (fc[f].invalidate_fsal || (!st->accepted && !k1_current(F, st))) st->fsal_valid = 0;
+    if (fc[f].invalidate_fsal || (c.steps && !st->accepted && !k1_current(F, st))) st->fsal_valid = 0;
     if (c.reset_time) st->t = 0.0;
     if (isfinite(c.t_end)) {
         double rem = c.t_end - st->t;
@@ -1503,6 +1504,7 @@ struct Engine final : EngineBase {
         c.dt_min = dt_min;
         c.dt_max = dt_max;
         c.attempts = 1;
+        c.steps = 1;
         std::unique_ptr<bool[]> inv(new bool[nf]);
         fsal_flags(kind, p, fmask, inv.get());
         if ((rc = set_control(c, p, inv.get(), false))) return rc;
@@ -1548,6 +1550,7 @@ struct Engine final : EngineBase {
         c.target_acc = n_acc;
         c.attempts = max_attempts > 0 ? max_attempts : -1;
         c.reset_time = 1;
+        c.steps = 1;
         // A film whose k1 was evaluated with another gamma or alpha than this call's keeps it
         // after an accepted step and needs a new one after a rejected one (k1_current): as
         // long as there is such a film, attempts go out one by one, each after its stage 1.
